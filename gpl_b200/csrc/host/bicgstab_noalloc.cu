@@ -24,7 +24,7 @@ namespace {
 // rounded up to 256 bytes), the reduction partials and the solver's scalars.
 constexpr int64_t kMaxRows = GPL_BICGSTAB_NOALLOC_MAX_ROWS;
 constexpr size_t kVecBytes = ((size_t)kMaxRows * sizeof(float) + 255) / 256 * 256;
-constexpr size_t kScratchBytes = 7 * kVecBytes + (size_t)gpl::kBicgBlocks * 3 * sizeof(double) + 64 * sizeof(double);
+constexpr size_t kScratchBytes = 7 * kVecBytes + (size_t)gpl::kBicgBlocks * gpl::kBicgParts * sizeof(double) + 64 * sizeof(double);
 
 // In host code this name is only a host-side stand-in for the device array: its address is
 // looked up per device with cudaGetSymbolAddress before a kernel is given it.

@@ -1,13 +1,12 @@
 // The engine's autotuner: picks, where it runs, the fastest of a launch group's forms that
-// give the same results bit for bit (the SpMV's three row layouts, the scatter's shared-tile
-// and straight-to-HBM forms, the small nets' three WA kernels). Which form wins depends on
-// the data (row lengths, how far a block's cells spread, the degree mix) and changes as the
+// give the same results bit for bit (the scatter's shared-tile and straight-to-HBM forms, the
+// small nets' three WA kernels). Which form wins depends on
+// the data (how far a block's cells spread, the degree mix) and changes as the
 // loop moves cells, so each Tuner times its candidates in place with CUDA events on the
 // stream they run on: every candidate in turn for a few uses, then the fastest by its median
 // time, and the probe again every `period` uses. A use is bracketed by start() and stop();
-// finish() is called once the stream has synchronised (the trial's read-back, the solver's
-// batch read), reads the use's time and counts it or, for a use that did less work than the
-// others (a solver batch that ended part-way), drops it. A probe that keeps the form in use
+// finish() is called once the stream has synchronised (the trial's read-back), reads the use's
+// time and counts it or, for a use that did less work than the others, drops it. A probe that keeps the form in use
 // doubles the period to the next (up to 16 times `period`); one that changes it starts over.
 //
 // An environment variable can fix the form instead (its accepted values name the candidates

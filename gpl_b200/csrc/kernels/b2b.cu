@@ -1049,13 +1049,14 @@ cudaError_t IpDevice::solver_order() {
 }
 
 cudaError_t IpDevice::solve(int max_iters, IpAxisResult out[2]) {
-  // the forms give the same products bit for bit, so the choice changes only the speed
-  // GPL_SPMV_FORM=0|1|2 fixes the form (a thread per row, tiled, sliced); else the tuner picks
-  // between the tiled and the sliced form (a thread per row is never the faster)
-  if (!spmv_tune_) {
-    spmv_tune_ = std::make_unique<Tuner>("initial placement SpMV", std::vector<std::string>{"tiled", "sliced"}, nullptr, 2, 48);
+  // The forms give the same products bit for bit, so the choice changes only the speed:
+  // GPL_SPMV_FORM=0|1|2 (a thread per row, tiled, sliced), else the sliced form, the faster at
+  // every size measured (eight iterations, sliced against tiled: 300 cells 255 / 242 us, level;
+  // 100k 454 / 632 us; 400k 1152 / 1829 us).
+  if (spmv_form_ < 0) {
+    spmv_form_ = kSpmvSliced;
     if (const char *f = std::getenv("GPL_SPMV_FORM"))
-      if (f[0] >= '0' && f[0] <= '2' && f[1] == 0) spmv_fixed_ = f[0] - '0';
+      if (f[0] >= '0' && f[0] <= '2' && f[1] == 0) spmv_form_ = f[0] - '0';
   }
   if (ip_order_ < 0) {
     // off by default: measured, the x gathers' locality it buys (under 1 % of a batch) does
@@ -1067,8 +1068,7 @@ cudaError_t IpDevice::solve(int max_iters, IpAxisResult out[2]) {
   const bool ordered = ip_order_ && solves_ > 0 && n_ > 0;
   solves_++;
   if (ordered) CK(solver_order());
-  // the sliced copies whenever the sliced form may run
-  const bool sliced = spmv_fixed_ < 0 || spmv_fixed_ == kSpmvSliced;
+  const bool sliced = spmv_form_ == kSpmvSliced;  // it reads copies of its own
   CsrDev m[2];
   const float *b[2];
   float *x[2];
@@ -1089,12 +1089,10 @@ cudaError_t IpDevice::solve(int max_iters, IpAxisResult out[2]) {
     scratch[a] = (char *)scratch_ + a * scratch_bytes_;
   }
   BicgResult r[2]{};
-  Tuner *t = spmv_fixed_ >= 0 ? nullptr : spmv_tune_.get();
-  const int form = spmv_fixed_ >= 0 ? spmv_fixed_ : kSpmvTiled + spmv_tune_->best();
-  cudaError_t e = bicgstab_solve_pair(m, b, x, max_iters, scratch, s_, r, form, t);
-  const int iters = std::max(r[0].iterations, r[1].iterations);
-  launches += 10 + (int64_t)iters * 7;
-  d2h_bytes += (int64_t)(iters / 8 + 2) * 2 * 120;
+  cudaError_t e = bicgstab_solve_pair(m, b, x, max_iters, scratch, s_, r, spmv_form_);
+  // the starts' launches and a persistent loop (one more for each restart)
+  launches += 2 * 7 + 1;
+  d2h_bytes += 4 * 512;
   out[0].solve = r[0];
   out[1].solve = r[1];
   if (e == cudaSuccess && ordered) {

@@ -1,17 +1,15 @@
 // The initial placement's solver (`bicgstab`, src/bicgstab.rs:615-669) on the device: CSR
 // SpMV with each row summed in column order (the reference's `Csr::mul` order), float vectors,
-// and the inner products and residual norms in double (deterministic block partials). The
-// scalars (rho, alpha, omega) live on the device, and so do the loop's tests: the last kernel
-// of an iteration decides whether the loop goes on, ends (the residual bound, the iteration
-// cap) or must restart (rho too small), and every kernel of the next iteration returns at once
-// unless it goes on. The host enqueues iterations in batches, reads the loop's state once per
-// batch and runs a restart itself when the device asks for one.
+// and the inner products and residual norms in double (deterministic partials). The whole loop
+// is one persistent cooperative kernel (k_solve): the scalars (rho, alpha, omega) and the
+// loop's tests (the residual bound, the iteration cap, the restart) stay on the device, the
+// steps of an iteration are separated by barriers among the system's blocks, and the host
+// reads the loop's state once per launch and runs a restart itself when the device asks for one.
 #include "bicgstab.h"
 
 #include <algorithm>
 
 #include "common.cuh"
-#include "tune.h"
 
 namespace gpl {
 
@@ -22,15 +20,10 @@ enum Scal { S_RHO = 0, S_RHO_OLD, S_ALPHA, S_W, S_RR, S_R0R, S_R0SQ, S_BB, S_COU
 // count, the state (0 iterate, 1 waiting for a restart, 2 ended), and the bounds the tests
 // compare with. Small integers, exact in double.
 enum Loop { S_I = 10, S_STATE, S_TOL2, S_EPS2, S_MAXIT, S_END };
-constexpr int S_TICKET = 16;  // the fused reductions' arrival count (an unsigned int)
+// The persistent loop's words (unsigned ints, each in a 128-byte line of its own past the
+// scalars): the blocks' arrivals at its barriers, and whether a wait ran out.
+constexpr int S_ARRIVE = 16, S_ERROR = 32;
 constexpr double kIterate = 0.0, kRestart = 1.0, kEnded = 2.0;
-// Which launches run: every one (kAlways), or only while the loop iterates (kLive).
-enum Gate { kAlways = -1, kLive = 0 };
-__device__ __forceinline__ bool gated_off(const double *S, int gate) {
-  return gate == kLive && S[S_STATE] != kIterate;
-}
-
-
 // The loop's tests (`while rr > tol2 && i < max_iters`, then the restart test
 // |rho| < eps^2 |r0|^2 at the head of the next iteration), in the reference's order.
 __device__ __forceinline__ double loop_state(const double *S) {
@@ -60,11 +53,9 @@ __device__ __forceinline__ void spmv_rows_rows(int64_t n, const int64_t *__restr
     emit(i, __fadd_rn(0.0f, __fmul_rn(1.0f, tmp)));
   }
 }
-__device__ __forceinline__ void spmv_rows_body(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, float *__restrict__ y, const double *__restrict__ S, int gate) {
-  if (gated_off(S, gate)) return;
+__global__ void __launch_bounds__(kThreads) k_spmv_rows(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, float *__restrict__ y) {
   spmv_rows_rows(n, rs, cols, vals, x, [&](int64_t r, float v) { y[r] = v; });
 }
-__global__ void __launch_bounds__(kThreads) k_spmv_rows(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, float *__restrict__ y, const double *__restrict__ S, int gate) { spmv_rows_body(n, rs, cols, vals, x, y, S, gate); }
 
 template <class Emit>
 __device__ __forceinline__ void spmv_tiled_rows(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, Emit emit) {
@@ -113,11 +104,9 @@ __device__ __forceinline__ void spmv_tiled_rows(int64_t n, const int64_t *__rest
     emit(i, __fadd_rn(0.0f, __fmul_rn(1.0f, tmp)));
   }
 }
-__device__ __forceinline__ void spmv_tiled_body(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, float *__restrict__ y, const double *__restrict__ S, int gate) {
-  if (gated_off(S, gate)) return;
+__global__ void __launch_bounds__(kThreads) k_spmv_tiled(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, float *__restrict__ y) {
   spmv_tiled_rows(n, rs, cols, vals, x, [&](int64_t r, float v) { y[r] = v; });
 }
-__global__ void __launch_bounds__(kThreads) k_spmv_tiled(int64_t n, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const float *__restrict__ x, float *__restrict__ y, const double *__restrict__ S, int gate) { spmv_tiled_body(n, rs, cols, vals, x, y, S, gate); }
 
 //  sliced: over the sliced copy (rows in order of length). The long rows first, a warp per
 //         row: the lanes form 32 products at a time from the CSR arrays (coalesced, several
@@ -186,11 +175,9 @@ __device__ __forceinline__ void spmv_sliced_rows(int64_t n, int64_t n_long, cons
   }
   emit(row, __fadd_rn(0.0f, __fmul_rn(1.0f, tmp)));
 }
-__device__ __forceinline__ void spmv_sliced_body(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, float *__restrict__ y, const double *__restrict__ S, int gate) {
-  if (gated_off(S, gate)) return;
+__global__ void __launch_bounds__(kThreads) k_spmv_sliced(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, float *__restrict__ y) {
   spmv_sliced_rows(n, n_long, rs, cols, vals, sl_row, sl_len, sl_start, sl_ent, x, [&](int64_t r, float v) { y[r] = v; });
 }
-__global__ void __launch_bounds__(kThreads) k_spmv_sliced(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, float *__restrict__ y, const double *__restrict__ S, int gate) { spmv_sliced_body(n, n_long, rs, cols, vals, sl_row, sl_len, sl_start, sl_ent, x, y, S, gate); }
 
 // The order by length: a histogram of the (capped) lengths per block in shared memory, the
 // buckets' starts longest first, then each row's position from its bucket's cursor (a warp's
@@ -265,74 +252,20 @@ __global__ void __launch_bounds__(kThreads) k_slice_fill(int64_t n, int64_t n_lo
   for (int32_t k = 0; k < len; k++) sl_ent[base + (int64_t)k * kSliceRows] = make_int2(cols[b + k], __float_as_int(vals[b + k]));
 }
 
-static void spmv_launch(int form, int eb, cudaStream_t st, const CsrDev &A, const float *in, float *o, const double *S, int gate) {
+static void spmv_launch(int form, cudaStream_t st, const CsrDev &A, const float *in, float *o) {
+  if (A.n <= 0) return;
+  const unsigned eb = (unsigned)((A.n + kThreads - 1) / kThreads);
   if (form == kSpmvSliced)
-    k_spmv_sliced<<<(unsigned)std::max<int64_t>(sliced_blocks(A.n, A.sl_long), 1), kThreads, 0, st>>>(A.n, A.sl_long, A.rs, A.cols, A.vals, A.sl_row, A.sl_len, A.sl_start, A.sl_ent, in, o, S, gate);
+    k_spmv_sliced<<<(unsigned)std::max<int64_t>(sliced_blocks(A.n, A.sl_long), 1), kThreads, 0, st>>>(A.n, A.sl_long, A.rs, A.cols, A.vals, A.sl_row, A.sl_len, A.sl_start, A.sl_ent, in, o);
   else if (form == kSpmvTiled)
-    k_spmv_tiled<<<eb, kThreads, 0, st>>>(A.n, A.rs, A.cols, A.vals, in, o, S, gate);
+    k_spmv_tiled<<<eb, kThreads, 0, st>>>(A.n, A.rs, A.cols, A.vals, in, o);
   else
-    k_spmv_rows<<<eb, kThreads, 0, st>>>(A.n, A.rs, A.cols, A.vals, in, o, S, gate);
+    k_spmv_rows<<<eb, kThreads, 0, st>>>(A.n, A.rs, A.cols, A.vals, in, o);
 }
 
-// Reduce the partials and apply one scalar step (the block's threads over the blocks'
-// partials, in a fixed order, so every launch shape gives the same sums):
-//  which 0: S[dst0..dst0+2] = sums
-//  which 1 (alpha): S_ALPHA = rho / sum0
-//  which 2 (omega): S_W = sum0 > 0 ? sum1 / sum0 : 0
-//  which 3 (end of iteration): S_RR = sum0; S_RHO_OLD = S_RHO; S_RHO = sum1; one more
-//           iteration; the loop's tests for the next one
-//  which 4 (restart): S_R0SQ = S_RHO = S_RR = sum0
-__device__ void scalar_step(const double *part, int nblk, double *S, int which, int dst0, double *sh) {
-  double v[3];
-  for (int j = 0; j < 3; j++) {
-    double s = 0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += __ldcg(part + 3 * b + j);
-    v[j] = block_sum<kThreads>(s, sh);
-  }
-  if (threadIdx.x != 0) return;
-  switch (which) {
-    case 0:
-      S[dst0] = v[0];
-      S[dst0 + 1] = v[1];
-      S[dst0 + 2] = v[2];
-      break;
-    case 1: S[S_ALPHA] = S[S_RHO] / v[0]; break;
-    case 2: S[S_W] = v[0] > 0.0 ? v[1] / v[0] : 0.0; break;
-    case 3:
-      S[S_RR] = v[0];
-      S[S_RHO_OLD] = S[S_RHO];
-      S[S_RHO] = v[1];
-      S[S_I] += 1.0;
-      S[S_STATE] = loop_state(S);
-      break;
-    case 4:
-      S[S_R0SQ] = v[0];
-      S[S_RHO] = v[0];
-      S[S_RR] = v[0];
-      break;
-  }
-}
-
-// Whether this block is the last of its launch to finish (its partial written and fenced
-// before it counts itself); the last one then sees every block's partial. The count is left
-// at zero for the next launch.
-__device__ bool last_block(unsigned int *ticket) {
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    if (last) *ticket = 0;
-  }
-  __syncthreads();
-  if (last) __threadfence();
-  return last;
-}
-
-// Up to three dot products at once; partials[blk * 3 + j]. With which >= 0 the last block to
-// finish also takes that scalar step (one launch fewer than a separate k_scalar).
-__device__ __forceinline__ void dots_body(int64_t n, const float *__restrict__ a0, const float *__restrict__ b0, const float *__restrict__ a1, const float *__restrict__ b1, const float *__restrict__ a2, const float *__restrict__ b2, double *__restrict__ part, double *__restrict__ S, int gate, int which, unsigned int *ticket) {
-  if (gated_off(S, gate)) return;
+// ---- the start: residual and inner products, in launches of their own
+// Up to three dot products at once; partials[blk * 3 + j].
+__global__ void k_dots(int64_t n, const float *__restrict__ a0, const float *__restrict__ b0, const float *__restrict__ a1, const float *__restrict__ b1, const float *__restrict__ a2, const float *__restrict__ b2, double *__restrict__ part) {
   __shared__ double sh[kThreads / 32];
   double s0 = 0, s1 = 0, s2 = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -348,81 +281,29 @@ __device__ __forceinline__ void dots_body(int64_t n, const float *__restrict__ a
     part[3 * blockIdx.x + 1] = t1;
     part[3 * blockIdx.x + 2] = t2;
   }
-  if (which >= 0 && last_block(ticket)) scalar_step(part, gridDim.x, S, which, 0, sh);
 }
 
-// The loop's two inner-product steps, each thread reading 16-byte runs of four, kVecUnroll
-// runs in flight (its terms summed in index order), when the vectors start on a 16-byte
-// boundary, else one element at a time: TWO 0 is r0.v (then alpha), TWO 1 is t.t and t.s
-// (then omega), t read once for both.
-constexpr int kVecUnroll = 2;
-__device__ __forceinline__ bool all_aligned16(const void *a, const void *b, const void *c, const void *d, const void *e, const void *f) {
-  return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d | (uintptr_t)e | (uintptr_t)f) & 15) == 0;
-}
-__device__ __forceinline__ double dot4(float4 a, float4 b, double s) {
-  s += (double)a.x * (double)b.x;
-  s += (double)a.y * (double)b.y;
-  s += (double)a.z * (double)b.z;
-  s += (double)a.w * (double)b.w;
-  return s;
-}
-template <int TWO>
-__device__ __forceinline__ void loop_dots_body(int64_t n, const float *__restrict__ a, const float *__restrict__ b, double *__restrict__ part, double *__restrict__ S, unsigned int *ticket) {
-  if (gated_off(S, kLive)) return;
+// The partials' sums (the block's threads over the blocks' partials, in a fixed order):
+//  which 0 (start): S[S_R0SQ..] = the three sums
+//  which 4 (restart): S_R0SQ = S_RHO = S_RR = sum0
+__global__ void k_scalar(const double *__restrict__ part, int nblk, double *__restrict__ S, int which) {
   __shared__ double sh[kThreads / 32];
-  double s0 = 0, s1 = 0;
-  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t done = 0;
-  if (all_aligned16(a, b, a, b, a, b)) {
-    const int64_t n4 = n / 4;
-    const float4 *A = (const float4 *)a, *B = (const float4 *)b;
-    for (int64_t i = tid; i < n4; i += kVecUnroll * stride) {
-      float4 x[kVecUnroll], y[kVecUnroll];
-#pragma unroll
-      for (int u = 0; u < kVecUnroll; u++) {
-        const int64_t k = i + u * stride;
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        x[u] = k < n4 ? A[k] : z;
-        y[u] = k < n4 ? B[k] : z;
-      }
-#pragma unroll
-      for (int u = 0; u < kVecUnroll; u++) {
-        if (i + u * stride >= n4) break;
-        if (TWO) {
-          s0 = dot4(x[u], x[u], s0);
-          s1 = dot4(x[u], y[u], s1);
-        } else {
-          s0 = dot4(x[u], y[u], s0);
-        }
-      }
-    }
-    done = 4 * n4;
+  double v[3];
+  for (int j = 0; j < 3; j++) {
+    double s = 0;
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += part[3 * b + j];
+    v[j] = block_sum<kThreads>(s, sh);
   }
-  for (int64_t i = done + tid; i < n; i += stride) {
-    if (TWO) {
-      s0 += (double)a[i] * (double)a[i];
-      s1 += (double)a[i] * (double)b[i];
-    } else {
-      s0 += (double)a[i] * (double)b[i];
-    }
+  if (threadIdx.x != 0) return;
+  if (which == 0) {
+    S[S_R0SQ] = v[0];
+    S[S_R0SQ + 1] = v[1];
+    S[S_R0SQ + 2] = v[2];
+  } else {
+    S[S_R0SQ] = v[0];
+    S[S_RHO] = v[0];
+    S[S_RR] = v[0];
   }
-  double t0 = block_sum<kThreads>(s0, sh);
-  double t1 = TWO ? block_sum<kThreads>(s1, sh) : 0.0;
-  if (threadIdx.x == 0) {
-    part[3 * blockIdx.x] = t0;
-    part[3 * blockIdx.x + 1] = t1;
-    part[3 * blockIdx.x + 2] = 0.0;
-  }
-  if (last_block(ticket)) scalar_step(part, gridDim.x, S, TWO ? 2 : 1, 0, sh);
-}
-__global__ void __launch_bounds__(kThreads, 4) k_loop_dots_alpha(int64_t n, const float *__restrict__ r0, const float *__restrict__ v, double *__restrict__ part, double *__restrict__ S, unsigned int *ticket) { loop_dots_body<0>(n, r0, v, part, S, ticket); }
-__global__ void __launch_bounds__(kThreads, 4) k_loop_dots_omega(int64_t n, const float *__restrict__ t, const float *__restrict__ s, double *__restrict__ part, double *__restrict__ S, unsigned int *ticket) { loop_dots_body<1>(n, t, s, part, S, ticket); }
-__global__ void k_dots(int64_t n, const float *__restrict__ a0, const float *__restrict__ b0, const float *__restrict__ a1, const float *__restrict__ b1, const float *__restrict__ a2, const float *__restrict__ b2, double *__restrict__ part, double *__restrict__ S, int gate, int which, unsigned int *ticket) { dots_body(n, a0, b0, a1, b1, a2, b2, part, S, gate, which, ticket); }
-
-__global__ void k_scalar(const double *__restrict__ part, int nblk, double *__restrict__ S, int which, int dst0, int gate) {
-  if (gated_off(S, gate)) return;
-  __shared__ double sh[kThreads / 32];
-  scalar_step(part, nblk, S, which, dst0, sh);
 }
 
 // After a restart (which 4 above): the first one sets the iteration count back to zero.
@@ -432,6 +313,11 @@ __global__ void k_restart_done(double *S, int first) {
 }
 
 __global__ void k_loop_init(double *S, double tol2, double eps2, int max_iters) {
+  S[S_RHO] = S[S_COUNT];  // dot(r0, r) of the start point
+  S[S_RR] = S[S_R0SQ];
+  S[S_RHO_OLD] = 1.0;
+  S[S_ALPHA] = 1.0;
+  S[S_W] = 1.0;
   S[S_I] = 0.0;
   S[S_TOL2] = tol2;
   S[S_EPS2] = eps2;
@@ -439,112 +325,40 @@ __global__ void k_loop_init(double *S, double tol2, double eps2, int max_iters) 
   S[S_STATE] = loop_state(S);
 }
 
-__global__ void k_residual(int64_t n, const float *__restrict__ b, const float *__restrict__ ax, float *__restrict__ r, float *__restrict__ r0, const double *__restrict__ S, int gate) {
-  if (gated_off(S, gate)) return;
+__global__ void k_residual(int64_t n, const float *__restrict__ b, const float *__restrict__ ax, float *__restrict__ r, float *__restrict__ r0) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   float v = __fsub_rn(b[i], ax[i]);
   r[i] = v;
   r0[i] = v;
 }
-
-// The elementwise updates: a thread per run of four elements (one 16-byte load per vector
-// when they all start on a 16-byte boundary); vec_blocks(n) blocks.
-__host__ __device__ __forceinline__ int64_t vec_blocks(int64_t n) { return std::max<int64_t>((n + 4 * kThreads - 1) / (4 * kThreads), 1); }
-// p = r + beta (p - w v), beta = (rho / rho_old) (alpha / w)
-__device__ __forceinline__ void update_p_body(int64_t n, const double *__restrict__ S, const float *__restrict__ r, const float *__restrict__ v, float *__restrict__ p) {
-  if (gated_off(S, kLive)) return;
-  const int64_t i = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
-  if (i >= n) return;
-  const float beta = (float)((S[S_RHO] / S[S_RHO_OLD]) * (S[S_ALPHA] / S[S_W]));
-  const float w = (float)S[S_W];
-  auto f = [&](float ri, float pi, float vi) { return __fadd_rn(ri, __fmul_rn(beta, __fsub_rn(pi, __fmul_rn(w, vi)))); };
-  if (i + 4 <= n && all_aligned16(r, v, p, r, v, p)) {
-    const float4 R = *(const float4 *)(r + i), V = *(const float4 *)(v + i), Pv = *(const float4 *)(p + i);
-    *(float4 *)(p + i) = make_float4(f(R.x, Pv.x, V.x), f(R.y, Pv.y, V.y), f(R.z, Pv.z, V.z), f(R.w, Pv.w, V.w));
-  } else {
-    for (int64_t k = i; k < min(n, i + 4); k++) p[k] = f(r[k], p[k], v[k]);
-  }
+__global__ void k_set_ended(double *S) { S[S_STATE] = kEnded; }
+__global__ void k_fill(int64_t n, float *a, float v) {
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) a[i] = v;
 }
-__global__ void k_update_p(int64_t n, const double *__restrict__ S, const float *__restrict__ r, const float *__restrict__ v, float *__restrict__ p) { update_p_body(n, S, r, v, p); }
 
-__device__ __forceinline__ void update_s_body(int64_t n, const double *__restrict__ S, const float *__restrict__ r, const float *__restrict__ v, float *__restrict__ s) {
-  if (gated_off(S, kLive)) return;
-  const int64_t i = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
-  if (i >= n) return;
-  const float a = (float)S[S_ALPHA];
-  auto f = [&](float ri, float vi) { return __fsub_rn(ri, __fmul_rn(a, vi)); };
-  if (i + 4 <= n && all_aligned16(r, v, s, r, v, s)) {
-    const float4 R = *(const float4 *)(r + i), V = *(const float4 *)(v + i);
-    *(float4 *)(s + i) = make_float4(f(R.x, V.x), f(R.y, V.y), f(R.z, V.z), f(R.w, V.w));
-  } else {
-    for (int64_t k = i; k < min(n, i + 4); k++) s[k] = f(r[k], v[k]);
-  }
-}
-__global__ void k_update_s(int64_t n, const double *__restrict__ S, const float *__restrict__ r, const float *__restrict__ v, float *__restrict__ s) { update_s_body(n, S, r, v, s); }
+// ---- the loop: one persistent cooperative kernel for one or two systems
+//
+// An iteration is seven steps that each need the whole of the one before: p, A p, r0.v, s,
+// A s, (t.t, t.s), and x, r with their two inner products. As launches (seven an iteration,
+// chained) they cost 65 us an iteration for two systems of 100k rows, most of it launch and
+// drain latency; here each system's blocks stay resident and meet at barriers in global memory
+// (1.4 us among 148 blocks), and every block takes the scalar steps itself from the partials
+// instead of waiting for one to publish them. Measured, the initial placement's pair: 37 us an
+// iteration at 100k rows (65 before), 149 us at 400k (165), 10 us at 300 (45); one system of
+// 300k rows 72 us (310, a thread per row). What is left at 100k: two products of 9.7 us each,
+// bound by their gathers of x (1.3 of them a clock and SM), seven barriers, five vector steps
+// of 1.2 to 2.3 us. Two blocks of 512 threads an SM (64 registers); the two systems' barriers
+// are their own, so each takes exactly the steps it would take alone.
+constexpr int kSolveThreads = 512;
+// A block's products of the tiled form at once (40 KB); longer runs go in pieces.
+constexpr int kSolveTile = 10240;
+// Iterations a launch may run before the host looks at the loop's state again.
+constexpr int kSolveBudget = 128;
+// A barrier's wait gives up after this long (a block of the system is gone).
+constexpr unsigned long long kWaitNs = 2000000000ull;
 
-// x += alpha p + w s; r = s - w t; partials of |r|^2 and r0.r, the last block taking the
-// iteration's end (scalar step 3). Runs of four as in the loop's dot products.
-__device__ __forceinline__ void update_xr_body(int64_t n, double *__restrict__ S, const float *__restrict__ p, const float *__restrict__ s, const float *__restrict__ t, const float *__restrict__ r0, float *__restrict__ x, float *__restrict__ r, double *__restrict__ part, unsigned int *ticket) {
-  if (gated_off(S, kLive)) return;
-  __shared__ double sh[kThreads / 32];
-  const float a = (float)S[S_ALPHA], w = (float)S[S_W];
-  double rr = 0, r0r = 0;
-  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
-  auto fx = [&](float xi, float pi, float si) { return __fadd_rn(xi, __fadd_rn(__fmul_rn(a, pi), __fmul_rn(w, si))); };
-  auto fr = [&](float si, float ti) { return __fsub_rn(si, __fmul_rn(w, ti)); };
-  int64_t done = 0;
-  if (all_aligned16(p, s, t, r0, x, r)) {
-    const int64_t n4 = n / 4;
-    constexpr int U = 1;
-    for (int64_t i = tid; i < n4; i += U * stride) {
-      float4 X[U], Pp[U], Sv[U], T[U], R0[U];
-      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t k = i + u * stride;
-        const bool in = k < n4;
-        X[u] = in ? ((const float4 *)x)[k] : z;
-        Pp[u] = in ? ((const float4 *)p)[k] : z;
-        Sv[u] = in ? ((const float4 *)s)[k] : z;
-        T[u] = in ? ((const float4 *)t)[k] : z;
-        R0[u] = in ? ((const float4 *)r0)[k] : z;
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int64_t k = i + u * stride;
-        if (k >= n4) break;
-        ((float4 *)x)[k] = make_float4(fx(X[u].x, Pp[u].x, Sv[u].x), fx(X[u].y, Pp[u].y, Sv[u].y), fx(X[u].z, Pp[u].z, Sv[u].z), fx(X[u].w, Pp[u].w, Sv[u].w));
-        const float4 R = make_float4(fr(Sv[u].x, T[u].x), fr(Sv[u].y, T[u].y), fr(Sv[u].z, T[u].z), fr(Sv[u].w, T[u].w));
-        ((float4 *)r)[k] = R;
-        rr = dot4(R, R, rr);
-        r0r = dot4(R0[u], R, r0r);
-      }
-    }
-    done = 4 * n4;
-  }
-  for (int64_t i = done + tid; i < n; i += stride) {
-    x[i] = fx(x[i], p[i], s[i]);
-    float rv = fr(s[i], t[i]);
-    r[i] = rv;
-    rr += (double)rv * (double)rv;
-    r0r += (double)r0[i] * (double)rv;
-  }
-  double t0 = block_sum<kThreads>(rr, sh);
-  double t1 = block_sum<kThreads>(r0r, sh);
-  if (threadIdx.x == 0) {
-    part[3 * blockIdx.x] = t0;
-    part[3 * blockIdx.x + 1] = t1;
-    part[3 * blockIdx.x + 2] = 0.0;
-  }
-  if (last_block(ticket)) scalar_step(part, gridDim.x, S, 3, 0, sh);  // the iteration's end
-}
-__global__ void __launch_bounds__(kThreads, 4) k_update_xr(int64_t n, double *__restrict__ S, const float *__restrict__ p, const float *__restrict__ s, const float *__restrict__ t, const float *__restrict__ r0, float *__restrict__ x, float *__restrict__ r, double *__restrict__ part, unsigned int *ticket) { update_xr_body(n, S, p, s, t, r0, x, r, part, ticket); }
-
-// Both axes' systems in one launch (blockIdx.y picks the system): the initial placement solves
-// its x and y systems side by side, so each launch carries twice the work and the loop half
-// the launches. Each system keeps its own scalars, state and arrival count, so every one
-// takes exactly the steps it would take alone.
 struct SysDev {
   int64_t n;
   const int64_t *rs;
@@ -556,83 +370,451 @@ struct SysDev {
   const int2 *sl_ent;
   float *x, *r, *r0, *v, *p, *s, *t;
   double *part, *S;
-  unsigned int *ticket;
 };
 struct SysPair {
   SysDev a[2];
 };
-__device__ __forceinline__ SysDev pick(const SysPair &P) { return blockIdx.y ? P.a[1] : P.a[0]; }
 
-// The loop's kernels are launched chained (common.cuh: chain_enter, launch_chained).
-
-__global__ void __launch_bounds__(kThreads) k2_update_p(SysPair P) {
-  chain_enter();
-  SysDev q = pick(P);
-  update_p_body(q.n, q.S, q.r, q.v, q.p);
+__device__ __forceinline__ unsigned int load_acquire(const unsigned int *p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
-// sel 0: v = A p; sel 1: t = A s (each system's rows in the form's order, gated as a whole).
-__global__ void __launch_bounds__(kThreads) k2_spmv_rows(SysPair P, int sel) {
-  chain_enter();
-  SysDev q = pick(P);
-  spmv_rows_body(q.n, q.rs, q.cols, q.vals, sel ? q.s : q.p, sel ? q.t : q.v, q.S, kLive);
-}
-__global__ void __launch_bounds__(kThreads) k2_spmv_tiled(SysPair P, int sel) {
-  chain_enter();
-  SysDev q = pick(P);
-  spmv_tiled_body(q.n, q.rs, q.cols, q.vals, sel ? q.s : q.p, sel ? q.t : q.v, q.S, kLive);
-}
-__global__ void __launch_bounds__(kThreads) k2_spmv_sliced(SysPair P, int sel) {
-  chain_enter();
-  SysDev q = pick(P);
-  spmv_sliced_body(q.n, q.sl_long, q.rs, q.cols, q.vals, q.sl_row, q.sl_len, q.sl_start, q.sl_ent, sel ? q.s : q.p, sel ? q.t : q.v, q.S, kLive);
-}
-// The inner products after each product, in their own launch over the vectors in order
-// (sel 0: r0.v, then alpha; sel 1: t.t and t.s, then omega), the last block taking the scalar
-// step. (Forming them in the SpMV's own launch was measured 11 % slower over the whole
-// initial placement: the sliced form's rows are in length order, so their r0 and s reads
-// scatter, and the fused tail's block reductions stall every block.)
-__global__ void __launch_bounds__(kThreads, 4) k2_dots(SysPair P, int sel) {
-  chain_enter();
-  SysDev q = pick(P);
-  if (sel == 0)
-    loop_dots_body<0>(q.n, q.r0, q.v, q.part, q.S, q.ticket);
-  else
-    loop_dots_body<1>(q.n, q.t, q.s, q.part, q.S, q.ticket);
+// Waits until *p has reached `target` (counts that wrap); false once the wait has run out
+// here or in another block.
+__device__ __forceinline__ bool wait_for(const unsigned int *p, unsigned int target, unsigned int *err) {
+  unsigned long long t0 = 0;
+  for (unsigned int k = 1;; k++) {
+    if ((int)(load_acquire(p) - target) >= 0) return true;
+    if ((k & 255u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+      if (!t0) t0 = t;
+      if (t - t0 > kWaitNs || load_acquire(err)) {
+        atomicExch(err, 1u);
+        return false;
+      }
+    }
+  }
 }
 
-__global__ void __launch_bounds__(kThreads) k2_update_s(SysPair P) {
-  chain_enter();
-  SysDev q = pick(P);
-  update_s_body(q.n, q.S, q.r, q.v, q.s);
+// The system's blocks meeting: what any of them wrote before is visible to all after (one
+// thread's release of the block's writes, its acquire of everyone's; the block's other threads
+// through the block barriers). About 1.5 us among 148 blocks; nothing but the block barrier in
+// a system of one block. False once a wait has run out.
+struct Meet {
+  unsigned int *arrive, *err;
+  unsigned int blocks;   // the system's blocks
+  unsigned int gen;      // barriers passed since the launch
+};
+__device__ __forceinline__ bool meet(Meet &m) {
+  if (m.blocks == 1) {
+    __syncthreads();
+    return true;
+  }
+  bool good = true;
+  m.gen++;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(m.arrive) : "memory");
+    good = wait_for(m.arrive, m.gen * m.blocks, m.err);
+  }
+  return __syncthreads_and(good);
 }
-__global__ void __launch_bounds__(kThreads, 4) k2_update_xr(SysPair P) {
-  chain_enter();
-  SysDev q = pick(P);
-  update_xr_body(q.n, q.S, q.p, q.s, q.t, q.r0, q.x, q.r, q.part, q.ticket);
-}
-__global__ void k_set_ended(double *S) { S[S_STATE] = kEnded; }
 
-__global__ void k_fill(int64_t n, float *a, float v) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) a[i] = v;
+// Two sums, each of 256 threads' values (a half of the block), in block_sum's order, in each
+// half's thread 0. sh: 32 doubles, not used again before the next block barrier.
+__device__ __forceinline__ void half_sums(double &a, double &b, double *sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) sh[w] = a, sh[16 + w] = b;
+  __syncthreads();
+  if ((w & 7) == 0) {
+    a = l < 8 ? sh[w + l] : 0.0;
+    b = l < 8 ? sh[16 + w + l] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+  }
 }
-__global__ void k_scal_init(double *S) {
-  S[S_RHO] = S[S_COUNT];  // dot(r0, r) of the start point
-  S[S_RR] = S[S_R0SQ];
-  S[S_RHO_OLD] = 1.0;
-  S[S_ALPHA] = 1.0;
-  S[S_W] = 1.0;
+
+// The scalars: thread 0 of every block holds them all and takes every scalar step itself from
+// the partials (the same sums in the same order in each block), the steps' factors as floats
+// in shared memory.
+struct Scalars {
+  double rho, rho_old, alpha, w, rr, i;
+};
+struct Factors {
+  float alpha, w, beta;
+  int live;  // the loop goes on
+};
+__device__ __forceinline__ float beta_of(const Scalars &s) { return (float)((s.rho / s.rho_old) * (s.alpha / s.w)); }
+
+// Columns [col, col + 2) of the partials summed (`live` parts of 256 threads; the others'
+// partials are zero), after a barrier; in thread 0.
+__device__ __forceinline__ void sum_parts(const double *part, int col, int live, double *sh, double &s0, double &s1) {
+  s0 = s1 = 0;
+  if (threadIdx.x < kThreads)
+    for (int b = threadIdx.x; b < live; b += kThreads) {
+      s0 += __ldcg(part + kBicgParts * b + col);
+      s1 += __ldcg(part + kBicgParts * b + col + 1);
+    }
+  half_sums(s0, s1, sh);
+}
+
+__device__ __forceinline__ bool aligned16(const void *a, const void *b) { return (((uintptr_t)a | (uintptr_t)b) & 15) == 0; }
+__device__ __forceinline__ double dot4(float4 a, float4 b, double s) {
+  s += (double)a.x * (double)b.x;
+  s += (double)a.y * (double)b.y;
+  s += (double)a.z * (double)b.z;
+  s += (double)a.w * (double)b.w;
+  return s;
+}
+// How many of the kBicgBlocks blocks of 256 threads have a term of an inner product: their
+// threads take runs of four (n4 of them, then the tail one element a thread), or, off 16-byte
+// boundaries, one element each.
+__device__ __forceinline__ int live_parts(int64_t n, int64_t n4) {
+  const int64_t a = (n4 + kThreads - 1) / kThreads, b = (n - 4 * n4 + kThreads - 1) / kThreads;
+  return (int)min((int64_t)kBicgBlocks, max(max(a, b), (int64_t)1));
+}
+constexpr int64_t kPartStride = (int64_t)kBicgBlocks * kThreads;
+
+// The loop's two inner-product steps: TWO 0 is a.b (r0.v), TWO 1 is a.a and a.b (t.t and t.s).
+// The sums are those of kBicgBlocks blocks of 256 threads, each thread over runs of four
+// elements in index order; a block here takes one such block a half (parts c and blocks + c),
+// so the partials and their order do not depend on the launch's shape.
+template <int TWO>
+__device__ __forceinline__ int loop_dots(int64_t n, const float *a, const float *b, double *part, int col, int c, int blocks, double *sh) {
+  const int h = threadIdx.x / kThreads, t = threadIdx.x % kThreads;
+  const int64_t n4 = aligned16(a, b) ? n / 4 : 0;
+  const int live = live_parts(n, n4);
+  for (int base = 0; base < live; base += 2 * blocks) {
+    const int vb = base + h * blocks + c;
+    double s0 = 0, s1 = 0;
+    if (vb < live) {
+      const int64_t tid = (int64_t)vb * kThreads + t;
+      const float4 *A = (const float4 *)a, *B = (const float4 *)b;
+      for (int64_t i = tid; i < n4; i += 2 * kPartStride) {
+        const int64_t j = i + kPartStride;
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 x0 = A[i], y0 = B[i], x1 = j < n4 ? A[j] : z, y1 = j < n4 ? B[j] : z;
+        if (TWO) s0 = dot4(x0, x0, s0);
+        (TWO ? s1 : s0) = dot4(x0, y0, TWO ? s1 : s0);
+        if (j < n4) {
+          if (TWO) s0 = dot4(x1, x1, s0);
+          (TWO ? s1 : s0) = dot4(x1, y1, TWO ? s1 : s0);
+        }
+      }
+      for (int64_t i = 4 * n4 + tid; i < n; i += kPartStride) {
+        if (TWO) {
+          s0 += (double)a[i] * (double)a[i];
+          s1 += (double)a[i] * (double)b[i];
+        } else {
+          s0 += (double)a[i] * (double)b[i];
+        }
+      }
+    }
+    if (base) __syncthreads();  // the sums' shared words again
+    half_sums(s0, s1, sh);
+    if (t == 0 && vb < live) {
+      part[kBicgParts * vb + col] = s0;
+      part[kBicgParts * vb + col + 1] = s1;
+    }
+  }
+  return live;
+}
+
+// x += alpha p + w s; r = s - w t; partials of |r|^2 and r0.r, in the same parts.
+__device__ __forceinline__ int update_xr(const SysDev &q, float al, float w, int col, int c, int blocks, double *sh) {
+  const int h = threadIdx.x / kThreads, t = threadIdx.x % kThreads;
+  auto fx = [&](float xi, float pi, float si) { return __fadd_rn(xi, __fadd_rn(__fmul_rn(al, pi), __fmul_rn(w, si))); };
+  auto fr = [&](float si, float ti) { return __fsub_rn(si, __fmul_rn(w, ti)); };
+  const int64_t n4 = aligned16(q.x, q.r) ? q.n / 4 : 0;  // the scratch's vectors lie alike
+  const int live = live_parts(q.n, n4);
+  for (int base = 0; base < live; base += 2 * blocks) {
+    const int vb = base + h * blocks + c;
+    double rr = 0, r0r = 0;
+    if (vb < live) {
+      const int64_t tid = (int64_t)vb * kThreads + t;
+      for (int64_t k = tid; k < n4; k += kPartStride) {
+        const float4 X = ((const float4 *)q.x)[k], P = ((const float4 *)q.p)[k], Sv = ((const float4 *)q.s)[k], T = ((const float4 *)q.t)[k], R0 = ((const float4 *)q.r0)[k];
+        ((float4 *)q.x)[k] = make_float4(fx(X.x, P.x, Sv.x), fx(X.y, P.y, Sv.y), fx(X.z, P.z, Sv.z), fx(X.w, P.w, Sv.w));
+        const float4 R = make_float4(fr(Sv.x, T.x), fr(Sv.y, T.y), fr(Sv.z, T.z), fr(Sv.w, T.w));
+        ((float4 *)q.r)[k] = R;
+        rr = dot4(R, R, rr);
+        r0r = dot4(R0, R, r0r);
+      }
+      for (int64_t i = 4 * n4 + tid; i < q.n; i += kPartStride) {
+        q.x[i] = fx(q.x[i], q.p[i], q.s[i]);
+        const float rv = fr(q.s[i], q.t[i]);
+        q.r[i] = rv;
+        rr += (double)rv * (double)rv;
+        r0r += (double)q.r0[i] * (double)rv;
+      }
+    }
+    if (base) __syncthreads();  // the sums' shared words again
+    half_sums(rr, r0r, sh);
+    if (t == 0 && vb < live) {
+      q.part[kBicgParts * vb + col] = rr;
+      q.part[kBicgParts * vb + col + 1] = r0r;
+    }
+  }
+  return live;
+}
+
+// out[i] = f(i, a run of four or one element) over the system's threads.
+template <class F>
+__device__ __forceinline__ void each4(int64_t n, bool aligned, int c, int blocks, F f) {
+  const int64_t tid = (int64_t)c * kSolveThreads + threadIdx.x, stride = (int64_t)blocks * kSolveThreads;
+  const int64_t n4 = aligned ? n / 4 : 0;
+  for (int64_t i = tid; i < n4; i += stride) f(4 * i, true);
+  for (int64_t i = 4 * n4 + tid; i < n; i += stride) f(i, false);
+}
+
+// y = A x over the system's blocks, each row's products summed in column order (the forms of
+// SpmvForm, bit for bit the same y). x and y are written in this kernel: plain loads.
+//  rows:   a thread per row straight from memory;
+//  tiled:  a block's run of rows, its entries' products formed by all its threads into shared
+//          memory (coalesced, eight gathers a thread in flight), then a thread per row;
+//  sliced: a warp per long row (products through shuffles), then per slice of 32 rows.
+template <int FORM>
+__device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, float *y, int c, int blocks, float *prod) {
+  const int64_t n = q.n;
+  if (FORM == kSpmvRows) {
+    for (int64_t i = (int64_t)c * kSolveThreads + threadIdx.x; i < n; i += (int64_t)blocks * kSolveThreads) {
+      float tmp = 0.0f;
+      const int64_t b = __ldg(q.rs + i), e = __ldg(q.rs + i + 1);
+      for (int64_t k = b; k < e; k++) tmp = __fadd_rn(tmp, __fmul_rn(__ldg(q.vals + k), x[__ldg(q.cols + k)]));
+      y[i] = __fadd_rn(0.0f, __fmul_rn(1.0f, tmp));
+    }
+  } else if (FORM == kSpmvTiled) {
+    // runs of at most kSolveThreads rows, as many a block as fill them evenly
+    const int64_t per = (n + (int64_t)blocks * kSolveThreads - 1) / ((int64_t)blocks * kSolveThreads);
+    const int64_t run = min((int64_t)kSolveThreads, ((n + blocks * per - 1) / (blocks * per) + 31) / 32 * 32);
+    for (int64_t r0 = c * run; r0 < n; r0 += blocks * run) {
+      const int64_t r1 = min(n, r0 + run), i = r0 + threadIdx.x;
+      const int64_t k0 = __ldg(q.rs + r0), k1 = __ldg(q.rs + r1);
+      int64_t at = 0, e = 0;
+      if (i < r1) {
+        at = __ldg(q.rs + i);
+        e = __ldg(q.rs + i + 1);
+      }
+      float tmp = 0.0f;
+      for (int64_t m0 = k0; m0 < k1; m0 += kSolveTile) {
+        const int cnt = (int)min((int64_t)kSolveTile, k1 - m0);
+        const int32_t *cc = q.cols + m0;
+        const float *vv = q.vals + m0;
+        for (int j = threadIdx.x; j < cnt; j += kSpmvUnroll * kSolveThreads) {
+          int ci[kSpmvUnroll];
+          float va[kSpmvUnroll], xv[kSpmvUnroll];
+#pragma unroll
+          for (int u = 0; u < kSpmvUnroll; u++) {
+            const int w = j + u * kSolveThreads;
+            ci[u] = w < cnt ? __ldg(cc + w) : 0;
+            va[u] = w < cnt ? __ldg(vv + w) : 0.0f;
+          }
+#pragma unroll
+          for (int u = 0; u < kSpmvUnroll; u++) xv[u] = j + u * kSolveThreads < cnt ? x[ci[u]] : 0.0f;
+#pragma unroll
+          for (int u = 0; u < kSpmvUnroll; u++) {
+            const int w = j + u * kSolveThreads;
+            if (w < cnt) prod[w] = __fmul_rn(va[u], xv[u]);
+          }
+        }
+        __syncthreads();
+        const int lb = (int)(at - m0), le = (int)(min(e, m0 + cnt) - m0);
+        int k = lb;
+        if (le - lb >= 4 * kSpmvUnroll) {
+          // a long row: 16-byte loads, the next eight products beside the eight dependent adds
+          for (; k & 3; k++) tmp = __fadd_rn(tmp, prod[k]);
+          const float4 *p4 = reinterpret_cast<const float4 *>(prod + k);
+          float4 c0 = p4[0], c1 = p4[1];
+          for (; k + 16 <= le; k += 8) {
+            p4 += 2;
+            const float4 n0 = p4[0], n1 = p4[1];
+            tmp = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tmp, c0.x), c0.y), c0.z), c0.w);
+            tmp = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tmp, c1.x), c1.y), c1.z), c1.w);
+            c0 = n0;
+            c1 = n1;
+          }
+          tmp = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tmp, c0.x), c0.y), c0.z), c0.w);
+          tmp = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(tmp, c1.x), c1.y), c1.z), c1.w);
+          k += 8;
+        }
+        for (; k < le; k++) tmp = __fadd_rn(tmp, prod[k]);
+        if (le > lb) at = m0 + le;
+        __syncthreads();
+      }
+      if (i < r1) y[i] = __fadd_rn(0.0f, __fmul_rn(1.0f, tmp));
+    }
+  } else {
+    const int lane = threadIdx.x & 31;
+    const int64_t ns = (n - q.sl_long + kSliceRows - 1) / kSliceRows, items = q.sl_long + ns;
+    const int64_t warps = (int64_t)blocks * (kSolveThreads / 32);
+    // neighbouring items on different blocks: the longest rows spread over the SMs
+    for (int64_t w = (int64_t)(threadIdx.x >> 5) * blocks + c; w < items; w += warps) {
+      if (w < q.sl_long) {
+        const int32_t row = __ldg(q.sl_row + w);
+        const int64_t b = __ldg(q.rs + row), e = __ldg(q.rs + row + 1);
+        float sum = 0.0f;
+        for (int64_t m = b; m < e; m += 32 * kLongChunks) {
+          float pr[kLongChunks];
+#pragma unroll
+          for (int u = 0; u < kLongChunks; u++) {
+            const int64_t k = m + 32 * u + lane;
+            pr[u] = k < e ? __fmul_rn(__ldg(q.vals + k), x[__ldg(q.cols + k)]) : 0.0f;
+          }
+#pragma unroll
+          for (int u = 0; u < kLongChunks; u++) {
+            const int64_t c0 = m + 32 * u;
+            if (c0 >= e) break;  // uniform across the warp
+            if (e - c0 >= 32) {
+#pragma unroll
+              for (int z = 0; z < 32; z++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, pr[u], z));
+            } else {
+              const int cnt = (int)(e - c0);
+              for (int z = 0; z < cnt; z++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, pr[u], z));
+            }
+          }
+        }
+        if (lane == 0) y[row] = __fadd_rn(0.0f, __fmul_rn(1.0f, sum));
+        continue;
+      }
+      const int64_t slice = w - q.sl_long, j = q.sl_long + slice * kSliceRows + lane;
+      if (j >= n) continue;
+      const int32_t len = __ldg(q.sl_len + j), row = __ldg(q.sl_row + j);
+      const int2 *ent = q.sl_ent + __ldg(q.sl_start + slice) + lane;
+      float tmp = 0.0f;
+      for (int32_t k = 0; k < len; k += kSpmvUnroll) {
+        int2 cv[kSpmvUnroll];
+        float xv[kSpmvUnroll];
+#pragma unroll
+        for (int u = 0; u < kSpmvUnroll; u++) cv[u] = k + u < len ? __ldg(ent + (int64_t)(k + u) * kSliceRows) : make_int2(0, 0);
+#pragma unroll
+        for (int u = 0; u < kSpmvUnroll; u++) xv[u] = k + u < len ? x[cv[u].x] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < kSpmvUnroll; u++)
+          if (k + u < len) tmp = __fadd_rn(tmp, __fmul_rn(__int_as_float(cv[u].y), xv[u]));
+      }
+      y[row] = __fadd_rn(0.0f, __fmul_rn(1.0f, tmp));
+    }
+  }
+}
+
+// blocks: a system's blocks; block b belongs to system b % nsys (with an even count of SMs and
+// two blocks an SM, both of an SM's are one system's, so they share its vectors in L1).
+template <int FORM>
+__global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys, int blocks) {
+  __shared__ double shp[32], shs[32];  // the partials' sums, the scalar steps' sums
+  __shared__ __align__(16) float prod[FORM == kSpmvTiled ? kSolveTile : 4];
+  __shared__ Factors f;
+  const int sys = (int)(blockIdx.x % nsys), c = (int)(blockIdx.x / nsys);
+  const SysDev q = sys ? P.a[1] : P.a[0];
+  const int64_t n = q.n;
+  double *S = q.S;
+  Meet m{reinterpret_cast<unsigned int *>(S + S_ARRIVE), reinterpret_cast<unsigned int *>(S + S_ERROR), (unsigned int)blocks, 0u};
+  const bool al = aligned16(q.r, q.r);
+  Scalars k{};
+  double s0, s1;
+  if (threadIdx.x == 0) {
+    k = Scalars{S[S_RHO], S[S_RHO_OLD], S[S_ALPHA], S[S_W], S[S_RR], S[S_I]};
+    f.live = S[S_STATE] == kIterate;
+    f.beta = beta_of(k);
+    f.w = (float)k.w;
+  }
+  const double tol2 = S[S_TOL2], eps2r = S[S_EPS2] * S[S_R0SQ], maxit = S[S_MAXIT];
+  double state = S[S_STATE];  // thread 0's follows the loop
+  __syncthreads();
+  if (!f.live) return;
+  for (int it = 0; it < kSolveBudget && f.live; it++) {
+    // p = r + beta (p - w v), beta = (rho / rho_old) (alpha / w)
+    {
+      const float beta = f.beta, w = f.w;
+      auto g = [&](float ri, float pi, float vi) { return __fadd_rn(ri, __fmul_rn(beta, __fsub_rn(pi, __fmul_rn(w, vi)))); };
+      each4(n, al, c, blocks, [&](int64_t i, bool four) {
+        if (four) {
+          const float4 R = *(const float4 *)(q.r + i), V = *(const float4 *)(q.v + i), Pv = *(const float4 *)(q.p + i);
+          *(float4 *)(q.p + i) = make_float4(g(R.x, Pv.x, V.x), g(R.y, Pv.y, V.y), g(R.z, Pv.z, V.z), g(R.w, Pv.w, V.w));
+        } else {
+          q.p[i] = g(q.r[i], q.p[i], q.v[i]);
+        }
+      });
+    }
+    if (!meet(m)) return;
+    solve_spmv<FORM>(q, q.p, q.v, c, blocks, prod);
+    if (!meet(m)) return;
+    int live = loop_dots<0>(n, q.r0, q.v, q.part, 0, c, blocks, shp);
+    if (!meet(m)) return;
+    sum_parts(q.part, 0, live, shs, s0, s1);
+    if (threadIdx.x == 0) {
+      k.alpha = k.rho / s0;
+      f.alpha = (float)k.alpha;
+    }
+    __syncthreads();
+    const float alpha = f.alpha;
+    // s = r - alpha v
+    {
+      auto g = [&](float ri, float vi) { return __fsub_rn(ri, __fmul_rn(alpha, vi)); };
+      each4(n, al, c, blocks, [&](int64_t i, bool four) {
+        if (four) {
+          const float4 R = *(const float4 *)(q.r + i), V = *(const float4 *)(q.v + i);
+          *(float4 *)(q.s + i) = make_float4(g(R.x, V.x), g(R.y, V.y), g(R.z, V.z), g(R.w, V.w));
+        } else {
+          q.s[i] = g(q.r[i], q.v[i]);
+        }
+      });
+    }
+    if (!meet(m)) return;
+    solve_spmv<FORM>(q, q.s, q.t, c, blocks, prod);
+    if (!meet(m)) return;
+    live = loop_dots<1>(n, q.t, q.s, q.part, 0, c, blocks, shp);
+    if (!meet(m)) return;
+    sum_parts(q.part, 0, live, shs, s0, s1);
+    if (threadIdx.x == 0) {
+      k.w = s0 > 0.0 ? s1 / s0 : 0.0;
+      f.w = (float)k.w;
+    }
+    __syncthreads();
+    // the third pair's columns are its own: a block may still read the second's
+    live = update_xr(q, alpha, f.w, 2, c, blocks, shp);
+    if (!meet(m)) return;
+    sum_parts(q.part, 2, live, shs, s0, s1);
+    if (threadIdx.x == 0) {
+      // the iteration's end and the loop's tests (`while rr > tol2 && i < max_iters`, then the
+      // restart test |rho| < eps^2 |r0|^2 at the head of the next iteration), in that order
+      k.rr = s0;
+      k.rho_old = k.rho;
+      k.rho = s1;
+      k.i += 1.0;
+      state = !(k.rr > tol2 && k.i < maxit) ? kEnded : fabs(k.rho) < eps2r ? kRestart : kIterate;
+      f.live = state == kIterate;
+      f.beta = beta_of(k);
+    }
+    __syncthreads();
+  }
+  if (c == 0 && threadIdx.x == 0) {
+    S[S_RHO] = k.rho;
+    S[S_RHO_OLD] = k.rho_old;
+    S[S_ALPHA] = k.alpha;
+    S[S_W] = k.w;
+    S[S_RR] = k.rr;
+    S[S_I] = k.i;
+    S[S_STATE] = state;
+  }
 }
 
 }  // namespace
 
-// Iterations enqueued between two reads of the loop's state.
-constexpr int kBicgBatch = 8;
-
 size_t bicgstab_scratch_bytes(int64_t n) {
   size_t vec = (size_t)n * sizeof(float);
   vec = (vec + 255) / 256 * 256;
-  return 7 * vec + (size_t)kBicgBlocks * 3 * sizeof(double) + 64 * sizeof(double);
+  return 7 * vec + (size_t)kBicgBlocks * kBicgParts * sizeof(double) + 64 * sizeof(double);
 }
 
 size_t bicgstab_pair_scratch_bytes(int64_t n) { return bicgstab_scratch_bytes(n); }
@@ -664,107 +846,41 @@ cudaError_t spmv(const CsrDev &A, const float *x, float *y, int form, cudaStream
   if (form != kSpmvRows && form != kSpmvTiled && form != kSpmvSliced) return cudaErrorInvalidValue;
   if (form == kSpmvSliced && (!A.sl_start || !A.sl_row || !A.sl_len)) return cudaErrorInvalidValue;
   if (A.n <= 0) return cudaSuccess;
-  spmv_launch(form, (int)((A.n + kThreads - 1) / kThreads), st, A, x, y, nullptr, kAlways);
+  spmv_launch(form, st, A, x, y);
   return cudaGetLastError();
 }
 
-cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t st, BicgResult *out, int form) {
-  static_assert(S_END <= S_TICKET && S_TICKET < 64, "the scalars fit the scratch's 64 doubles");
-  if (form == kSpmvSliced && (!A.sl_start || !A.sl_row || !A.sl_len)) return cudaErrorInvalidValue;
-  int64_t n = A.n;
-  size_t vec = ((size_t)n * sizeof(float) + 255) / 256 * 256;
-  char *base = (char *)scratch;
-  float *r = (float *)(base), *r0 = (float *)(base + vec), *v = (float *)(base + 2 * vec), *p = (float *)(base + 3 * vec);
-  float *s = (float *)(base + 4 * vec), *t = (float *)(base + 5 * vec), *ax = (float *)(base + 6 * vec);
-  double *part = (double *)(base + 7 * vec);
-  double *S = part + (size_t)kBicgBlocks * 3;
-  unsigned int *ticket = (unsigned int *)(S + S_TICKET);
-  int eb = (int)((n + kThreads - 1) / kThreads);
-  if (eb < 1) eb = 1;
-  int rb = kBicgBlocks;
-  const float tol = 1.1920929e-07f;
-  double hs[S_END];
-  auto spmv = [&](const float *in, float *o, int gate) { spmv_launch(form, eb, st, A, in, o, S, gate); };
-  auto pull = [&]() -> cudaError_t {
-    cudaError_t e = cudaMemcpyAsync(hs, S, sizeof hs, cudaMemcpyDeviceToHost, st);
-    if (e != cudaSuccess) return e;
-    return cudaStreamSynchronize(st);
-  };
-  cudaError_t e;
-  spmv(x, ax, kAlways);
-  k_residual<<<eb, kThreads, 0, st>>>(n, b, ax, r, r0, S, kAlways);
-  cudaMemsetAsync(ticket, 0, sizeof(unsigned int), st);
-  k_dots<<<rb, kThreads, 0, st>>>(n, r0, r0, b, b, r0, r, part, S, kAlways, -1, ticket);
-  k_scalar<<<1, kThreads, 0, st>>>(part, rb, S, 0, S_R0SQ, kAlways);  // S_R0SQ, S_BB, then dot(r0, r) in S[S_COUNT]
-  if ((e = pull()) != cudaSuccess) return e;
-  double rhs_sqnorm = hs[S_BB];
-  if (rhs_sqnorm == 0.0) {
-    k_fill<<<eb, kThreads, 0, st>>>(n, x, 0.0f);
-    out->iterations = max_iters;
-    out->error = tol;
-    out->converged = true;
-    return cudaGetLastError();
-  }
-  k_scal_init<<<1, 1, 0, st>>>(S);
-  cudaMemsetAsync(v, 0, (size_t)n * sizeof(float), st);
-  cudaMemsetAsync(p, 0, (size_t)n * sizeof(float), st);
-  double tol2 = (double)tol * (double)tol * rhs_sqnorm;
-  double eps2 = (double)tol * (double)tol;
-  k_loop_init<<<1, 1, 0, st>>>(S, tol2, eps2, max_iters);
-  // Every iteration counts one and only the first restart sets the count back, so the loop
-  // ends within 2 max_iters + 1 iterations; a batch that asks for a restart holds until the
-  // host has run it, and every batch but the last runs at least one iteration.
-  const int64_t max_batches = 2 * (int64_t)max_iters + 3;
-  int64_t batches = 0;
-  int restarts = 0;
-  for (;;) {
-    for (int k = 0; k < kBicgBatch; k++) {
-      k_update_p<<<(unsigned)vec_blocks(n), kThreads, 0, st>>>(n, S, r, v, p);
-      spmv(p, v, kLive);
-      k_loop_dots_alpha<<<rb, kThreads, 0, st>>>(n, r0, v, part, S, ticket);
-      k_update_s<<<(unsigned)vec_blocks(n), kThreads, 0, st>>>(n, S, r, v, s);
-      spmv(s, t, kLive);
-      k_loop_dots_omega<<<rb, kThreads, 0, st>>>(n, t, s, part, S, ticket);
-      k_update_xr<<<rb, kThreads, 0, st>>>(n, S, p, s, t, r0, x, r, part, ticket);
-    }
-    if ((e = pull()) != cudaSuccess) return e;
-    if (hs[S_STATE] == kEnded) break;
-    if (++batches > max_batches) return cudaErrorUnknown;  // cannot happen: the count above
-    if (hs[S_STATE] == kRestart) {
-      // too orthogonal to r0: restart from the current residual
-      spmv(x, ax, kAlways);
-      k_residual<<<eb, kThreads, 0, st>>>(n, b, ax, r, r0, S, kAlways);
-      k_dots<<<rb, kThreads, 0, st>>>(n, r, r, nullptr, nullptr, nullptr, nullptr, part, S, kAlways, -1, ticket);
-      k_scalar<<<1, kThreads, 0, st>>>(part, rb, S, 4, 0, kAlways);
-      k_restart_done<<<1, 1, 0, st>>>(S, restarts == 0 ? 1 : 0);
-      restarts++;
-    }
-  }
-  double rr = hs[S_RR];
-  out->iterations = (int)hs[S_I];
-  out->error = (float)std::sqrt(rr / rhs_sqnorm);
-  out->converged = out->error <= tol;
-  return cudaGetLastError();
+// One launch of the loop: its blocks are all resident at once (a cooperative launch), at most
+// two an SM. A system of up to kSolveThreads rows runs in one block, where a barrier is the
+// block's own (300 rows: 10 us an iteration against 17 in three blocks). Beyond that the
+// tiled form, whose threads share a run's entries, takes a block for every 128 rows (3000 rows:
+// 19.5 us against 22.4 with 512), the others a thread per row (10k rows, sliced, two systems:
+// 24 us against 25 with 128).
+static cudaError_t solve_launch(int form, SysPair P, int nsys, cudaStream_t st) {
+  const void *fn = form == kSpmvSliced ? (const void *)k_solve<kSpmvSliced> : form == kSpmvTiled ? (const void *)k_solve<kSpmvTiled> : (const void *)k_solve<kSpmvRows>;
+  int dev = 0, sms = 0, per = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kSolveThreads, 0);
+  if (e != cudaSuccess) return e;
+  const int most = std::max(1, sms * std::min(per, 2) / nsys);
+  const int64_t rows = form == kSpmvTiled && P.a[0].n > kSolveThreads ? kSolveThreads / 4 : kSolveThreads;
+  int blocks = (int)std::min<int64_t>(most, std::max<int64_t>(1, (P.a[0].n + rows - 1) / rows));
+  for (int a = 0; a < nsys; a++)
+    if ((e = cudaMemsetAsync(P.a[a].S + S_ARRIVE, 0, (64 - S_ARRIVE) * sizeof(double), st)) != cudaSuccess) return e;
+  void *args[] = {&P, &nsys, &blocks};
+  return cudaLaunchCooperativeKernel(fn, dim3((unsigned)(blocks * nsys)), dim3(kSolveThreads), args, 0, st);
 }
 
-// One chained launch of a loop kernel (kThreads a block, no dynamic shared memory).
-template <typename... KArgs, typename... Args>
-static cudaError_t chained(void (*kernel)(KArgs...), dim3 grid, cudaStream_t st, Args... args) {
-  return launch_chained(kernel, grid, dim3(kThreads), 0, st, args...);
-}
-#define CK_LAUNCH(x)                        \
-  do {                                      \
-    if ((e = (x)) != cudaSuccess) return e; \
-  } while (0)
-
-cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], float *const x[2], int max_iters, void *const scratch[2], cudaStream_t st, BicgResult out[2], int form, Tuner *tune) {
+// One or two systems of the same size, each with its own scalars and state.
+static cudaError_t solve_systems(int nsys, const CsrDev *A, const float *const *b, float *const *x, int max_iters, void *const *scratch, cudaStream_t st, BicgResult *out, int form) {
+  static_assert(S_END <= S_ARRIVE && S_ERROR < 64, "the scalars fit the scratch's 64 doubles");
   const int64_t n = A[0].n;
-  if (A[1].n != n) return cudaErrorInvalidValue;
-  for (int a = 0; a < 2; a++)
-    if ((form == kSpmvSliced || tune) && (!A[a].sl_start || !A[a].sl_row || !A[a].sl_len)) return cudaErrorInvalidValue;
   const size_t vec = ((size_t)n * sizeof(float) + 255) / 256 * 256;
   SysPair P{};
-  for (int a = 0; a < 2; a++) {
+  for (int a = 0; a < nsys; a++) {
+    if (A[a].n != n) return cudaErrorInvalidValue;
+    if (form == kSpmvSliced && (!A[a].sl_start || !A[a].sl_row || !A[a].sl_len)) return cudaErrorInvalidValue;
     char *base = (char *)scratch[a];
     SysDev &q = P.a[a];
     q.n = n;
@@ -784,45 +900,32 @@ cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], floa
     q.s = (float *)(base + 4 * vec);
     q.t = (float *)(base + 5 * vec);
     q.part = (double *)(base + 7 * vec);
-    q.S = q.part + (size_t)kBicgBlocks * 3;
-    q.ticket = (unsigned int *)(q.S + S_TICKET);
+    q.S = q.part + (size_t)kBicgBlocks * kBicgParts;
   }
   auto ax_of = [&](int a) { return (float *)((char *)scratch[a] + 6 * vec); };
-  int eb = (int)((n + kThreads - 1) / kThreads);
-  if (eb < 1) eb = 1;
+  const int eb = (int)std::max<int64_t>((n + kThreads - 1) / kThreads, 1);
   const int rb = kBicgBlocks;
   const float tol = 1.1920929e-07f;
-  double hs[2][S_END];
+  double hs[2][64];
   auto pull = [&]() -> cudaError_t {
-    for (int a = 0; a < 2; a++) {
+    for (int a = 0; a < nsys; a++) {
       cudaError_t e = cudaMemcpyAsync(hs[a], P.a[a].S, sizeof hs[a], cudaMemcpyDeviceToHost, st);
       if (e != cudaSuccess) return e;
     }
     return cudaStreamSynchronize(st);
   };
-  auto restart = [&](int a, bool first) {
-    // too orthogonal to r0: restart from the current residual (that system alone)
-    const SysDev &q = P.a[a];
-    spmv_launch(form, eb, st, A[a], q.x, ax_of(a), q.S, kAlways);
-    k_residual<<<eb, kThreads, 0, st>>>(n, b[a], ax_of(a), q.r, q.r0, q.S, kAlways);
-    k_dots<<<rb, kThreads, 0, st>>>(n, q.r, q.r, nullptr, nullptr, nullptr, nullptr, q.part, q.S, kAlways, -1, q.ticket);
-    k_scalar<<<1, kThreads, 0, st>>>(q.part, rb, q.S, 4, 0, kAlways);
-    k_restart_done<<<1, 1, 0, st>>>(q.S, first ? 1 : 0);
-  };
   cudaError_t e;
-  // each system's start, as the single solve takes it
-  for (int a = 0; a < 2; a++) {
+  for (int a = 0; a < nsys; a++) {
     const SysDev &q = P.a[a];
-    spmv_launch(form, eb, st, A[a], q.x, ax_of(a), q.S, kAlways);
-    k_residual<<<eb, kThreads, 0, st>>>(n, b[a], ax_of(a), q.r, q.r0, q.S, kAlways);
-    cudaMemsetAsync(q.ticket, 0, sizeof(unsigned int), st);
-    k_dots<<<rb, kThreads, 0, st>>>(n, q.r0, q.r0, b[a], b[a], q.r0, q.r, q.part, q.S, kAlways, -1, q.ticket);
-    k_scalar<<<1, kThreads, 0, st>>>(q.part, rb, q.S, 0, S_R0SQ, kAlways);
+    spmv_launch(form, st, A[a], q.x, ax_of(a));
+    k_residual<<<eb, kThreads, 0, st>>>(n, b[a], ax_of(a), q.r, q.r0);
+    k_dots<<<rb, kThreads, 0, st>>>(n, q.r0, q.r0, b[a], b[a], q.r0, q.r, q.part);
+    k_scalar<<<1, kThreads, 0, st>>>(q.part, rb, q.S, 0);  // S_R0SQ, S_BB, then dot(r0, r) in S[S_COUNT]
   }
   if ((e = pull()) != cudaSuccess) return e;
   double rhs_sqnorm[2];
-  bool live[2];
-  for (int a = 0; a < 2; a++) {
+  bool live[2] = {false, false};
+  for (int a = 0; a < nsys; a++) {
     const SysDev &q = P.a[a];
     rhs_sqnorm[a] = hs[a][S_BB];
     live[a] = rhs_sqnorm[a] != 0.0;
@@ -834,46 +937,42 @@ cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], floa
       out[a].converged = true;
       continue;
     }
-    k_scal_init<<<1, 1, 0, st>>>(q.S);
-    cudaMemsetAsync(q.v, 0, (size_t)n * sizeof(float), st);
-    cudaMemsetAsync(q.p, 0, (size_t)n * sizeof(float), st);
+    if ((e = cudaMemsetAsync(q.v, 0, (size_t)n * sizeof(float), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(q.p, 0, (size_t)n * sizeof(float), st)) != cudaSuccess) return e;
     double tol2 = (double)tol * (double)tol * rhs_sqnorm[a];
     double eps2 = (double)tol * (double)tol;
     k_loop_init<<<1, 1, 0, st>>>(q.S, tol2, eps2, max_iters);
   }
   if (!live[0] && !live[1]) return cudaGetLastError();
-  // both systems' iterations in each launch; the bound on batches is the single solve's
-  const int64_t max_batches = 2 * (int64_t)max_iters + 3;
-  int64_t batches = 0;
+  // Every iteration counts one and only the first restart sets the count back, so a system
+  // ends within 2 max_iters + 1 iterations; a launch whose systems wait for a restart holds
+  // until the host has run it, and every launch but the last runs at least one iteration.
+  const int64_t max_launches = 2 * (2 * (int64_t)max_iters + 3);
+  int64_t n_launches = 0;
   int restarts[2] = {0, 0};
-  const dim3 ge(eb, 2), gr(rb, 2), gv((unsigned)vec_blocks(n), 2);
-  const dim3 gs((unsigned)std::max<int64_t>({sliced_blocks(n, A[0].sl_long), sliced_blocks(n, A[1].sl_long), 1}), 2);
   for (;;) {
-    const int f = tune ? kSpmvTiled + tune->start(st) : form;  // the tuner's candidates: tiled, sliced
-    for (int k = 0; k < kBicgBatch; k++) {
-      CK_LAUNCH(chained(k2_update_p, gv, st, P));
-      for (int sel = 0; sel < 2; sel++) {
-        if (f == kSpmvSliced)
-          CK_LAUNCH(chained(k2_spmv_sliced, gs, st, P, sel));
-        else if (f == kSpmvTiled)
-          CK_LAUNCH(chained(k2_spmv_tiled, ge, st, P, sel));
-        else
-          CK_LAUNCH(chained(k2_spmv_rows, ge, st, P, sel));
-        CK_LAUNCH(chained(k2_dots, gr, st, P, sel));
-        if (sel == 0) CK_LAUNCH(chained(k2_update_s, gv, st, P));
-      }
-      CK_LAUNCH(chained(k2_update_xr, gr, st, P));
-    }
-    if (tune) tune->stop(st);
+    if ((e = solve_launch(form, P, nsys, st)) != cudaSuccess) return e;
     if ((e = pull()) != cudaSuccess) return e;
-    // a batch counts for the tuner when both systems ran all of it
-    if (tune) tune->finish(hs[0][S_STATE] == kIterate && hs[1][S_STATE] == kIterate);
-    if (hs[0][S_STATE] == kEnded && hs[1][S_STATE] == kEnded) break;
-    if (++batches > max_batches) return cudaErrorUnknown;  // cannot happen: the single solve's count
-    for (int a = 0; a < 2; a++)
-      if (hs[a][S_STATE] == kRestart) restart(a, restarts[a]++ == 0);
+    bool ended = true;
+    for (int a = 0; a < nsys; a++) {
+      if (hs[a][S_ERROR] != 0.0) return cudaErrorLaunchTimeout;  // a barrier's wait ran out (its word is never set otherwise)
+      ended = ended && hs[a][S_STATE] == kEnded;
+    }
+    if (ended) break;
+    if (++n_launches > max_launches) return cudaErrorUnknown;  // cannot happen: the count above
+    for (int a = 0; a < nsys; a++) {
+      if (hs[a][S_STATE] != kRestart) continue;
+      // too orthogonal to r0: restart from the current residual (that system alone)
+      const SysDev &q = P.a[a];
+      spmv_launch(form, st, A[a], q.x, ax_of(a));
+      k_residual<<<eb, kThreads, 0, st>>>(n, b[a], ax_of(a), q.r, q.r0);
+      k_dots<<<rb, kThreads, 0, st>>>(n, q.r, q.r, nullptr, nullptr, nullptr, nullptr, q.part);
+      k_scalar<<<1, kThreads, 0, st>>>(q.part, rb, q.S, 4);
+      k_restart_done<<<1, 1, 0, st>>>(q.S, restarts[a] == 0 ? 1 : 0);
+      restarts[a]++;
+    }
   }
-  for (int a = 0; a < 2; a++) {
+  for (int a = 0; a < nsys; a++) {
     if (!live[a]) continue;
     out[a].iterations = (int)hs[a][S_I];
     out[a].error = (float)std::sqrt(hs[a][S_RR] / rhs_sqnorm[a]);
@@ -882,11 +981,14 @@ cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], floa
   return cudaGetLastError();
 }
 
+cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t st, BicgResult *out) { return solve_systems(1, &A, &b, &x, max_iters, &scratch, st, out, kSpmvTiled); }
+
+cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], float *const x[2], int max_iters, void *const scratch[2], cudaStream_t st, BicgResult out[2], int form) { return solve_systems(2, A, b, x, max_iters, scratch, st, out, form); }
 
 // Loads this file's module (the driver loads a module at its first launch otherwise).
 void load_module_bicgstab() {
   cudaFuncAttributes a;
-  cudaFuncGetAttributes(&a, k2_update_xr);
+  cudaFuncGetAttributes(&a, k_solve<kSpmvSliced>);
 }
 
 }  // namespace gpl

@@ -6,9 +6,8 @@
 
 namespace gpl {
 
-class Tuner;
-
-constexpr int kBicgBlocks = 296;  // two blocks per SM for the reductions
+constexpr int kBicgParts = 4;     // columns of partials
+constexpr int kBicgBlocks = 296;  // the partials of an inner product (fixed: they set its order)
 
 // Rows per slice of the sliced copy of a matrix (below).
 constexpr int kSliceRows = 32;
@@ -57,17 +56,15 @@ cudaError_t csr_slice_widths(int64_t n, int64_t n_long, const int32_t *len, int6
 cudaError_t csr_slice_fill(const CsrDev &A, int2 *sl_ent, cudaStream_t s);
 // Scratch the solve needs (seven vectors of n floats, the partials and the scalars).
 size_t bicgstab_scratch_bytes(int64_t n);
-// Solve A x = b from the start point in x; `scratch` holds bicgstab_scratch_bytes(n) bytes.
-cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t s, BicgResult *out, int spmv = kSpmvRows);
+// Solve A x = b from the start point in x; `scratch` holds bicgstab_scratch_bytes(n) bytes
+// (256-byte aligned). The tiled form: no copy of the matrix, any row length.
+cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t s, BicgResult *out);
 // y = A x in the given form (SpmvForm).
 cudaError_t spmv(const CsrDev &A, const float *x, float *y, int form, cudaStream_t s);
 // Two systems of the same size solved side by side (each launch carries both): each takes
 // the steps of bicgstab_solve on its own; scratch[a] holds bicgstab_pair_scratch_bytes(n)
-// bytes for system a.
+// bytes for system a. The sliced form needs the systems' sliced copies.
 size_t bicgstab_pair_scratch_bytes(int64_t n);
-// With `tune` (two candidates: the tiled and the sliced form), each batch of iterations runs
-// the form the tuner picks (A then needs its sliced copy), timed in place; `spmv` is then the
-// form of the start and restarts.
-cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], float *const x[2], int max_iters, void *const scratch[2], cudaStream_t s, BicgResult out[2], int spmv = kSpmvRows, Tuner *tune = nullptr);
+cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], float *const x[2], int max_iters, void *const scratch[2], cudaStream_t s, BicgResult out[2], int form);
 
 }  // namespace gpl
