@@ -107,9 +107,175 @@ __global__ void __launch_bounds__(256) k_gemm_tn(GemmBatchT<T> gb) {
   gemm_tile<T>(P, m0, n0);
 }
 
+// ---------------------------------------------------------------- FP32, spread over the SMs
+// BM x BN output tile per block, K in chunks of 32 through two shared buffers (the next chunk's
+// loads in flight beside the current one's products), TM x 4 outputs a thread, pairs of rows in
+// one packed FMA. Each output is one chain of fused multiply-adds over k in order, whatever the
+// tile, so every shape gives the same bits.
+constexpr int FG_BK = 32;
+
+// The second GEMM's output taken through the spectral step (src/nesterov.rs:425-440) where it
+// is formed: phi = Ah / (wx2 + wy2), Ex = phi wx, Ey = phi wy, zero at (0, 0). wx NULL: none.
+struct GemmEpi {
+  const float *wx, *wx2, *wy, *wy2;
+  float *exh, *eyh;
+};
+
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+
+// One operand's chunk: `rows` of 32 k values, four at a time; element (r, k) sits at
+// [k][(r / 4 ^ k / 4) * 4 + r % 4], so the transposing stores of a warp and the 16-byte reads
+// along r meet no bank conflict.
+template <int R, int NT>
+struct Chunk {
+  static constexpr int V = R * FG_BK / 4 / NT;
+  float4 v[V];
+  __device__ __forceinline__ void load(const float *__restrict__ A, int lda, int r0, int rows, int k0, int K, bool vec) {
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+      const int e = threadIdx.x + i * NT, r = r0 + e / (FG_BK / 4), k = k0 + e % (FG_BK / 4) * 4;
+      v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r >= rows) continue;
+      const float *p = A + (size_t)r * lda + k;
+      if (vec) {
+        if (k < K) v[i] = *reinterpret_cast<const float4 *>(p);
+      } else {
+        if (k < K) v[i].x = p[0];
+        if (k + 1 < K) v[i].y = p[1];
+        if (k + 2 < K) v[i].z = p[2];
+        if (k + 3 < K) v[i].w = p[3];
+      }
+    }
+  }
+  __device__ __forceinline__ void store(float *s) const {
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+      const int e = threadIdx.x + i * NT, r = e / (FG_BK / 4), k4 = e % (FG_BK / 4);
+      float *p = s + k4 * 4 * R + ((r >> 2) ^ k4) * 4 + (r & 3);
+      p[0] = v[i].x;
+      p[R] = v[i].y;
+      p[2 * R] = v[i].z;
+      p[3 * R] = v[i].w;
+    }
+  }
+};
+
+template <int BM, int BN, int TM>
+__device__ __forceinline__ void gemm_tile_f32(const GemmProblem &P, const GemmEpi &E, const int m0, const int n0) {
+  static_assert(BM % 32 == 0 && BN % 32 == 0 && TM % 4 == 0, "the chunks' layout");
+  constexpr int NT = (BM / TM) * (BN / 4);
+  __shared__ __align__(16) float As[2][FG_BK * BM];
+  __shared__ __align__(16) float Bs[2][FG_BK * BN];
+  const int tx = threadIdx.x % (BN / 4), ty = threadIdx.x / (BN / 4);
+  const bool vec = ((P.K | P.lda | P.ldb) & 3) == 0 && (((uintptr_t)P.A | (uintptr_t)P.B) & 15) == 0;
+  unsigned long long acc[TM / 2][4];
+#pragma unroll
+  for (int i = 0; i < TM / 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+  Chunk<BM, NT> ca;
+  Chunk<BN, NT> cb;
+  ca.load(P.A, P.lda, m0, P.M, 0, P.K, vec);
+  cb.load(P.B, P.ldb, n0, P.N, 0, P.K, vec);
+  int buf = 0;
+  for (int k0 = 0; k0 < P.K; k0 += FG_BK) {
+    ca.store(As[buf]);
+    cb.store(Bs[buf]);
+    __syncthreads();
+    if (k0 + FG_BK < P.K) {
+      ca.load(P.A, P.lda, m0, P.M, k0 + FG_BK, P.K, vec);
+      cb.load(P.B, P.ldb, n0, P.N, k0 + FG_BK, P.K, vec);
+    }
+    const float *as = As[buf], *bs = Bs[buf];
+#pragma unroll
+    for (int kk = 0; kk < FG_BK; kk++) {
+      unsigned long long a[TM / 2], b[4];
+#pragma unroll
+      for (int g = 0; g < TM / 4; g++) {
+        const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(as + kk * BM + (((ty * TM / 4 + g) ^ (kk >> 2)) * 4));
+        a[2 * g] = q.x;
+        a[2 * g + 1] = q.y;
+      }
+      const float4 bv = *reinterpret_cast<const float4 *>(bs + kk * BN + ((tx ^ (kk >> 2)) * 4));
+      b[0] = pack2(bv.x, bv.x);
+      b[1] = pack2(bv.y, bv.y);
+      b[2] = pack2(bv.z, bv.z);
+      b[3] = pack2(bv.w, bv.w);
+#pragma unroll
+      for (int i = 0; i < TM / 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fma2(a[i], b[j], acc[i][j]);
+    }
+    buf ^= 1;
+  }
+  const int n = n0 + tx * 4;
+  if (n >= P.N) return;
+  const bool vs = n + 4 <= P.N && (P.ldd & 3) == 0 && (((uintptr_t)P.D | (uintptr_t)E.exh | (uintptr_t)E.eyh) & 15) == 0;
+  auto put = [&](float *D, int m, const float *v) {
+    float *p = D + (size_t)m * P.ldd + n;
+    if (vs) {
+      *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (n + j < P.N) p[j] = v[j];
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < TM; i++) {
+    const int m = m0 + ty * TM + i;
+    if (m >= P.M) break;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      float lo, hi;
+      unpack2(acc[i >> 1][j], lo, hi);
+      v[j] = (i & 1) ? hi : lo;
+    }
+    if (!E.wx) {
+      put(P.D, m, v);
+      continue;
+    }
+    const float wx = E.wx[m], wx2 = E.wx2[m];
+    float ex[4], ey[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      ex[j] = ey[j] = 0.0f;
+      if (n + j < P.N && (m != 0 || n + j != 0)) {
+        const float p = __fdiv_rn(v[j], __fadd_rn(wx2, E.wy2[n + j]));
+        ex[j] = __fmul_rn(p, wx);
+        ey[j] = __fmul_rn(p, E.wy[n + j]);
+      }
+    }
+    put(E.exh, m, ex);
+    put(E.eyh, m, ey);
+  }
+}
+
+template <int BM, int BN, int TM>
+__global__ void __launch_bounds__((BM / TM) * (BN / 4)) k_gemm_f32(GemmBatch gb, GemmEpi E) {
+  chain_enter();
+  const GemmProblem P = gb.p[blockIdx.z];
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  if (m0 >= P.M || n0 >= P.N) return;
+  gemm_tile_f32<BM, BN, TM>(P, E, m0, n0);
+}
+
 // Many problems in one launch: block b takes tile b - first[k] of problem k (the last with
-// first[k] <= b), tiles row-major over the problem's (M / 128) x (N / 64) grid.
-__global__ void __launch_bounds__(256) k_gemm_grouped(const GemmProblem *__restrict__ probs, const int *__restrict__ first, int n) {
+// first[k] <= b), tiles row-major over the problem's grid; epis NULL: no spectral step.
+template <int BM, int BN, int TM>
+__global__ void __launch_bounds__((BM / TM) * (BN / 4)) k_gemm_grouped(const GemmProblem *__restrict__ probs, const GemmEpi *__restrict__ epis, const int *__restrict__ first, int n) {
+  chain_enter();
   __shared__ int s_k;
   if (threadIdx.x == 0) {
     int lo = 0, hi = n - 1;
@@ -121,9 +287,10 @@ __global__ void __launch_bounds__(256) k_gemm_grouped(const GemmProblem *__restr
   }
   __syncthreads();
   const GemmProblem P = probs[s_k];
+  const GemmEpi E = epis ? epis[s_k] : GemmEpi{};
   const int t = (int)blockIdx.x - first[s_k];
-  const int tn = (P.N + SG_BN - 1) / SG_BN;
-  gemm_tile<float>(P, (t / tn) * SG_BM, (t % tn) * SG_BN);
+  const int tn = (P.N + BN - 1) / BN;
+  gemm_tile_f32<BM, BN, TM>(P, E, (t / tn) * BM, (t % tn) * BN);
 }
 
 template <typename T>
@@ -137,26 +304,28 @@ cudaError_t gemm_tn(const GemmBatchT<T> &gb, int count, cudaStream_t s) {
   k_gemm_tn<T><<<grid, 256, 0, s>>>(gb);
   return cudaGetLastError();
 }
-cudaError_t sgemm_tn(const GemmBatch &gb, int count, cudaStream_t s) { return gemm_tn<float>(gb, count, s); }
+
+// One stage of the FP32 solve.
+template <int BM, int BN, int TM>
+static cudaError_t gemm_f32_launch(const GemmBatch &gb, int count, const GemmEpi &E, cudaStream_t s) {
+  int M = 0, N = 0;
+  for (int i = 0; i < count; i++) {
+    M = std::max(M, gb.p[i].M);
+    N = std::max(N, gb.p[i].N);
+  }
+  return launch_chained(k_gemm_f32<BM, BN, TM>, dim3((N + BN - 1) / BN, (M + BM - 1) / BM, count), dim3((BM / TM) * (BN / 4)), 0, s, gb, E);
+}
+// 128 x 64 tiles once they give nearly every SM one (a 1024 x 1024 solve 334 us, 388 with
+// 64 x 32, 640 with the unpacked 128 x 64 tile before); below that 64 x 32 tiles, so a small
+// grid's products spread over the chip (512 x 512 80 us, 126 with 128 x 64; 64 x 64 8 blocks
+// instead of one).
+static cudaError_t gemm_f32(const GemmBatch &gb, int count, const GemmEpi &E, cudaStream_t s) {
+  const GemmProblem &P = gb.p[0];
+  if ((int64_t)((P.M + 127) / 128) * ((P.N + 63) / 64) >= 128) return gemm_f32_launch<128, 64, 8>(gb, count, E, s);
+  return gemm_f32_launch<64, 32, 4>(gb, count, E, s);
+}
 cudaError_t dgemm_tn(const GemmBatchT<double> &gb, int count, cudaStream_t s) { return gemm_tn<double>(gb, count, s); }
 
-// ---------------------------------------------------------------- the spectral step
-// (src/nesterov.rs:425-440) on the scaled forward transform: phi = Ah / (wx2 + wy2),
-// Ex = phi wx, Ey = phi wy, in float as the reference; all three zero at (0, 0).
-__global__ void k_spectral(int nx, int ny, const float *__restrict__ ah, const float *__restrict__ wx, const float *__restrict__ wx2, const float *__restrict__ wy, const float *__restrict__ wy2, float *__restrict__ exh, float *__restrict__ eyh) {
-  int64_t n = (int64_t)nx * ny;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
-    int u = (int)(k / ny), v = (int)(k % ny);
-    float ex = 0.0f, ey = 0.0f;
-    if (u != 0 || v != 0) {
-      float p = __fdiv_rn(ah[k], __fadd_rn(wx2[u], wy2[v]));
-      ex = __fmul_rn(p, wx[u]);
-      ey = __fmul_rn(p, wy[v]);
-    }
-    exh[k] = ex;
-    eyh[k] = ey;
-  }
-}
 // The FP64 yardstick's spectral step: the same in double (wavenumbers widened from float).
 __global__ void k_spectral_d(int nx, int ny, const double *__restrict__ ah, const float *__restrict__ wx, const float *__restrict__ wy, double *__restrict__ exh, double *__restrict__ eyh) {
   int64_t n = (int64_t)nx * ny;
@@ -220,7 +389,7 @@ static cudaError_t upload_f32(const std::vector<double> &h, float **d) {
 size_t poisson_workspace_bytes(int nx, int ny) {
   size_t n = (size_t)nx * ny;
   size_t basis = 3 * (size_t)nx * nx + 3 * (size_t)ny * ny;
-  return (basis + 6 * n) * sizeof(float) + 2 * (size_t)(nx + ny) * sizeof(float);
+  return (basis + 5 * n) * sizeof(float) + 2 * (size_t)(nx + ny) * sizeof(float);
 }
 
 PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const float *wy_host, int mode, cudaError_t *err) {
@@ -272,7 +441,6 @@ PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const flo
     TRY(upload_f32(b.Sx, &p->Sx));
     TRY(upload_f32(b.Cx, &p->Cx));
     TRY(pool_alloc((void **)&p->t1, n * sizeof(float)));
-    TRY(pool_alloc((void **)&p->ah, n * sizeof(float)));
     TRY(pool_alloc((void **)&p->exh, n * sizeof(float)));
     TRY(pool_alloc((void **)&p->eyh, n * sizeof(float)));
     TRY(pool_alloc((void **)&p->t2, n * sizeof(float)));
@@ -297,7 +465,7 @@ PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const flo
 void poisson_plan_destroy(PoissonPlan *p) {
   if (!p) return;
   cudaDeviceSynchronize();
-  float *bufs[] = {p->wx, p->wx2, p->wy, p->wy2, p->CyTs, p->CxTs, p->Cy, p->Sy, p->Sx, p->Cx, p->t1, p->ah, p->exh, p->eyh, p->t2, p->t3};
+  float *bufs[] = {p->wx, p->wx2, p->wy, p->wy2, p->CyTs, p->CxTs, p->Cy, p->Sy, p->Sx, p->Cx, p->t1, p->exh, p->eyh, p->t2, p->t3};
   for (float *b : bufs)
     pool_free(b);
   for (double *b : p->d_basis)
@@ -335,7 +503,7 @@ cudaError_t poisson_split_density(PoissonPlan *p, const float *density, cudaStre
 
 int poisson_plan_mode(const PoissonPlan *p) { return p->mode; }
 
-int poisson_launches(const PoissonPlan *p) { return p->mode == 0 ? 5 : p->mode == 2 ? 9 : tc_launches(p); }
+int poisson_launches(const PoissonPlan *p) { return p->mode == 0 ? 4 : p->mode == 2 ? 9 : tc_launches(p); }
 
 // The FP64 form: the density widened to double, the FP32 form's six GEMMs and spectral step
 // in double throughout, the fields rounded to float once at the end. The yardstick the
@@ -367,55 +535,23 @@ static cudaError_t solve_fp64(PoissonPlan *p, const float *density, float *field
 }
 
 // ---------------------------------------------------------------- many FP32 solves at once
-// The FP32 solves of several regions (each its own grid) as five launches: each GEMM stage
-// over every region's problems, the spectral step over every region's spectrum. Each
-// problem's tiles are those poisson_solve computes, so every field is the same bit for bit.
-struct SpectralJob {
-  int nx, ny, first, blocks;
-  const float *ah, *wx, *wx2, *wy, *wy2;
-  float *exh, *eyh;
-};
-__global__ void k_spectral_grouped(const SpectralJob *__restrict__ jobs, int n) {
-  __shared__ int s_k;
-  if (threadIdx.x == 0) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (jobs[mid].first <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-    }
-    s_k = lo;
-  }
-  __syncthreads();
-  const SpectralJob J = jobs[s_k];
-  const int64_t cnt = (int64_t)J.nx * J.ny;
-  for (int64_t k = ((int64_t)blockIdx.x - J.first) * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)J.blocks * blockDim.x) {
-    int u = (int)(k / J.ny), v = (int)(k % J.ny);
-    float ex = 0.0f, ey = 0.0f;
-    if (u != 0 || v != 0) {
-      float p = __fdiv_rn(J.ah[k], __fadd_rn(J.wx2[u], J.wy2[v]));
-      ex = __fmul_rn(p, J.wx[u]);
-      ey = __fmul_rn(p, J.wy[v]);
-    }
-    J.exh[k] = ex;
-    J.eyh[k] = ey;
-  }
-}
-
+// The FP32 solves of several regions (each its own grid) as four launches, each GEMM stage
+// over every region's problems; every field is poisson_solve's bit for bit.
+constexpr int kGroupTile = 32;
 struct PoissonGroup {
-  // per stage: problems and each one's first tile; the spectral jobs
+  // per stage: problems and each one's first tile; the second stage's spectral steps
   GemmProblem *probs[4] = {};
   int *first[4] = {};
   int count[4] = {}, tiles[4] = {};
-  SpectralJob *jobs = nullptr;
-  int n_jobs = 0, job_blocks = 0;
+  GemmEpi *epis = nullptr;
+  int regions = 0;
 };
 
 PoissonGroup *poisson_group_create(PoissonPlan *const *plans, const float *const *density, float *const *field_x, float *const *field_y, int n, cudaError_t *err) {
   *err = cudaSuccess;
   PoissonGroup *g = new PoissonGroup();
   std::vector<GemmProblem> st[4];
-  std::vector<SpectralJob> jobs;
-  int jb = 0;
+  std::vector<GemmEpi> epis;
   for (int k = 0; k < n; k++) {
     PoissonPlan *p = plans[k];
     if (p->mode != 0) {
@@ -425,15 +561,12 @@ PoissonGroup *poisson_group_create(PoissonPlan *const *plans, const float *const
     }
     const int nx = p->nx, ny = p->ny;
     st[0].push_back(GemmProblem{ny, nx, ny, p->CyTs, ny, density[k], ny, p->t1, nx});
-    st[1].push_back(GemmProblem{nx, ny, nx, p->CxTs, nx, p->t1, nx, p->ah, ny});
+    st[1].push_back(GemmProblem{nx, ny, nx, p->CxTs, nx, p->t1, nx, nullptr, ny});
     st[2].push_back(GemmProblem{ny, nx, ny, p->Cy, ny, p->exh, ny, p->t2, nx});
     st[2].push_back(GemmProblem{ny, nx, ny, p->Sy, ny, p->eyh, ny, p->t3, nx});
     st[3].push_back(GemmProblem{nx, ny, nx, p->Sx, nx, p->t2, nx, field_x[k], ny});
     st[3].push_back(GemmProblem{nx, ny, nx, p->Cx, nx, p->t3, nx, field_y[k], ny});
-    const int64_t cells = (int64_t)nx * ny;
-    const int blocks = (int)std::min<int64_t>((cells + 255) / 256, 148 * 8);
-    jobs.push_back(SpectralJob{nx, ny, jb, blocks, p->ah, p->wx, p->wx2, p->wy, p->wy2, p->exh, p->eyh});
-    jb += blocks;
+    epis.push_back(GemmEpi{p->wx, p->wx2, p->wy, p->wy2, p->exh, p->eyh});
   }
   auto put = [&](auto **d, const auto &v) {
     if (*err != cudaSuccess || v.empty()) return;
@@ -446,16 +579,15 @@ PoissonGroup *poisson_group_create(PoissonPlan *const *plans, const float *const
     int t = 0;
     for (const GemmProblem &P : st[q]) {
       first.push_back(t);
-      t += ((P.M + SG_BM - 1) / SG_BM) * ((P.N + SG_BN - 1) / SG_BN);
+      t += ((P.M + kGroupTile - 1) / kGroupTile) * ((P.N + kGroupTile - 1) / kGroupTile);
     }
     g->count[q] = (int)st[q].size();
     g->tiles[q] = t;
     put(&g->probs[q], st[q]);
     put(&g->first[q], first);
   }
-  g->n_jobs = (int)jobs.size();
-  g->job_blocks = jb;
-  put(&g->jobs, jobs);
+  g->regions = n;
+  put(&g->epis, epis);
   if (*err == cudaSuccess) *err = cudaStreamSynchronize(0);
   if (*err != cudaSuccess) {
     poisson_group_destroy(g);
@@ -471,48 +603,45 @@ void poisson_group_destroy(PoissonGroup *g) {
     pool_free(g->probs[q]);
     pool_free(g->first[q]);
   }
-  pool_free(g->jobs);
+  pool_free(g->epis);
   delete g;
 }
 
 cudaError_t poisson_group_solve(const PoissonGroup *g, cudaStream_t s) {
-  if (!g || g->n_jobs == 0) return cudaSuccess;
-  for (int q = 0; q < 4; q++) {
-    k_gemm_grouped<<<g->tiles[q], 256, 0, s>>>(g->probs[q], g->first[q], g->count[q]);
-    if (q == 1) k_spectral_grouped<<<g->job_blocks, 256, 0, s>>>(g->jobs, g->n_jobs);
-  }
-  return cudaGetLastError();
+  if (!g || g->regions == 0) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  for (int q = 0; q < 4 && e == cudaSuccess; q++)
+    e = launch_chained(k_gemm_grouped<kGroupTile, kGroupTile, 4>, dim3(g->tiles[q]), dim3(kGroupTile * kGroupTile / 16), 0, s, (const GemmProblem *)g->probs[q],
+                       (const GemmEpi *)(q == 1 ? g->epis : nullptr), (const int *)g->first[q], g->count[q]);
+  return e;
 }
 
-int poisson_group_launches(const PoissonGroup *g) { return g && g->n_jobs ? 5 : 0; }
+int poisson_group_launches(const PoissonGroup *g) { return g && g->regions ? 4 : 0; }
 
 cudaError_t poisson_solve(PoissonPlan *p, const float *density, float *field_x, float *field_y, cudaStream_t s) {
   if (p->mode == 2) return solve_fp64(p, density, field_x, field_y, s);
   if (p->mode != 0) return tc_solve(p, field_x, field_y, s);
   int nx = p->nx, ny = p->ny;
+  const GemmEpi none{}, spectral{p->wx, p->wx2, p->wy, p->wy2, p->exh, p->eyh};
   GemmBatch g{};
   g.p[0] = GemmProblem{ny, nx, ny, p->CyTs, ny, density, ny, p->t1, nx};
-  cudaError_t e = sgemm_tn(g, 1, s);
+  cudaError_t e = gemm_f32(g, 1, none, s);
   if (e != cudaSuccess) return e;
-  g.p[0] = GemmProblem{nx, ny, nx, p->CxTs, nx, p->t1, nx, p->ah, ny};
-  if ((e = sgemm_tn(g, 1, s)) != cudaSuccess) return e;
-  int64_t n = (int64_t)nx * ny;
-  int blocks = (int)std::min<int64_t>((n + 255) / 256, 148 * 8);
-  k_spectral<<<blocks, 256, 0, s>>>(nx, ny, p->ah, p->wx, p->wx2, p->wy, p->wy2, p->exh, p->eyh);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  g.p[0] = GemmProblem{nx, ny, nx, p->CxTs, nx, p->t1, nx, nullptr, ny};
+  if ((e = gemm_f32(g, 1, spectral, s)) != cudaSuccess) return e;
   g.p[0] = GemmProblem{ny, nx, ny, p->Cy, ny, p->exh, ny, p->t2, nx};
   g.p[1] = GemmProblem{ny, nx, ny, p->Sy, ny, p->eyh, ny, p->t3, nx};
-  if ((e = sgemm_tn(g, 2, s)) != cudaSuccess) return e;
+  if ((e = gemm_f32(g, 2, none, s)) != cudaSuccess) return e;
   g.p[0] = GemmProblem{nx, ny, nx, p->Sx, nx, p->t2, nx, field_x, ny};
   g.p[1] = GemmProblem{nx, ny, nx, p->Cx, nx, p->t3, nx, field_y, ny};
-  return sgemm_tn(g, 2, s);
+  return gemm_f32(g, 2, none, s);
 }
 
 
 // Loads this file's module (the driver loads a module at its first launch otherwise).
 void load_module_poisson() {
   cudaFuncAttributes a;
-  cudaFuncGetAttributes(&a, k_gemm_grouped);
+  cudaFuncGetAttributes(&a, k_gemm_grouped<kGroupTile, kGroupTile, 4>);
 }
 
 }  // namespace gpl

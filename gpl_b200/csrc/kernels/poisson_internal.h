@@ -25,7 +25,6 @@ struct GemmBatchT {
 };
 using GemmProblem = GemmProblemT<float>;
 using GemmBatch = GemmBatchT<float>;
-cudaError_t sgemm_tn(const GemmBatch &gb, int count, cudaStream_t s);
 cudaError_t dgemm_tn(const GemmBatchT<double> &gb, int count, cudaStream_t s);
 
 // The six basis matrices in double (see poisson.cu): CyTs[v][y], CxTs[u][x] (forward, scaled
@@ -52,7 +51,7 @@ struct PoissonPlan {
   float *wx = nullptr, *wx2 = nullptr, *wy = nullptr, *wy2 = nullptr;
   // FP32 path
   float *CyTs = nullptr, *CxTs = nullptr, *Cy = nullptr, *Sy = nullptr, *Sx = nullptr, *Cx = nullptr;
-  float *t1 = nullptr, *ah = nullptr, *exh = nullptr, *eyh = nullptr, *t2 = nullptr, *t3 = nullptr;
+  float *t1 = nullptr, *exh = nullptr, *eyh = nullptr, *t2 = nullptr, *t3 = nullptr;
   // tensor-core path
   __nv_bfloat16 *tc_dens = nullptr;  // density as [nx][2*ny] bf16 (hi | lo)
   TcState *tc = nullptr;
