@@ -160,7 +160,7 @@ int gpl_kernel_gradients(int64_t n_cells, const int32_t *centre, const int32_t *
   e = cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s);
   if (e == cudaSuccess) {
     k_gradients<<<blocks, kThreadsPerBlock, 0, s>>>(r, c, reinterpret_cast<const float2 *>(pin_force), penalty, reinterpret_cast<float2 *>(sum), reinterpret_cast<const float2 *>(a1),
-                                                    reinterpret_cast<const float2 *>(b1), reinterpret_cast<const float2 *>(b2), partials, ticket, out);
+                                                    reinterpret_cast<const float2 *>(b1), reinterpret_cast<const float2 *>(b2), partials, ticket, out, Publish{});
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(sums, out, 4 * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -285,8 +285,13 @@ int gpl_kernel_wa(int64_t n_nets, const int64_t *net_start, const int32_t *pin_x
     e = d.build(n_nets, net_start, pin_xy, net_weight);
     if (e == cudaSuccess) {
       WaArgs w = d.args(grad);
-      launch_wa_small(w, coef_x, coef_y, 1, s);
-      if (w.n_tiles) launch_wa_tiles(w, coef_x, coef_y, s);
+      // in the engine's launches: joint for few nets
+      if (wa_joint_fits(w.small, w.n_tiles) && !std::getenv("GPL_WA_SMALL")) {
+        launch_wa_joint(w, coef_x, coef_y, s);
+      } else {
+        launch_wa_small(w, coef_x, coef_y, 1, s);
+        if (w.n_tiles) launch_wa_tiles(w, coef_x, coef_y, s);
+      }
       if (w.n_nets) k_wa<<<(unsigned)((w.n_nets + kThreadsPerBlock - 1) / kThreadsPerBlock), kThreadsPerBlock, 0, s>>>(w, coef_x, coef_y);
       e = cudaGetLastError();
     }

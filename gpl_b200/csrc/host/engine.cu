@@ -108,7 +108,7 @@ Engine::Engine(int device) : device_(device) {
 void Engine::join() {
   if (!wa_pending_) return;
   check(cudaStreamWaitEvent(stream_, ev_join_, 0), "join");
-  check(cudaStreamWaitEvent(stream_, ev_join2_, 0), "join");
+  if (wa_split_) check(cudaStreamWaitEvent(stream_, ev_join2_, 0), "join");
   wa_pending_ = false;
 }
 
@@ -171,7 +171,7 @@ static cudaError_t upload_vec(T **p, const std::vector<T, A> &v, cudaStream_t s)
 
 // ---------------------------------------------------------------- Nesterov state
 void Engine::free_globals() {
-  void *ptrs[] = {dc_, hx_, hy_, dscale_, area_, kind_, locked_, cell_pin_start_, net_start_, pin_cell_, pin_slot_, big_nets_, pin_base_, tiles_, net_weight_, pin_grad_, hpwl_acc_, dev_scal_};
+  void *ptrs[] = {dc_, hx_, hy_, dscale_, area_, kind_, locked_, cell_pin_start_, net_start_, pin_cell_, pin_slot_, big_nets_, pin_base_, tiles_, net_weight_, pin_grad_, hpwl_acc_, dev_scal_, pub_count_};
   for (void *p : ptrs)
     if (p) cudaFreeAsync(p, stream_);
   dc_ = nullptr;
@@ -189,6 +189,8 @@ void Engine::free_globals() {
   pin_grad_ = nullptr;
   hpwl_acc_ = nullptr;
   dev_scal_ = nullptr;
+  pub_count_ = nullptr;
+  published_ = hpwl_zeroed_ = false;
 }
 
 void Engine::release() {
@@ -324,16 +326,20 @@ void Engine::upload(const EngineSetup &s) {
   check(dmalloc(&pin_grad_, s.cell_pins.size(), st), "alloc pins");
   check(dmalloc(&hpwl_acc_, 1, st), "alloc");
   check(dmalloc(&dev_scal_, s.regions.size(), st), "alloc");
+  check(dmalloc(&pub_count_, 1, st), "alloc");
+  if (!failed()) check(cudaMemsetAsync(pub_count_, 0, sizeof(unsigned int), st), "memset");
   host_scal_.assign(s.regions.size(), RegionScalars{});
   {
-    size_t need = s.regions.size() * sizeof(RegionScalars) + sizeof(unsigned long long);
+    size_t need = 2 * (s.regions.size() * sizeof(RegionScalars) + sizeof(unsigned long long));
     if (need > pinned_bytes_) {
       if (pinned_) cudaFreeHost(pinned_);
       pinned_ = nullptr;
       pinned_bytes_ = 0;
-      check(cudaHostAlloc((void **)&pinned_, need, cudaHostAllocDefault), "alloc pinned");
+      check(cudaHostAlloc((void **)&pinned_, need, cudaHostAllocMapped), "alloc pinned");
       if (pinned_) pinned_bytes_ = need;
     }
+    // no number of an earlier upload's
+    if (pinned_) std::memset(pinned_, 0, pinned_bytes_);
   }
   region_wx_.clear();
   region_wy_.clear();
@@ -417,6 +423,7 @@ void Engine::upload(const EngineSetup &s) {
 void Engine::update_bins(int b, const RegionSetup &rs) {
   flush();
   join();
+  published_ = false;
   Region *r = regions_[b];
   r->args.target_density = rs.target_density;
   size_t nb = rs.scaled.size();
@@ -432,6 +439,7 @@ void Engine::update_bins(int b, const RegionSetup &rs) {
 void Engine::rewrite_cells(const EngineSetup &s) {
   flush();
   join();
+  published_ = false;
   // sizes and density sizes of every cell (routability's inflation and filler changes keep
   // the cell count of a region's block only when no filler moved; the caller re-uploads then)
   size_t n = s.hx.size();
@@ -471,6 +479,7 @@ static CellArgs cell_args(const int64_t off, int2 *dc, int32_t *hx, int32_t *hy,
 void Engine::set_coords(int b, SlotId slot, const std::vector<float> &xy) {
   flush();
   join();
+  published_ = false;
   Region *r = regions_[b];
   if (r->n_cells) check(cudaMemcpyAsync(r->slot[slot], xy.data(), r->n_cells * sizeof(float2), cudaMemcpyHostToDevice, stream_), "set_coords");
   h2d_bytes += r->n_cells * 8;
@@ -479,6 +488,7 @@ void Engine::set_coords(int b, SlotId slot, const std::vector<float> &xy) {
 std::vector<float> Engine::get_coords(int b, SlotId slot) {
   flush();
   join();
+  published_ = false;
   Region *r = regions_[b];
   std::vector<float> xy(2 * r->n_cells);
   if (r->n_cells) check(cudaMemcpyAsync(xy.data(), r->slot[slot], r->n_cells * sizeof(float2), cudaMemcpyDeviceToHost, stream_), "get_coords");
@@ -499,12 +509,15 @@ void Engine::place_at(int b, SlotId slot) {
   join();
   if (failed()) return;
   hpwl_ready_ = hpwl_fetched_ = false;  // the density centres move
+  published_ = false;
   Region *r = regions_[b];
   CellArgs c = CELLS(r);
   ph_begin(PH_PLACE);
   launches += (r->n_cells ? 1 : 0) + 1;
   RegionArgs a = r->args;
   a.scatter_form = r->scatter_tune->best();
+  a.hpwl_zero = hpwl_acc_;
+  if (r->n_cells) hpwl_zeroed_ = true;
   if (r->n_cells) k_place_cells<<<blocks_for(r->n_cells), kThreadsPerBlock, 0, stream_>>>(a, c, PLACE_AT, 0.0f, 0.0f, r->slot[slot]);
   ph_end(PH_PLACE);
   ph_begin(PH_FINALIZE);
@@ -533,6 +546,7 @@ void Engine::nesterov_step(int b, float step, float coeff) {
     }
   }
   hpwl_ready_ = hpwl_fetched_ = false;  // the density centres move
+  published_ = false;
   Region *r = regions_[b];
   CellArgs c = CELLS(r);
   if (packed()) {
@@ -556,6 +570,8 @@ void Engine::nesterov_step(int b, float step, float coeff) {
   if (r->n_cells) {
     RegionArgs a = r->args;
     a.scatter_form = r->scatter_tune->start(stream_);
+    a.hpwl_zero = hpwl_acc_;
+    hpwl_zeroed_ = true;
     k_place_cells<<<blocks_for(r->n_cells), kThreadsPerBlock, 0, stream_>>>(a, c, PLACE_NESTEROV, step, coeff, nullptr);
     fork_after_place();
     r->scatter_tune->stop(stream_);
@@ -577,11 +593,17 @@ void Engine::field(int b) {
     return;
   }
   Region *r = regions_[b];
+  published_ = false;
   ph_begin(PH_POISSON);
   check(poisson_solve(r->plan, r->density, r->fx, r->fy, stream_), "poisson");
   ph_end(PH_POISSON);
   launches += poisson_launches(r->plan);
 }
+
+// A small design's WA: both parts in one launch, queued before the density solve (two launches
+// on two streams, after the solve's, kept the 294-cell design's trial waiting for the tiles: 53
+// us a trial, 41 in one launch before it). Not when GPL_WA_SMALL asks for another form.
+bool Engine::wa_joint() const { return wa_joint_fits(small_, n_tiles_) && !wa_tune_->fixed(); }
 
 WaArgs Engine::wa_args() const {
   WaArgs w{};
@@ -614,25 +636,34 @@ void Engine::wa(float cx, float cy) {
     check(cudaStreamWaitEvent(wa_stream_, ev_fork_, 0), "wa fork");
   }
   fork_early_ = false;
-  // the kernels add the HPWL of these same positions: hpwl() reads it without a launch
-  check(cudaMemsetAsync(hpwl_acc_, 0, sizeof(unsigned long long), st), "wa");
+  published_ = false;
+  // the kernels add the HPWL of these same positions: hpwl() reads it without a launch (the
+  // scatter has cleared it; a WA again at the same centres clears it itself)
+  if (!hpwl_zeroed_) check(cudaMemsetAsync(hpwl_acc_, 0, sizeof(unsigned long long), st), "wa");
+  hpwl_zeroed_ = false;
   w.hpwl_out = hpwl_acc_;
   hpwl_ready_ = true;
   hpwl_fetched_ = false;
   cudaStream_t st2 = st;
-  if (overlap_) {
+  wa_split_ = overlap_ && !wa_joint();
+  if (wa_split_) {
     check(cudaEventRecord(ev_split_, st), "wa split");
     check(cudaStreamWaitEvent(wa2_stream_, ev_split_, 0), "wa split");
     st2 = wa2_stream_;
   }
   ph_begin(PH_WA, st);
-  if (wa_small_blocks(small_)) {
+  const bool joint = wa_joint();
+  if (joint) {
+    launches += 1;
+    launch_wa_joint(w, cx, cy, st);
+  }
+  if (!joint && wa_small_blocks(small_)) {
     launches += 1;
     const int form = wa_tune_->start(st2);
     launch_wa_small(w, cx, cy, 1, st2, form);
     wa_tune_->stop(st2);
   }
-  if (n_tiles_) {
+  if (!joint && n_tiles_) {
     launches += 1;
     launch_wa_tiles(w, cx, cy, st);
   }
@@ -644,7 +675,7 @@ void Engine::wa(float cx, float cy) {
   check(cudaGetLastError(), "wa");
   if (overlap_) {
     check(cudaEventRecord(ev_join_, st), "wa join");
-    check(cudaEventRecord(ev_join2_, st2), "wa join");
+    if (wa_split_) check(cudaEventRecord(ev_join2_, st2), "wa join");
     wa_pending_ = true;
   }
 }
@@ -678,17 +709,64 @@ void Engine::gradients(int b, SlotId out, float penalty, SlotId a1, SlotId b1, S
   if (r->n_cells) {
     ph_begin(PH_GRAD);
     launches += 1;
-    check(launch_chained(k_gradients, dim3(r->nb_cells), dim3(kThreadsPerBlock), 0, stream_, r->args, c, pin_grad_, penalty, r->slot[out], pa1, pb1, pb2, r->part, r->ticket, &dev_scal_[b].wl_sum), "gradients");
+    const Publish pub = regions_.size() == 1 ? publish(1) : Publish{};
+    check(launch_chained(k_gradients, dim3(r->nb_cells), dim3(kThreadsPerBlock), 0, stream_, r->args, c, pin_grad_, penalty, r->slot[out], pa1, pb1, pb2, r->part, r->ticket, &dev_scal_[b].wl_sum, pub), "gradients");
     ph_end(PH_GRAD);
   } else {
     check(cudaMemsetAsync(&dev_scal_[b].wl_sum, 0, 4 * sizeof(double), stream_), "gradients");
+    published_ = false;
   }
   check(cudaGetLastError(), "gradients");
+}
+
+// What the next gradient update (of `expected` regions) publishes: every region's scalars and
+// the HPWL. Not while phases are timed: their events are read after a synchronisation.
+Publish Engine::publish(int expected) {
+  published_ = false;
+  void *dev = nullptr;
+  if (profile_ || !pinned_ || cudaHostGetDevicePointer(&dev, pinned_, 0) != cudaSuccess) return Publish{};
+  Publish p{};
+  p.scal = reinterpret_cast<const double *>(dev_scal_);
+  p.hpwl = hpwl_acc_;
+  p.host = static_cast<unsigned long long *>(dev);
+  p.count = pub_count_;
+  p.words = (int)(host_scal_.size() * sizeof(RegionScalars) / sizeof(double));
+  p.expected = expected;
+  if (++pub_seq_ == 0) pub_seq_ = 1;
+  p.seq = pub_seq_;
+  published_ = true;
+  return p;
+}
+
+// Waits for the published scalars; false when the stream has run dry without them (a failed
+// launch: the caller's synchronising read reports it).
+bool Engine::wait_published() {
+  const unsigned long long *at = reinterpret_cast<const unsigned long long *>(pinned_);
+  const size_t words = host_scal_.size() * sizeof(RegionScalars) / sizeof(double) + 1;
+  unsigned long long *to = reinterpret_cast<unsigned long long *>(host_scal_.data());
+  bool dry = false;
+  unsigned spins = 0;
+  for (size_t w = 0; w < words;) {
+    const unsigned long long lo = __atomic_load_n(at + 2 * w, __ATOMIC_RELAXED), hi = __atomic_load_n(at + 2 * w + 1, __ATOMIC_RELAXED);
+    if (lo >> 32 == pub_seq_ && hi >> 32 == pub_seq_) {
+      const unsigned long long v = hi << 32 | (lo & 0xffffffffull);
+      if (w + 1 < words)
+        to[w] = v;
+      else
+        hpwl_published_ = v;
+      w++;
+      continue;
+    }
+    if (dry) return false;
+    if ((++spins & 0xffff) == 0) dry = cudaStreamQuery(stream_) != cudaErrorNotReady;  // then one look more
+  }
+  return true;
 }
 
 void Engine::prev_slp(int b, float coef) {
   flush();
   join();
+  published_ = false;
   if (failed()) return;
   Region *r = regions_[b];
   if (!r->n_cells) return;
@@ -699,6 +777,7 @@ void Engine::prev_slp(int b, float coef) {
 void Engine::hold_locked(int b) {
   flush();
   join();
+  published_ = false;
   if (failed() || !any_locked_) return;
   Region *r = regions_[b];
   if (!r->n_cells) return;
@@ -711,6 +790,7 @@ void Engine::swap_slots(int b, SlotId a, SlotId c) { std::swap(regions_[b]->slot
 void Engine::copy_slot(int b, SlotId dst, SlotId src) {
   flush();
   join();
+  published_ = false;
   Region *r = regions_[b];
   if (r->n_cells) check(cudaMemcpyAsync(r->slot[dst], r->slot[src], r->n_cells * sizeof(float2), cudaMemcpyDeviceToDevice, stream_), "copy_slot");
 }
@@ -721,17 +801,21 @@ void Engine::fetch() {
   if (failed() || host_scal_.empty()) return;
   const size_t bytes = host_scal_.size() * sizeof(RegionScalars);
   const bool with_hpwl = hpwl_ready_ && !hpwl_fetched_;
-  check(cudaMemcpyAsync(pinned_, dev_scal_, bytes, cudaMemcpyDeviceToHost, stream_), "fetch");
-  d2h_bytes += (int64_t)bytes;
-  if (with_hpwl) {
-    check(cudaMemcpyAsync(pinned_ + bytes, hpwl_acc_, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_), "fetch");
-    d2h_bytes += (int64_t)sizeof(unsigned long long);
+  d2h_bytes += (int64_t)bytes + (with_hpwl ? (int64_t)sizeof(unsigned long long) : 0);
+  const bool published = published_ && wait_published();
+  published_ = false;
+  if (!published) {
+    check(cudaMemcpyAsync(pinned_, dev_scal_, bytes, cudaMemcpyDeviceToHost, stream_), "fetch");
+    if (with_hpwl) check(cudaMemcpyAsync(pinned_ + bytes, hpwl_acc_, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_), "fetch");
+    check(cudaStreamSynchronize(stream_), "fetch sync");
+    if (failed()) return;
+    std::memcpy(host_scal_.data(), pinned_, bytes);
+    std::memcpy(&hpwl_published_, pinned_ + bytes, sizeof hpwl_published_);
+    // no number of a publish among the copied words
+    std::memset(pinned_, 0, pinned_bytes_);
   }
-  check(cudaStreamSynchronize(stream_), "fetch sync");
-  if (failed()) return;
-  std::memcpy(host_scal_.data(), pinned_, bytes);
   if (with_hpwl) {
-    std::memcpy(&hpwl_host_, pinned_ + bytes, sizeof hpwl_host_);
+    hpwl_host_ = hpwl_published_;
     hpwl_fetched_ = true;
   }
   ph_flush();
@@ -739,7 +823,7 @@ void Engine::fetch() {
   for (Region *r : regions_) r->scatter_tune->finish();
   wa_tune_->finish();
   pk_scatter_tune_->finish();
-  pk_slot_ = 0;  // the stream has drained: every table slot is free
+  pk_slot_ = 0;  // the trial's last launch has ended: every table slot's copy is done
 }
 
 // ---- packed launches
@@ -827,7 +911,12 @@ void Engine::flush_place(const std::vector<QueueEntry> &q, size_t a, size_t b) {
     f.blocks = f.r.nx;  // one block per x row
     fb += f.blocks;
   }
+  if (ns) {
+    h[0].r.hpwl_zero = hpwl_acc_;  // the launch's first block clears the next WA's HPWL
+    hpwl_zeroed_ = true;
+  }
   copy_tables(*this, h, d, ns + n, stream_, h2d_bytes);
+  published_ = false;
   if (ns) {
     k_place_packed<<<blocks, kThreadsPerBlock, 0, stream_>>>(d, ns);
     fork_after_place();
@@ -854,6 +943,7 @@ void Engine::flush_field(const std::vector<QueueEntry> &q, size_t a, size_t b) {
     else
       alone.push_back(q[k].region);
   }
+  published_ = false;
   ph_begin(PH_POISSON);
   if (std::count(set.begin(), set.end(), 1)) {
     if (!group_ || set != group_set_) {
@@ -907,7 +997,7 @@ void Engine::flush_grad(const std::vector<QueueEntry> &q, size_t a, size_t b) {
   if (!n) return;
   copy_tables(*this, h, d, n, stream_, h2d_bytes);
   ph_begin(PH_GRAD);
-  k_gradients_packed<<<blocks, kThreadsPerBlock, 0, stream_>>>(d, n);
+  k_gradients_packed<<<blocks, kThreadsPerBlock, 0, stream_>>>(d, n, publish(n));
   launches += 1;
   ph_end(PH_GRAD);
   check(cudaGetLastError(), "packed gradients");
@@ -935,7 +1025,9 @@ int64_t Engine::hpwl() {
   if (failed()) return 0;
   if (hpwl_ready_ && hpwl_fetched_) return (int64_t)hpwl_host_;  // read with the trial's scalars
   WaArgs w = wa_args();
+  published_ = false;
   if (!hpwl_ready_) {
+  hpwl_zeroed_ = false;
   check(cudaMemsetAsync(hpwl_acc_, 0, sizeof(unsigned long long), stream_), "hpwl");
   ph_begin(PH_HPWL);
   if (wa_small_blocks(small_)) {
@@ -970,6 +1062,7 @@ int64_t Engine::hpwl() {
 void Engine::centres(std::vector<int32_t> &dcx, std::vector<int32_t> &dcy) {
   flush();
   join();
+  published_ = false;
   std::vector<int2> dc(n_cells_);
   if (n_cells_) {
     check(cudaMemcpyAsync(dc.data(), dc_, n_cells_ * sizeof(int2), cudaMemcpyDeviceToHost, stream_), "centres");
@@ -987,6 +1080,7 @@ void Engine::centres(std::vector<int32_t> &dcx, std::vector<int32_t> &dcy) {
 void Engine::set_net_weights(const std::vector<float> &w) {
   flush();
   join();
+  published_ = false;
   if (w.empty()) return;
   if (w.size() != net_order_.size()) {
     check(cudaErrorInvalidValue, "net weights");
@@ -1006,6 +1100,7 @@ void Engine::set_net_weights(const std::vector<float> &w) {
 void Engine::reorder(int b) {
   flush();
   join();
+  published_ = false;
   Region *r = regions_[b];
   const int32_t n = (int32_t)r->n_cells;
   if (failed() || n < 2) return;
@@ -1096,6 +1191,7 @@ void Engine::reorder(int b) {
 bool Engine::take_order(int b, std::vector<int32_t> &order) {
   flush();
   join();
+  published_ = false;
   Region *r = regions_[b];
   if (!r->order_moved || failed()) return false;
   order.resize((size_t)r->n_cells);
@@ -1110,6 +1206,7 @@ bool Engine::take_order(int b, std::vector<int32_t> &order) {
 void Engine::rebuild_poisson(int mode) {
   flush();
   join();
+  published_ = false;
   poisson_mode_ = mode;
   check(cudaStreamSynchronize(stream_), "rebuild sync");
   poisson_group_destroy(group_);

@@ -93,6 +93,7 @@ class Engine {
   void nesterov_step(int b, float step, float coeff);
   void field(int b);
   void wa(float coef_x, float coef_y);
+  bool wa_joint() const;
   // updateGradients into `out` with the penalty; distances |a1 - b1| and |out - b2| (pass
   // S_NUM to skip one).
   void gradients(int b, SlotId out, float penalty, SlotId a1, SlotId b1, SlotId b2);
@@ -183,11 +184,19 @@ class Engine {
   float2 *pin_grad_ = nullptr;  // the WA force of every pin of a cell, cell-major (cell_pins order)
   unsigned long long *hpwl_acc_ = nullptr;
   bool hpwl_ready_ = false;  // hpwl_acc_ holds the HPWL of the current centres (from the WA)
-  // Page-locked read-back: the trial's region scalars and, beside them, the HPWL the WA
-  // added up (hpwl_fetched_: that value is in hpwl_host_), so one copy and one wait serve
-  // both each trial.
+  bool hpwl_zeroed_ = false;  // a scatter since the last WA has cleared hpwl_acc_
+  // Page-locked read-back: the trial's region scalars, beside them the HPWL the WA added up
+  // (hpwl_fetched_: that value is in hpwl_host_). A trial's are written there by its gradient
+  // update itself (Publish), which the host waits for (published_: that update is the last work
+  // queued); other reads copy and synchronise.
   uint8_t *pinned_ = nullptr;
   size_t pinned_bytes_ = 0;
+  unsigned int *pub_count_ = nullptr;
+  unsigned int pub_seq_ = 0;
+  unsigned long long hpwl_published_ = 0;
+  bool published_ = false;
+  Publish publish(int expected);
+  bool wait_published();
   bool hpwl_fetched_ = false;
   unsigned long long hpwl_host_ = 0;
   // With overlap on (the default), the WA runs on its own stream beside the density solve
@@ -219,6 +228,7 @@ class Engine {
   void flush_grad(const std::vector<QueueEntry> &q, size_t a, size_t b);
   bool stage_tables(size_t n);
   bool wa_pending_ = false;
+  bool wa_split_ = false;    // the pending WA's small nets run on wa2_stream_
   bool fork_early_ = false;  // ev_fork_ holds the point right after the trial's last scatter
   void fork_after_place();
   bool overlap_ = true;

@@ -1254,9 +1254,14 @@ struct Placer {
       for (size_t b = 0; b < nbs.size(); b++)
         if (!nbs[b].is_converged) eng.nesterov_step((int)b, nbs[b].step_length, coeff);
       hpwl_dirty = true;
-      wa();  // beside the density solves: it needs the new centres, not the field
+      // the WA runs beside the density solves (it needs the new centres, not the field, and
+      // waits for the scatter alone): queued first when it is one launch, else after them, as
+      // its calls would hold back the solve's
+      const bool wa_first = eng.wa_joint();
+      if (wa_first) wa();
       for (size_t b = 0; b < nbs.size(); b++)
         if (!nbs[b].is_converged) eng.field((int)b);
+      if (!wa_first) wa();
       for (size_t b = 0; b < nbs.size(); b++)
         if (!nbs[b].is_converged) eng.gradients((int)b, S_NEXT_SLP_SUM, nbs[b].density_penalty, S_CUR_SLP, S_NEXT_SLP, S_CUR_SLP_SUM);
       eng.fetch();

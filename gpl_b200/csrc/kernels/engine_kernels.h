@@ -39,6 +39,20 @@ struct RegionArgs {
   // blocks of the last scatter whose cells spread past the shared tile (NULL: not counted);
   // the finalize reports the count (out[6]) and clears it
   unsigned int *spread;
+  unsigned long long *hpwl_zero; // the scatter clears the HPWL the next WA adds up (NULL: not)
+};
+
+// The trial's scalars written to page-locked host memory by the gradient update's last block
+// (of `expected` regions in the launch, the last region's): `words` doubles and the HPWL, each
+// as two 64-bit words, a half of its bits below the update's number. The host waits for that
+// number in every word, so no word needs a fence behind another. host NULL: not.
+struct Publish {
+  const double *scal;
+  const unsigned long long *hpwl;
+  unsigned long long *host;  // 2 (words + 1)
+  unsigned int *count;
+  int words, expected;
+  unsigned int seq;
 };
 
 // One region's cells, SoA, region-local index.
@@ -98,7 +112,7 @@ struct PackedRegion {
 // regions, each region's blocks doing exactly what its own launch's would.
 __global__ void k_place_packed(const PackedRegion *t, int n);
 __global__ void k_finalize_packed(const PackedRegion *t, int n);
-__global__ void k_gradients_packed(const PackedRegion *t, int n);
+__global__ void k_gradients_packed(const PackedRegion *t, int n, Publish pub);
 __global__ void k_place_cells(RegionArgs r, CellArgs c, int mode, float step, float coeff, const float2 *coords);
 __global__ void k_bins_finalize(RegionArgs r, double *partials, __nv_bfloat16 *dens_split, int split_ld, unsigned int *ticket, double *out);
 __global__ void k_wa(WaArgs w, float cx, float cy);
@@ -119,10 +133,17 @@ __global__ void k_wa_lean(WaArgs w, float cx, float cy, int forces);
 void launch_wa_small(const WaArgs &w, float cx, float cy, int forces, cudaStream_t s, int form = -1);
 // The degree-2..4 ranges of nets already in degree order.
 WaSmall wa_small_ranges(const int64_t *net_start, int32_t n_nets);
+// Both in one launch: the small nets as k_wa_pins, then the tiles; worth it up to two blocks
+// an SM (both then run at once in any case).
+inline bool wa_joint_fits(const WaSmall &s, int32_t n_tiles) {
+  const int b = wa_pins_blocks(s) + n_tiles;
+  return b > 0 && b <= 2 * 148;
+}
+void launch_wa_joint(const WaArgs &w, float cx, float cy, cudaStream_t s);
 // k_wa_tiles over every tile: a persistent grid of the blocks the device holds at once.
 void launch_wa_tiles(const WaArgs &w, float cx, float cy, cudaStream_t s);
 __global__ void k_gradients(RegionArgs r, CellArgs c, const float2 *pin_grad, float penalty, float2 *out_sum,
-                            const float2 *a1, const float2 *b1, const float2 *b2, double *partials, unsigned int *ticket, double *out);
+                            const float2 *a1, const float2 *b1, const float2 *b2, double *partials, unsigned int *ticket, double *out, Publish pub);
 __global__ void k_prev_slp(RegionArgs r, CellArgs c, float coef);
 __global__ void k_hpwl(WaArgs w, unsigned long long *out);
 __global__ void k_hpwl_tiles(WaArgs w, unsigned long long *out);

@@ -195,6 +195,7 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
   __shared__ unsigned long long s_red[kThreads];
   __shared__ int s_box[5];  // the block's bin box, and its cells' (cell, bin) addends
   int i = blk * blockDim.x + threadIdx.x;
+  if (r.hpwl_zero && blk == 0 && threadIdx.x == 0) *r.hpwl_zero = 0ull;
   const bool valid = i < r.n_cells;
   int32_t x0 = INT32_MAX, x1 = INT32_MIN, y0 = INT32_MAX, y1 = INT32_MIN;
   int32_t dlx = 0, dux = 0, dly = 0, duy = 0;
@@ -534,18 +535,17 @@ __global__ void k_wa(WaArgs w, float cx, float cy) {
 static_assert(kWaTileNets <= 256, "a pin's net index in the tile is kept in 8 bits");
 static_assert(kWaTilePins <= 2 * kThreads, "a thread holds at most two of a tile's pins");
 
-__global__ void __launch_bounds__(kThreads) k_wa_tiles(WaArgs w, float cx, float cy) {
+// The tiles `tile`, tile + step, ... by one block.
+__device__ __forceinline__ void wa_tiles_block(const WaArgs &w, float cx, float cy, int tile, const int step) {
   __shared__ int2 s_pos[kWaTilePins];        // phases 1-3: the position; 3-5: its floats' bits
   __shared__ float4 s_v[kWaTilePins];
   __shared__ uint16_t s_pnet[kWaTilePins];   // the pin's net in the tile | taken-terms mask << 8
   __shared__ int32_t s_nstart[kWaTileNets + 1];
   __shared__ int4 s_box[kWaTileNets];
   __shared__ float s_sum[8][kWaTileNets];
-  // Persistent: the block walks tiles blockIdx.x, + gridDim.x, ...; the next tile's record and
-  // its pins' cells load while this tile computes, so a tile starts with one round trip (the
-  // cell centres) instead of three.
+  // The next tile's record and its pins' cells load while this tile computes, so a tile starts
+  // with one round trip (the cell centres) instead of three.
   const int ja = threadIdx.x, jb = threadIdx.x + kThreads;
-  int tile = blockIdx.x;
   if (tile >= w.n_tiles) return;
   int4 t = w.tiles[tile];
   int32_t ca = -1, cb = -1;  // this tile's pins' cells
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kThreads) k_wa_tiles(WaArgs w, float cx, float
       if (two) s_pos[jb] = make_int2(bb.x + db.x, bb.y + db.y);
     }
     __syncthreads();
-    const int next = tile + gridDim.x;
+    const int next = tile + step;
     const int4 tn = next < w.n_tiles ? w.tiles[next] : make_int4(0, 0, 0, 0);
     long long h = 0;  // the same pins' HPWL, for the iteration's report
     for (int j = threadIdx.x; j < nn; j += blockDim.x) {
@@ -665,6 +665,7 @@ __global__ void __launch_bounds__(kThreads) k_wa_tiles(WaArgs w, float cx, float
     cb = cbn;
   }
 }
+__global__ void __launch_bounds__(kThreads) k_wa_tiles(WaArgs w, float cx, float cy) { wa_tiles_block(w, cx, cy, blockIdx.x, gridDim.x); }
 
 // One net of degree D, a thread's own (the nets of the small ranges): its positions in
 // registers, the box and the HPWL, the exp terms, the sums in pin order and each pin's force,
@@ -925,16 +926,16 @@ __device__ __forceinline__ long long wa_lane(const WaArgs &w, int32_t first, int
 // Blocks per degree range of k_wa_pins: a block holds kThreads / 32 warps of 32 / D nets.
 __host__ __device__ __forceinline__ int wa_pins_range_blocks(int32_t count, int d) { return (int)((count + (kThreads / 32) * (32 / d) - 1) / ((kThreads / 32) * (32 / d))); }
 
-__global__ void __launch_bounds__(kThreads, 6) k_wa_pins(WaArgs w, float cx, float cy, int forces) {
+// Block b of the degree ranges' blocks.
+__device__ __forceinline__ void wa_pins_block(const WaArgs &w, float cx, float cy, bool forces, int b) {
   const int nb0 = wa_pins_range_blocks(w.small.count[0], 2), nb1 = wa_pins_range_blocks(w.small.count[1], 3);
-  const int b = blockIdx.x;
   long long h;
   if (b < nb0)
-    h = wa_lane<2>(w, w.small.first[0], w.small.count[0], w.small.pin0[0], b, cx, cy, forces != 0);
+    h = wa_lane<2>(w, w.small.first[0], w.small.count[0], w.small.pin0[0], b, cx, cy, forces);
   else if (b < nb0 + nb1)
-    h = wa_lane<3>(w, w.small.first[1], w.small.count[1], w.small.pin0[1], b - nb0, cx, cy, forces != 0);
+    h = wa_lane<3>(w, w.small.first[1], w.small.count[1], w.small.pin0[1], b - nb0, cx, cy, forces);
   else
-    h = wa_lane<4>(w, w.small.first[2], w.small.count[2], w.small.pin0[2], b - nb0 - nb1, cx, cy, forces != 0);
+    h = wa_lane<4>(w, w.small.first[2], w.small.count[2], w.small.pin0[2], b - nb0 - nb1, cx, cy, forces);
   __shared__ long long s_h[kThreads / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) h += __shfl_down_sync(0xffffffffu, h, o);
@@ -946,6 +947,17 @@ __global__ void __launch_bounds__(kThreads, 6) k_wa_pins(WaArgs w, float cx, flo
     for (int j = 0; j < kThreads / 32; j++) sum += s_h[j];
     if (sum) atomicAdd(w.hpwl_out, (unsigned long long)sum);
   }
+}
+
+__global__ void __launch_bounds__(kThreads, 6) k_wa_pins(WaArgs w, float cx, float cy, int forces) { wa_pins_block(w, cx, cy, forces != 0, blockIdx.x); }
+
+// Both parts of a small design's WA in one launch: blocks [0, small) the degree-2..4 nets, a
+// lane per pin, then a block per tile.
+__global__ void __launch_bounds__(kThreads) k_wa_joint(WaArgs w, float cx, float cy, int small) {
+  if ((int)blockIdx.x < small)
+    wa_pins_block(w, cx, cy, true, blockIdx.x);
+  else
+    wa_tiles_block(w, cx, cy, blockIdx.x - small, gridDim.x - small);
 }
 
 int wa_pins_blocks(const WaSmall &s) { return wa_pins_range_blocks(s.count[0], 2) + wa_pins_range_blocks(s.count[1], 3) + wa_pins_range_blocks(s.count[2], 4); }
@@ -969,6 +981,11 @@ void launch_wa_small(const WaArgs &w, float cx, float cy, int forces, cudaStream
     else
       k_wa_lean<<<nb, kThreads, 0, s>>>(w, cx, cy, forces);
   }
+}
+
+void launch_wa_joint(const WaArgs &w, float cx, float cy, cudaStream_t s) {
+  const int small = wa_pins_blocks(w.small), blocks = small + w.n_tiles;
+  if (blocks) k_wa_joint<<<blocks, kThreads, 0, s>>>(w, cx, cy, small);
 }
 
 // The WA tiles' launch: a persistent grid of as many blocks as fit on the device at once.
@@ -995,9 +1012,33 @@ void launch_wa_tiles(const WaArgs &w, float cx, float cy, cudaStream_t s) {
 // the ordered sums; larger cells walk their bins.
 constexpr int kGradPinTile = 2048;
 
+// The trial's scalars to the host by the launch's last block. As two copies after the kernel
+// (3.3 us each, 3 to 7 us before each) and a synchronisation the host had them 13 to 17 us
+// later; words that carry the update's number save the system-wide fence a flag would need
+// (3 us).
+__device__ __forceinline__ void publish(const Publish &pub) {
+  __shared__ bool s_all;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_all = pub.expected <= 1 || atomicAdd(pub.count, 1u) == (unsigned)pub.expected - 1u;
+    if (s_all && pub.expected > 1) {
+      *pub.count = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (!s_all) return;
+  for (int k = threadIdx.x; k < 2 * (pub.words + 1); k += blockDim.x) {
+    const int w = k >> 1;
+    const unsigned long long v = w < pub.words ? (unsigned long long)__double_as_longlong(__ldcg(pub.scal + w)) : __ldcg(pub.hpwl);
+    const unsigned long long half = k & 1 ? v >> 32 : v & 0xffffffffull;
+    asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(pub.host + k), "l"((unsigned long long)pub.seq << 32 | half) : "memory");
+  }
+}
+
 // One block (cells blk * 256 ..) of a region's gradient update over nblk blocks.
 __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellArgs &c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1,
-                                                const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, int blk, int nblk) {
+                                                const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, const Publish &pub, int blk, int nblk) {
   __shared__ double4 sh[kThreads / 32];
   __shared__ float2 s_pg[kGradPinTile];
   const int i0 = blk * blockDim.x;
@@ -1096,18 +1137,21 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
   }
   // the last block to finish sums the blocks' partials (|wl|, |density|, the two distances)
   __shared__ double shr[kThreads / 32];
-  if (last_block_done(ticket, nblk)) reduce_rows<kThreads>(partials, nblk, 4, out, shr);
+  if (last_block_done(ticket, nblk)) {
+    reduce_rows<kThreads>(partials, nblk, 4, out, shr);
+    if (pub.host) publish(pub);
+  }
 }
 
-__global__ void __launch_bounds__(kThreads, 6) k_gradients(RegionArgs r, CellArgs c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1, const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out) {
+__global__ void __launch_bounds__(kThreads, 6) k_gradients(RegionArgs r, CellArgs c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1, const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, Publish pub) {
   chain_enter();
-  gradients_block(r, c, pin_grad, penalty, out_sum, a1, b1, b2, partials, ticket, out, blockIdx.x, gridDim.x);
+  gradients_block(r, c, pin_grad, penalty, out_sum, a1, b1, b2, partials, ticket, out, pub, blockIdx.x, gridDim.x);
 }
 
-__global__ void __launch_bounds__(kThreads, 6) k_gradients_packed(const PackedRegion *__restrict__ t, int n) {
+__global__ void __launch_bounds__(kThreads, 6) k_gradients_packed(const PackedRegion *__restrict__ t, int n, Publish pub) {
   __shared__ PackedRegion e;
   packed_entry(t, n, e);
-  gradients_block(e.r, e.c, e.pin_grad, e.penalty, e.out_sum, e.a1, e.b1, e.b2, e.partials, e.ticket, e.out, (int)blockIdx.x - e.first, e.blocks);
+  gradients_block(e.r, e.c, e.pin_grad, e.penalty, e.out_sum, e.a1, e.b1, e.b2, e.partials, e.ticket, e.out, pub, (int)blockIdx.x - e.first, e.blocks);
 }
 
 // ---- updateInitialPrevSLPCoordi (:2583-2595): a back-step along the current gradient.
