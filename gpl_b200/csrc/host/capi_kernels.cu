@@ -11,9 +11,33 @@
 #include "../kernels/bicgstab.h"
 #include "../kernels/engine_kernels.h"
 #include "../kernels/rudy.h"
+#include "../kernels/scratch.h"
 #include "parallel.h"
 
 using namespace gpl;
+
+// A grid of the caller's bins as the trial kernels read it; its upper corner and the scatter's
+// 32-bit test are taken from the edges on the device, into `corner` (NULL: not needed), so the
+// call waits for nothing.
+static void region_args(RegionArgs &r, int4 *corner, int32_t nx, int32_t ny, int32_t grid_lx, int32_t grid_ly, const int32_t *bx, const int32_t *by, double size_x, double size_y, float target_density, cudaStream_t s) {
+  r.nx = nx;
+  r.ny = ny;
+  r.lx = grid_lx;
+  r.ly = grid_ly;
+  r.size_x = size_x;
+  r.size_y = size_y;
+  r.inv_size_x = 1.0 / size_x;
+  r.inv_size_y = 1.0 / size_y;
+  r.target_density = target_density;
+  // GPL_SCATTER=global|pooled: the scatter's other forms (the engine's tuner picks per region)
+  if (const char *f = std::getenv("GPL_SCATTER")) r.scatter_form = std::string(f) == "global" ? 1 : std::string(f) == "pooled" ? 2 : 0;
+  r.bx = bx;
+  r.by = by;
+  r.corner = corner;
+  if (corner) k_grid_corner<<<1, kThreadsPerBlock, 0, s>>>(nx, ny, bx, by, corner);
+}
+
+static bool counts_fit(int64_t n_cells, int32_t nx, int32_t ny) { return n_cells >= 0 && n_cells < ((int64_t)1 << 31) && nx > 0 && ny > 0; }
 
 extern "C" {
 
@@ -26,33 +50,13 @@ int gpl_kernel_density_scatter(int64_t n_cells, const int32_t *cx, const int32_t
   if (n_cells <= 0) return 0;
   RegionArgs r{};
   r.n_cells = (int32_t)n_cells;
-  r.nx = nx;
-  r.ny = ny;
-  r.lx = grid_lx;
-  r.ly = grid_ly;
-  r.size_x = size_x;
-  r.size_y = size_y;
-  r.inv_size_x = 1.0 / size_x;
-  r.inv_size_y = 1.0 / size_y;
-  {
-    std::vector<int32_t> hbx(nx + 1), hby(ny + 1);
-    e = cudaMemcpyAsync(hbx.data(), bx, hbx.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hby.data(), by, hby.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return (int)e;
-    r.narrow = narrow_tile(hbx, hby) ? 1 : 0;
-  }
-  r.target_density = target_density;
-  // GPL_SCATTER=global|pooled: the scatter's other forms (the engine's tuner picks per region)
-  if (const char *f = std::getenv("GPL_SCATTER")) r.scatter_form = std::string(f) == "global" ? 1 : std::string(f) == "pooled" ? 2 : 0;
-  r.bx = bx;
-  r.by = by;
+  // the engine keeps a cell's centre as one int2: pack the caller's two arrays
+  Scratch buf(sizeof(int4) + (size_t)n_cells * sizeof(int2), s);
+  if ((e = buf.error()) != cudaSuccess) return (int)e;
+  region_args(r, static_cast<int4 *>(buf.get()), nx, ny, grid_lx, grid_ly, bx, by, size_x, size_y, target_density, s);
   r.acc_inst = inst;
   r.acc_fill = filler;
-  // the engine keeps a cell's centre as one int2: pack the caller's two arrays
-  int2 *dc = nullptr;
-  e = cudaMallocAsync((void **)&dc, (size_t)n_cells * sizeof(int2), s);
-  if (e != cudaSuccess) return (int)e;
+  int2 *dc = reinterpret_cast<int2 *>(static_cast<int4 *>(buf.get()) + 1);
   unsigned blocks = (unsigned)((n_cells + kThreadsPerBlock - 1) / kThreadsPerBlock);
   k_pack_centres<<<blocks, kThreadsPerBlock, 0, s>>>(n_cells, cx, cy, dc);
   CellArgs c{};
@@ -62,54 +66,25 @@ int gpl_kernel_density_scatter(int64_t n_cells, const int32_t *cx, const int32_t
   c.dscale = scale;
   c.kind = kind;
   k_place_cells<<<blocks, kThreadsPerBlock, 0, s>>>(r, c, PLACE_GIVEN, 0.0f, 0.0f, nullptr);
-  e = cudaGetLastError();
-  cudaError_t e2 = cudaFreeAsync(dc, s);
-  return (int)(e != cudaSuccess ? e : e2);
-}
-
-// A grid of the caller's bins as the trial kernels read it; its edges are read back here (the
-// scatter's 32-bit tile test and the grid's upper corner).
-static cudaError_t region_args(RegionArgs &r, int64_t n_cells, int32_t nx, int32_t ny, int32_t grid_lx, int32_t grid_ly, const int32_t *bx, const int32_t *by, double size_x, double size_y, float target_density, cudaStream_t s) {
-  if (n_cells < 0 || n_cells >= ((int64_t)1 << 31) || nx <= 0 || ny <= 0) return cudaErrorInvalidValue;
-  r = RegionArgs{};
-  r.n_cells = (int32_t)n_cells;
-  r.nx = nx;
-  r.ny = ny;
-  r.lx = grid_lx;
-  r.ly = grid_ly;
-  r.size_x = size_x;
-  r.size_y = size_y;
-  r.inv_size_x = 1.0 / size_x;
-  r.inv_size_y = 1.0 / size_y;
-  std::vector<int32_t> hbx(nx + 1), hby(ny + 1);
-  cudaError_t e = cudaMemcpyAsync(hbx.data(), bx, hbx.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hby.data(), by, hby.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return e;
-  r.ux = hbx[nx];
-  r.uy = hby[ny];
-  r.narrow = narrow_tile(hbx, hby) ? 1 : 0;
-  r.target_density = target_density;
-  // GPL_SCATTER=global|pooled: the scatter's other forms (the engine's tuner picks per region)
-  if (const char *f = std::getenv("GPL_SCATTER")) r.scatter_form = std::string(f) == "global" ? 1 : std::string(f) == "pooled" ? 2 : 0;
-  r.bx = bx;
-  r.by = by;
-  return cudaSuccess;
+  return (int)cudaGetLastError();
 }
 
 static bool aligned8(const void *p) { return ((uintptr_t)p & 7u) == 0; }
 
 int gpl_kernel_nesterov_step(int64_t n_cells, const float *cur_slp, const float *cur_slp_sum, const float *cur, const int32_t *hx, const int32_t *hy, const float *scale, const uint8_t *kind, const uint8_t *locked, int32_t nx, int32_t ny, int32_t grid_lx, int32_t grid_ly, const int32_t *bx, const int32_t *by, double size_x, double size_y, float target_density, float step, float coeff, float *next, float *next_slp, int32_t *centre, int64_t *inst, int64_t *filler, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  RegionArgs r;
-  cudaError_t e = region_args(r, n_cells, nx, ny, grid_lx, grid_ly, bx, by, size_x, size_y, target_density, s);
-  if (e != cudaSuccess) return (int)e;
+  if (!counts_fit(n_cells, nx, ny)) return (int)cudaErrorInvalidValue;
   for (const void *p : {(const void *)cur_slp, (const void *)cur_slp_sum, (const void *)cur, (const void *)next, (const void *)next_slp, (const void *)centre})
     if (!aligned8(p)) return (int)cudaErrorMisalignedAddress;  // read and written as pairs
   size_t nb = (size_t)nx * ny;
-  e = cudaMemsetAsync(inst, 0, nb * sizeof(int64_t), s);
+  cudaError_t e = cudaMemsetAsync(inst, 0, nb * sizeof(int64_t), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(filler, 0, nb * sizeof(int64_t), s);
   if (e != cudaSuccess || n_cells == 0) return (int)e;
+  Scratch buf(sizeof(int4), s);
+  if ((e = buf.error()) != cudaSuccess) return (int)e;
+  RegionArgs r{};
+  r.n_cells = (int32_t)n_cells;
+  region_args(r, static_cast<int4 *>(buf.get()), nx, ny, grid_lx, grid_ly, bx, by, size_x, size_y, target_density, s);
   r.acc_inst = inst;
   r.acc_fill = filler;
   CellArgs c{};
@@ -133,13 +108,14 @@ int gpl_kernel_nesterov_step(int64_t n_cells, const float *cur_slp, const float 
 int gpl_kernel_gradients(int64_t n_cells, const int32_t *centre, const int32_t *hx, const int32_t *hy, const float *scale, const float *area, const int64_t *cell_pin_start, const float *pin_force, int32_t nx, int32_t ny, int32_t grid_lx, int32_t grid_ly, const int32_t *bx, const int32_t *by, double size_x, double size_y, const float *field_x, const float *field_y, float penalty, float *sum, const float *a1, const float *b1, const float *b2, double *sums, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   for (int k = 0; k < 4; k++) sums[k] = 0.0;
-  RegionArgs r;
-  cudaError_t e = region_args(r, n_cells, nx, ny, grid_lx, grid_ly, bx, by, size_x, size_y, 1.0f, s);
-  if (e != cudaSuccess) return (int)e;
+  if (!counts_fit(n_cells, nx, ny)) return (int)cudaErrorInvalidValue;
   for (const void *p : {(const void *)centre, (const void *)pin_force, (const void *)sum, (const void *)a1, (const void *)b1, (const void *)b2})
     if (!aligned8(p)) return (int)cudaErrorMisalignedAddress;
   if ((a1 == nullptr) != (b1 == nullptr)) return (int)cudaErrorInvalidValue;
   if (n_cells == 0) return 0;
+  RegionArgs r{};
+  r.n_cells = (int32_t)n_cells;
+  region_args(r, nullptr, nx, ny, grid_lx, grid_ly, bx, by, size_x, size_y, 1.0f, s);  // the update reads no corner
   r.field_x = const_cast<float *>(field_x);
   r.field_y = const_cast<float *>(field_y);
   CellArgs c{};
@@ -152,10 +128,10 @@ int gpl_kernel_gradients(int64_t n_cells, const int32_t *centre, const int32_t *
   const int blocks = (int)((n_cells + kThreadsPerBlock - 1) / kThreadsPerBlock);
   // the block partials, the arrival ticket and the four sums, in one scratch block
   const size_t bytes = (size_t)(4 * blocks + 4) * sizeof(double) + 256;
-  uint8_t *scratch = nullptr;
-  e = cudaMallocAsync((void **)&scratch, bytes, s);
+  Scratch buf(bytes, s);
+  cudaError_t e = buf.error();
   if (e != cudaSuccess) return (int)e;
-  double *partials = reinterpret_cast<double *>(scratch), *out = partials + 4 * blocks;
+  double *partials = static_cast<double *>(buf.get()), *out = partials + 4 * blocks;
   unsigned int *ticket = reinterpret_cast<unsigned int *>(out + 4);
   e = cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s);
   if (e == cudaSuccess) {
@@ -165,8 +141,7 @@ int gpl_kernel_gradients(int64_t n_cells, const int32_t *centre, const int32_t *
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(sums, out, 4 * sizeof(double), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaError_t e2 = cudaFreeAsync(scratch, s);
-  return (int)(e != cudaSuccess ? e : e2);
+  return (int)e;
 }
 
 int gpl_kernel_poisson(int32_t nx, int32_t ny, const float *wx, const float *wy, const float *density, float *field_x, float *field_y, int mode, void *stream) {

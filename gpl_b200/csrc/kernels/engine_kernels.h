@@ -39,6 +39,8 @@ struct RegionArgs {
   // blocks of the last scatter whose cells spread past the shared tile (NULL: not counted);
   // the finalize reports the count (out[6]) and clears it
   unsigned int *spread;
+  // the grid's upper corner and `narrow` on the device (ux, uy, narrow; NULL: the fields above)
+  const int4 *corner;
   unsigned long long *hpwl_zero; // the scatter clears the HPWL the next WA adds up (NULL: not)
 };
 
@@ -182,6 +184,8 @@ __global__ void k_order_pins(int64_t n_pins, int32_t off, int32_t n, const int32
 __global__ void k_order_starts(int32_t n, const int64_t *rel, int64_t *start);
 __global__ void k_iota(int32_t n, int32_t *a);
 
+// A grid's RegionArgs::corner from its edges on the device (one block of kThreadsPerBlock).
+__global__ void k_grid_corner(int32_t nx, int32_t ny, const int32_t *bx, const int32_t *by, int4 *out);
 // Whether a grid's bins are small enough for the scatter's 32-bit shared tile.
 bool narrow_tile(const std::vector<int32_t> &bx, const std::vector<int32_t> &by);
 

@@ -189,6 +189,36 @@ __device__ __forceinline__ void pooled_scatter(const RegionArgs &r, bool narrow,
   }
 }
 
+// A cell over more bins than this (a macro) is taken by its whole warp: one lane walking the
+// 1600 bins of a macro 40 bins a side kept the launch waiting (1.1M cells with 55 macros of up
+// to that size: the step 750 us, 226 with the macros spread over their warps; the gradient
+// update 186 us, 109).
+constexpr int kBigCell = 64;
+
+// The big cells of a warp's lanes, each lane's own in turn, every lane taking bins of it,
+// straight to HBM. Integer adds: any order.
+__device__ __forceinline__ void big_scatter(const RegionArgs &r, bool big, int32_t x0, int32_t x1, int32_t y0, int32_t y1, int32_t dlx, int32_t dux, int32_t dly, int32_t duy, float scale, uint8_t kind) {
+  for (unsigned m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {
+    const int s = __ffs(m) - 1;
+    const int32_t bx0 = __shfl_sync(0xffffffffu, x0, s), bx1 = __shfl_sync(0xffffffffu, x1, s), by0 = __shfl_sync(0xffffffffu, y0, s), by1 = __shfl_sync(0xffffffffu, y1, s);
+    const int32_t lx = __shfl_sync(0xffffffffu, dlx, s), ux = __shfl_sync(0xffffffffu, dux, s), ly = __shfl_sync(0xffffffffu, dly, s), uy = __shfl_sync(0xffffffffu, duy, s);
+    const float sc = __shfl_sync(0xffffffffu, scale, s);
+    const uint8_t kd = (uint8_t)__shfl_sync(0xffffffffu, (int)kind, s);
+    unsigned long long *acc = (unsigned long long *)(kd == CELL_FILLER ? r.acc_fill : r.acc_inst);
+    const int32_t h = by1 - by0;
+    // lanes along y (the accumulators' fast axis), the warp's columns side by side when the
+    // cell is narrower than a warp
+    const int32_t cols = h >= 32 ? 1 : 32 / h;
+    const int32_t lane = threadIdx.x & 31, c = h >= 32 ? 0 : lane / h, yy = h >= 32 ? lane : lane - c * h;
+    if (c < cols)
+      for (int32_t x = bx0 + c; x < bx1; x += cols)
+        for (int32_t y = by0 + yy; y < by1; y += 32) {
+          const int64_t v = cell_bin_addend(r, lx, ux, ly, uy, x, y, sc, kd);
+          if (v) atomicAdd(&acc[(size_t)x * r.ny + y], (unsigned long long)v);
+        }
+  }
+}
+
 // One block of a region's scatter: block `blk` of the region's cells.
 __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const CellArgs &c, int mode, float step, float coeff, const float2 *__restrict__ coords, int blk) {
   __shared__ __align__(16) unsigned long long s_tile[2 * kTileBins];  // cells then fillers; 32-bit when narrow
@@ -197,6 +227,7 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
   int i = blk * blockDim.x + threadIdx.x;
   if (r.hpwl_zero && blk == 0 && threadIdx.x == 0) *r.hpwl_zero = 0ull;
   const bool valid = i < r.n_cells;
+  const int4 corner = r.corner ? *r.corner : make_int4(r.ux, r.uy, r.narrow, 0);
   int32_t x0 = INT32_MAX, x1 = INT32_MIN, y0 = INT32_MAX, y1 = INT32_MIN;
   int32_t dlx = 0, dux = 0, dly = 0, duy = 0;
   float scale = 0.0f;
@@ -225,7 +256,7 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
         float sx = __fadd_rn(nx, __fmul_rn(coeff, __fsub_rn(nx, cu.x)));
         float sy = __fadd_rn(ny, __fmul_rn(coeff, __fsub_rn(ny, cu.y)));
         const float fhx = (float)hx, fhy = (float)hy;
-        float glx = (float)r.lx, gly = (float)r.ly, gux = (float)r.ux, guy = (float)r.uy;
+        float glx = (float)r.lx, gly = (float)r.ly, gux = (float)corner.x, guy = (float)corner.y;
         c.next[i] = make_float2(inside_axis(nx, fhx, glx, gux), inside_axis(ny, fhy, gly, guy));
         p = make_float2(inside_axis(sx, fhx, glx, gux), inside_axis(sy, fhy, gly, guy));
         c.next_slp[i] = p;
@@ -257,41 +288,71 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
     s_box[4] = 0;
   }
   __syncthreads();
-  const bool any = valid && x0 < x1 && y0 < y1;
+  bool any = valid && x0 < x1 && y0 < y1;
   const int nb_cell = any ? (x1 - x0) * (y1 - y0) : 0;
-  const int w_addends = __reduce_add_sync(0xffffffffu, nb_cell);
-  int32_t wx0 = __reduce_min_sync(0xffffffffu, any ? x0 : INT32_MAX), wx1 = __reduce_max_sync(0xffffffffu, any ? x1 : INT32_MIN);
-  int32_t wy0 = __reduce_min_sync(0xffffffffu, any ? y0 : INT32_MAX), wy1 = __reduce_max_sync(0xffffffffu, any ? y1 : INT32_MIN);
+  const bool big = nb_cell > kBigCell;
+  int32_t wx0, wx1, wy0, wy1;
+  int w_addends;
   const int lane = threadIdx.x & 31;
-  if (lane == 0) {
-    atomicMin(&s_box[0], wx0);
-    atomicMax(&s_box[1], wx1);
-    atomicMin(&s_box[2], wy0);
-    atomicMax(&s_box[3], wy1);
-    atomicAdd(&s_box[4], w_addends);
-  }
-  __syncthreads();
+  auto boxes = [&]() {
+    w_addends = __reduce_add_sync(0xffffffffu, any ? nb_cell : 0);
+    wx0 = __reduce_min_sync(0xffffffffu, any ? x0 : INT32_MAX), wx1 = __reduce_max_sync(0xffffffffu, any ? x1 : INT32_MIN);
+    wy0 = __reduce_min_sync(0xffffffffu, any ? y0 : INT32_MAX), wy1 = __reduce_max_sync(0xffffffffu, any ? y1 : INT32_MIN);
+    if (lane == 0) {
+      atomicMin(&s_box[0], wx0);
+      atomicMax(&s_box[1], wx1);
+      atomicMin(&s_box[2], wy0);
+      atomicMax(&s_box[3], wy1);
+      atomicAdd(&s_box[4], w_addends);
+    }
+  };
+  boxes();
+  const bool has_big = __syncthreads_or(big);
   // The block's cells share one tile when their bins fit it (32-bit slots hold twice as many
   // bins) and the tile is not mostly empty (at most twice as many slots as addends: a sparse
   // block's slots would cost more to clear and flush than its addends); else each warp takes a
   // slice of the tile for its own cells on the same terms, and a warp whose cells spread
   // wider adds straight to HBM.
-  const bool narrow = r.narrow != 0;
+  const bool narrow = corner.z != 0;
   const int bcap = narrow ? 2 * kTileBins : kTileBins;
-  const int64_t b_nt = (int64_t)(s_box[1] - s_box[0]) * (s_box[3] - s_box[2]);
+  auto fits = [&]() {
+    const int64_t b_nt = (int64_t)(s_box[1] - s_box[0]) * (s_box[3] - s_box[2]);
+    return s_box[1] > s_box[0] && s_box[3] > s_box[2] && b_nt <= bcap && b_nt <= 2 * (int64_t)s_box[4];
+  };
   // (the other forms add straight to HBM; the spread count is the same in every form)
-  const bool tile = s_box[1] > s_box[0] && s_box[3] > s_box[2] && b_nt <= bcap && b_nt <= 2 * (int64_t)s_box[4];
+  bool tile = fits();
+  if (!tile && threadIdx.x == 0 && r.spread) atomicAdd(r.spread, 1u);
+  if (has_big) {
+    // the big cells on their own; the others' boxes without them
+    big_scatter(r, big, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
+    any = any && !big;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_box[0] = s_box[2] = INT32_MAX;
+      s_box[1] = s_box[3] = INT32_MIN;
+      s_box[4] = 0;
+    }
+    __syncthreads();
+    boxes();
+    __syncthreads();
+    tile = fits();
+  }
   unsigned int *t32 = reinterpret_cast<unsigned int *>(s_tile);
   const bool tiles = r.scatter_form == 0;
-  if (tile && tiles) {
+  // A tile pays where its slots take many addends each: below kDense a slot the atomics on
+  // HBM's accumulators (in L2) seldom meet and the walk in step costs more than it saves.
+  // Measured on 1.1M cells, tiles against straight to HBM: spread evenly (8 addends a bin of a
+  // block's box) 226 against 72 us, 16 times as dense (51) 163 against 92, 100 times (120) 111
+  // against 155, 10^4 times 84 against 624.
+  constexpr int64_t kDense = 64;
+  if (tile && tiles && s_box[4] >= kDense * (int64_t)(s_box[1] - s_box[0]) * (s_box[3] - s_box[2])) {
     tile_scatter<true>(r, narrow, s_tile, t32, s_red, bcap, s_box[0], s_box[2], s_box[3] - s_box[2], s_box[1] - s_box[0], any, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
     return;
   }
-  if (!tile && threadIdx.x == 0 && r.spread) atomicAdd(r.spread, 1u);
   const int wcap = bcap / (kThreads / 32);
   const int64_t w_nt = (int64_t)(wx1 - wx0) * (wy1 - wy0);
   const bool wtile = wx1 > wx0 && wy1 > wy0 && w_nt <= wcap && w_nt <= 2 * (int64_t)w_addends;  // warp-uniform
-  if (wtile && tiles) {
+  if (wtile && tiles && w_addends >= kDense * w_nt) {
     const int w = threadIdx.x >> 5;
     tile_scatter<false>(r, narrow, s_tile + (size_t)w * 2 * wcap, t32 + (size_t)w * 2 * wcap, s_red, wcap, wx0, wy0, wy1 - wy0, wx1 - wx0, any, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
     return;
@@ -302,6 +363,34 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
   }
   if (any) {
     unsigned long long *acc = (unsigned long long *)(kind == CELL_FILLER ? r.acc_fill : r.acc_inst);
+    const int32_t w = x1 - x0, h = y1 - y0;
+    if (w <= 3 && h <= 3) {
+      // two or three bins an axis (a cell is widened to sqrt(2) bins): each edge read once
+      float ox[3], oy[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        ox[q] = oy[q] = 0.0f;
+        if (q < w) {
+          const int32_t lo = r.bx[x0 + q], hi = r.bx[x0 + q + 1];
+          const int32_t o = (dux < hi ? dux : hi) - (dlx > lo ? dlx : lo);
+          if (o > 0) ox[q] = small_i2f(o);
+        }
+        if (q < h) {
+          const int32_t lo = r.by[y0 + q], hi = r.by[y0 + q + 1];
+          const int32_t o = (duy < hi ? duy : hi) - (dly > lo ? dly : lo);
+          if (o > 0) oy[q] = small_i2f(o);
+        }
+      }
+      unsigned long long *at = acc + (size_t)x0 * r.ny + y0;
+#pragma unroll
+      for (int q = 0; q < 9; q++) {
+        float a = __fmul_rn(__fmul_rn(ox[q / 3], oy[q % 3]), scale);
+        if (kind == CELL_MACRO) a = __fmul_rn(a, r.target_density);
+        const int64_t v = small_f2l_rz(a);
+        if (v) atomicAdd(at + (size_t)(q / 3) * r.ny + q % 3, (unsigned long long)v);
+      }
+      return;
+    }
     for (int32_t y = y0; y < y1; y++)
       for (int32_t x = x0; x < x1; x++) {
         int64_t v = cell_bin_addend(r, dlx, dux, dly, duy, x, y, scale, kind);
@@ -310,7 +399,25 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_place_cells(RegionArgs r, CellArgs c, int mode, float step, float coeff, const float2 *__restrict__ coords) {
+__global__ void __launch_bounds__(kThreads) k_grid_corner(int32_t nx, int32_t ny, const int32_t *__restrict__ bx, const int32_t *__restrict__ by, int4 *__restrict__ out) {
+  // narrow_tile on the device: the largest bin's area, kThreads times, below 2^32
+  __shared__ unsigned s_w, s_h;
+  if (threadIdx.x == 0) s_w = s_h = 0u;
+  __syncthreads();
+  unsigned w = 0, h = 0;
+  for (int k = threadIdx.x; k < nx; k += kThreads) w = max(w, (unsigned)max(0ll, (long long)bx[k + 1] - bx[k]));
+  for (int k = threadIdx.x; k < ny; k += kThreads) h = max(h, (unsigned)max(0ll, (long long)by[k + 1] - by[k]));
+  w = __reduce_max_sync(0xffffffffu, w);
+  h = __reduce_max_sync(0xffffffffu, h);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_w, w);
+    atomicMax(&s_h, h);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *out = make_int4(bx[nx], by[ny], (double)s_w * (double)s_h * kThreads < 4294967295.0 ? 1 : 0, 0);
+}
+
+__global__ void __launch_bounds__(kThreads, 6) k_place_cells(RegionArgs r, CellArgs c, int mode, float step, float coeff, const float2 *__restrict__ coords) {
   place_cells_block(r, c, mode, step, coeff, coords, blockIdx.x);
 }
 
@@ -334,7 +441,7 @@ __device__ __forceinline__ void packed_entry(const PackedRegion *__restrict__ t,
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) k_place_packed(const PackedRegion *__restrict__ t, int n) {
+__global__ void __launch_bounds__(kThreads, 6) k_place_packed(const PackedRegion *__restrict__ t, int n) {
   __shared__ PackedRegion e;
   packed_entry(t, n, e);
   place_cells_block(e.r, e.c, PLACE_NESTEROV, e.step, e.coeff, nullptr, (int)blockIdx.x - e.first);
@@ -1008,8 +1115,8 @@ void launch_wa_tiles(const WaArgs &w, float cx, float cy, cudaStream_t s) {
 // |a1 - b1|^2 and |out - b2|^2.
 // A block's cells are consecutive, so their pins' forces (cell-major) are one run: staged in
 // shared memory with coalesced loads when the run fits kGradPinTile, then each cell sums its
-// own in order. A cell over at most 2 x 2 bins loads its bins' boundaries and fields before
-// the ordered sums; larger cells walk their bins.
+// own in order. A cell over at most 3 x 3 bins loads its bins' boundaries and fields before
+// the ordered sums; larger cells walk their bins, the largest (kBigCell) by their warp.
 constexpr int kGradPinTile = 2048;
 
 // The trial's scalars to the host by the launch's last block. As two copies after the kernel
@@ -1036,6 +1143,62 @@ __device__ __forceinline__ void publish(const Publish &pub) {
   }
 }
 
+// The density force of the big cells among a warp's lanes (kBigCell): the warp's lanes form
+// the bins' terms, four runs of 32 in flight, and every lane adds them in the reference's order
+// (x outer, y inner) through shuffles, so the sums are the serial walk's bit for bit.
+__device__ __forceinline__ void big_force(const RegionArgs &r, bool big, int32_t x0, int32_t x1, int32_t y0, int32_t y1, int32_t dlx, int32_t dux, int32_t dly, int32_t duy, float scale, float &fx, float &fy) {
+  const int lane = threadIdx.x & 31;
+  constexpr int U = 4;
+  for (unsigned m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {
+    const int s = __ffs(m) - 1;
+    const int32_t bx0 = __shfl_sync(0xffffffffu, x0, s), bx1 = __shfl_sync(0xffffffffu, x1, s), by0 = __shfl_sync(0xffffffffu, y0, s), by1 = __shfl_sync(0xffffffffu, y1, s);
+    const int32_t lx = __shfl_sync(0xffffffffu, dlx, s), ux = __shfl_sync(0xffffffffu, dux, s), ly = __shfl_sync(0xffffffffu, dly, s), uy = __shfl_sync(0xffffffffu, duy, s);
+    const float sc = __shfl_sync(0xffffffffu, scale, s);
+    const int32_t h = by1 - by0, n = (bx1 - bx0) * h;
+    float sx = 0.0f, sy = 0.0f;
+    for (int32_t k0 = 0; k0 < n; k0 += 32 * U) {
+      float px[U], py[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int32_t k = k0 + 32 * u + lane;
+        px[u] = py[u] = 0.0f;
+        if (k < n) {
+          const int32_t c = k / h, x = bx0 + c, y = by0 + (k - c * h);
+          const int32_t blx = r.bx[x], bux = r.bx[x + 1], bly = r.by[y], buy = r.by[y + 1];
+          const size_t at = (size_t)x * r.ny + y;
+          const int32_t olx = lx > blx ? lx : blx, oux = ux < bux ? ux : bux;
+          const int32_t oly = ly > bly ? ly : bly, ouy = uy < buy ? uy : buy;
+          float a = 0.0f;
+          if (olx < oux && oly < ouy) a = __fmul_rn((float)(oux - olx), (float)(ouy - oly));
+          a = __fmul_rn(a, sc);
+          px[u] = __fmul_rn(a, r.field_x[at]);
+          py[u] = __fmul_rn(a, r.field_y[at]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int32_t left = n - (k0 + 32 * u);
+        if (left >= 32) {
+#pragma unroll
+          for (int t = 0; t < 32; t++) {
+            sx = __fadd_rn(sx, __shfl_sync(0xffffffffu, px[u], t));
+            sy = __fadd_rn(sy, __shfl_sync(0xffffffffu, py[u], t));
+          }
+        } else {
+          for (int t = 0; t < left; t++) {
+            sx = __fadd_rn(sx, __shfl_sync(0xffffffffu, px[u], t));
+            sy = __fadd_rn(sy, __shfl_sync(0xffffffffu, py[u], t));
+          }
+        }
+      }
+    }
+    if (lane == s) {
+      fx = sx;
+      fy = sy;
+    }
+  }
+}
+
 // One block (cells blk * 256 ..) of a region's gradient update over nblk blocks.
 __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellArgs &c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1,
                                                 const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, const Publish &pub, int blk, int nblk) {
@@ -1050,7 +1213,75 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
     for (int k = threadIdx.x; k < (int)(p1 - p0); k += blockDim.x) s_pg[k] = pin_grad[p0 + k];
   __syncthreads();
   double s_wl = 0, s_den = 0, s_d1 = 0, s_d2 = 0;
-  if (i < r.n_cells) {
+  const bool valid = i < r.n_cells;
+  int32_t dlx = 0, dux = 0, dly = 0, duy = 0, x0 = 0, x1 = 0, y0 = 0, y1 = 0;
+  float scale = 0.0f, fx = 0.0f, fy = 0.0f;
+  if (valid) {
+    const int2 d = c.dc[i];
+    const int32_t hx = c.hx[i], hy = c.hy[i];
+    scale = c.dscale[i];
+    dlx = d.x - hx, dux = d.x + hx, dly = d.y - hy, duy = d.y + hy;
+    bin_span(dlx, dux, r.lx, r.size_x, r.inv_size_x, r.nx, x0, x1);
+    bin_span(dly, duy, r.ly, r.size_y, r.inv_size_y, r.ny, y0, y1);
+    const int32_t w = x1 - x0, h = y1 - y0;
+    // one bin's term in the reference's order: overlap area (float), times the scale, times
+    // the field, added to the running sums
+    if (w <= 0 || h <= 0) {
+    } else if (w <= 3 && h <= 3) {
+      // A cell is widened to sqrt(2) bins, so two or three bins an axis: every load first (the
+      // edges, up to nine bins' fields), then the sums in order (x outer, y inner).
+      float ox[3], oy[3], ex[9], ey[9];
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        ox[q] = oy[q] = 0.0f;
+        if (q < w) {
+          const int32_t lo = r.bx[x0 + q], hi = r.bx[x0 + q + 1];
+          const int32_t o = (dux < hi ? dux : hi) - (dlx > lo ? dlx : lo);
+          ox[q] = o > 0 ? (float)o : 0.0f;
+        }
+        if (q < h) {
+          const int32_t lo = r.by[y0 + q], hi = r.by[y0 + q + 1];
+          const int32_t o = (duy < hi ? duy : hi) - (dly > lo ? dly : lo);
+          oy[q] = o > 0 ? (float)o : 0.0f;
+        }
+      }
+      const size_t k0 = (size_t)x0 * r.ny + y0;
+#pragma unroll
+      for (int q = 0; q < 9; q++) {
+        ex[q] = ey[q] = 0.0f;
+        if (q / 3 < w && q % 3 < h) {
+          const size_t k = k0 + (size_t)(q / 3) * r.ny + q % 3;
+          ex[q] = r.field_x[k];
+          ey[q] = r.field_y[k];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 9; q++)
+        if (q / 3 < w && q % 3 < h) {
+          const float a = __fmul_rn(__fmul_rn(ox[q / 3], oy[q % 3]), scale);
+          fx = __fadd_rn(fx, __fmul_rn(a, ex[q]));
+          fy = __fadd_rn(fy, __fmul_rn(a, ey[q]));
+        }
+    } else if (w * h <= kBigCell) {
+      for (int32_t x = x0; x < x1; x++) {
+        const int32_t blx = r.bx[x], bux = r.bx[x + 1];
+        for (int32_t y = y0; y < y1; y++) {
+          const int32_t bly = r.by[y], buy = r.by[y + 1];
+          const size_t k = (size_t)x * r.ny + y;
+          const int32_t olx = dlx > blx ? dlx : blx, oux = dux < bux ? dux : bux;
+          const int32_t oly = dly > bly ? dly : bly, ouy = duy < buy ? duy : buy;
+          float a = 0.0f;
+          if (olx < oux && oly < ouy) a = __fmul_rn((float)(oux - olx), (float)(ouy - oly));
+          a = __fmul_rn(a, scale);
+          fx = __fadd_rn(fx, __fmul_rn(a, r.field_x[k]));
+          fy = __fadd_rn(fy, __fmul_rn(a, r.field_y[k]));
+        }
+      }
+    }
+  }
+  const bool big = x1 > x0 && y1 > y0 && (x1 - x0) * (y1 - y0) > kBigCell;
+  if (__any_sync(0xffffffffu, big)) big_force(r, big, x0, x1, y0, y1, dlx, dux, dly, duy, scale, fx, fy);
+  if (valid) {
     const int64_t pb = c.pin_start[i], pe = c.pin_start[i + 1];
     float wlx = 0.0f, wly = 0.0f;
     if (staged) {
@@ -1064,48 +1295,6 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
         float2 t = pin_grad[k];
         wlx = __fadd_rn(wlx, t.x);
         wly = __fadd_rn(wly, t.y);
-      }
-    }
-    int2 d = c.dc[i];
-    int32_t cx = d.x, cy = d.y, hx = c.hx[i], hy = c.hy[i];
-    int32_t dlx = cx - hx, dux = cx + hx, dly = cy - hy, duy = cy + hy;
-    int32_t x0, x1, y0, y1;
-    bin_span(dlx, dux, r.lx, r.size_x, r.inv_size_x, r.nx, x0, x1);
-    bin_span(dly, duy, r.ly, r.size_y, r.inv_size_y, r.ny, y0, y1);
-    float scale = c.dscale[i];
-    float fx = 0.0f, fy = 0.0f;
-    // one bin's term in the reference's order: overlap area (float), times the scale, times
-    // the field, added to the running sums
-    auto term = [&](int32_t blx, int32_t bux, int32_t bly, int32_t buy, float ex, float ey) {
-      int32_t olx = dlx > blx ? dlx : blx, oux = dux < bux ? dux : bux;
-      int32_t oly = dly > bly ? dly : bly, ouy = duy < buy ? duy : buy;
-      float a = 0.0f;
-      if (olx < oux && oly < ouy) a = __fmul_rn((float)(oux - olx), (float)(ouy - oly));
-      a = __fmul_rn(a, scale);
-      fx = __fadd_rn(fx, __fmul_rn(a, ex));
-      fy = __fadd_rn(fy, __fmul_rn(a, ey));
-    };
-    if (x1 - x0 <= 2 && y1 - y0 <= 2 && x1 > x0 && y1 > y0) {
-      // every load first (the boundaries and up to four bins' fields), then the sums in order
-      const int xb = min(x0 + 1, x1 - 1), yb = min(y0 + 1, y1 - 1);
-      const int32_t bx0 = r.bx[x0], bx1 = r.bx[x0 + 1], bx2 = r.bx[xb + 1];
-      const int32_t by0 = r.by[y0], by1 = r.by[y0 + 1], by2 = r.by[yb + 1];
-      const size_t k00 = (size_t)x0 * r.ny + y0, k01 = (size_t)x0 * r.ny + yb, k10 = (size_t)xb * r.ny + y0, k11 = (size_t)xb * r.ny + yb;
-      const float e00x = r.field_x[k00], e00y = r.field_y[k00], e01x = r.field_x[k01], e01y = r.field_y[k01];
-      const float e10x = r.field_x[k10], e10y = r.field_y[k10], e11x = r.field_x[k11], e11y = r.field_y[k11];
-      term(bx0, bx1, by0, by1, e00x, e00y);
-      if (y1 - y0 == 2) term(bx0, bx1, by1, by2, e01x, e01y);
-      if (x1 - x0 == 2) {
-        term(bx1, bx2, by0, by1, e10x, e10y);
-        if (y1 - y0 == 2) term(bx1, bx2, by1, by2, e11x, e11y);
-      }
-    } else {
-      for (int32_t x = x0; x < x1; x++) {
-        int32_t blx = r.bx[x], bux = r.bx[x + 1];
-        for (int32_t y = y0; y < y1; y++) {
-          size_t k = (size_t)x * r.ny + y;
-          term(blx, bux, r.by[y], r.by[y + 1], r.field_x[k], r.field_y[k]);
-        }
       }
     }
     float sx = __fadd_rn(wlx, __fmul_rn(penalty, fx));
