@@ -147,7 +147,7 @@ int gpl_kernel_gradients(int64_t n_cells, const int32_t *centre, const int32_t *
 int gpl_kernel_poisson(int32_t nx, int32_t ny, const float *wx, const float *wy, const float *density, float *field_x, float *field_y, int mode, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaSuccess;
-  PoissonPlan *p = poisson_plan_create(nx, ny, wx, wy, mode, &e);
+  PoissonPlan *p = poisson_plan_create(nx, ny, wx, wy, mode, &e, true, s);
   if (!p) return (int)e;
   int ld = 0;
   __nv_bfloat16 *split = poisson_split_input(p, &ld);

@@ -197,7 +197,7 @@ __global__ void k_hold_locked(RegionArgs r, CellArgs c);
 // The density solver (Fft::solve without the potential): FP32 SIMT GEMMs or split-BF16
 // tcgen05 GEMMs. Workspace layout and basis matrices are the solver's own.
 struct PoissonPlan;
-PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const float *wy_host, int mode, cudaError_t *err);
+PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const float *wy_host, int mode, cudaError_t *err, bool scratch = false, cudaStream_t s = nullptr);
 void poisson_plan_destroy(PoissonPlan *p);
 cudaError_t poisson_solve(PoissonPlan *p, const float *density, float *field_x, float *field_y, cudaStream_t s);
 // The split-BF16 density operand the bin finalize can write directly (NULL in FP32 mode).

@@ -27,9 +27,9 @@
 #include "engine_kernels.h"
 #include "poisson_internal.h"
 #include "parallel.h"
+#include "scratch.h"
 
 namespace gpl {
-void progress(const char *fmt, ...) __attribute__((format(printf, 1, 2)));
 
 // ---------------------------------------------------------------- FP32 SIMT GEMM
 // 128 x 64 output tile per block, K-step 8, 256 threads with 8 x 4 outputs each.
@@ -347,43 +347,109 @@ __global__ void k_convert(int64_t n, const A *__restrict__ in, B *__restrict__ o
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) out[k] = (B)in[k];
 }
 
-// ---------------------------------------------------------------- basis matrices (host)
-// Built in double from exact arguments, rounded once.
-void build_basis(int nx, int ny, BasisHost &b) {
-  auto cosv = [](int k, int j, int n) { return std::cos(M_PI * (double)k * ((double)j + 0.5) / (double)n); };
-  auto sinv = [](int k, int j, int n) { return k == 0 ? ((j & 1) ? -1.0 : 1.0) : std::sin(M_PI * (double)k * ((double)j + 0.5) / (double)n); };
-  b.CyTs.assign((size_t)ny * ny, 0);
-  b.Cy.assign((size_t)ny * ny, 0);
-  b.Sy.assign((size_t)ny * ny, 0);
-  parallel_for((size_t)ny, [&](size_t v0, size_t v1) {
-    for (int v = (int)v0; v < (int)v1; v++)
-      for (int y = 0; y < ny; y++) {
-        double h = (v == 0 ? 0.5 : 1.0) * 2.0 / (double)ny;
-        b.CyTs[(size_t)v * ny + y] = h * cosv(v, y, ny);
-        b.Cy[(size_t)y * ny + v] = cosv(v, y, ny);
-        b.Sy[(size_t)y * ny + v] = sinv(v, y, ny);
-      }
-  }, 16);
-  b.CxTs.assign((size_t)nx * nx, 0);
-  b.Cx.assign((size_t)nx * nx, 0);
-  b.Sx.assign((size_t)nx * nx, 0);
-  parallel_for((size_t)nx, [&](size_t u0, size_t u1) {
-    for (int u = (int)u0; u < (int)u1; u++)
-      for (int x = 0; x < nx; x++) {
-        double h = (u == 0 ? 0.5 : 1.0) * 2.0 / (double)nx;
-        b.CxTs[(size_t)u * nx + x] = h * cosv(u, x, nx);
-        b.Cx[(size_t)x * nx + u] = cosv(u, x, nx);
-        b.Sx[(size_t)x * nx + u] = sinv(u, x, nx);
-      }
-  }, 16);
+// ---------------------------------------------------------------- basis matrices
+// The host library's cosine and sine in double, the arguments exact products of the reference's
+// order, rounded once to the form's type.
+static double cos_entry(int k, int j, int n) { return std::cos(M_PI * (double)k * ((double)j + 0.5) / (double)n); }
+static double sin_entry(int k, int j, int n) { return k == 0 ? ((j & 1) ? -1.0 : 1.0) : std::sin(M_PI * (double)k * ((double)j + 0.5) / (double)n); }
+// Entry (r, c) of a basis matrix of side n.
+static double basis_entry(int which, int r, int c, int n) {
+  if (which == B_CYTS || which == B_CXTS) {
+    const double h = (r == 0 ? 0.5 : 1.0) * 2.0 / (double)n;
+    return h * cos_entry(r, c, n);
+  }
+  return which == B_SY || which == B_SX ? sin_entry(c, r, n) : cos_entry(c, r, n);
 }
 
-static cudaError_t upload_f32(const std::vector<double> &h, float **d) {
-  std::vector<float> f(h.size());
-  for (size_t i = 0; i < h.size(); i++) f[i] = (float)h[i];
-  cudaError_t e = pool_alloc((void **)d, f.size() * sizeof(float));
+void build_basis(int nx, int ny, BasisHost &b) {
+  for (int w = 0; w < B_COUNT; w++) {
+    const int n = basis_of_x(w) ? nx : ny;
+    b.m[w].assign((size_t)n * n, 0);
+    parallel_for((size_t)n, [&](size_t r0, size_t r1) {
+      for (int r = (int)r0; r < (int)r1; r++)
+        for (int c = 0; c < n; c++) b.m[w][(size_t)r * n + c] = basis_entry(w, r, c, n);
+    }, 16);
+  }
+}
+
+// The float forms' matrices on the device. An entry's argument is the host's bit for bit (IEEE
+// products and quotient), and the device's cosine and sine are within a few ulp of it, as the
+// host library's are; where every double that near rounds to one float, that float is the
+// host's. The few entries left (one in 10^7) are listed and taken from the host library. On
+// the host the six matrices of a 1024 x 1024 grid took 12 ms on its threads and 4 ms to upload
+// 25 MB; here 0.1 ms.
+constexpr int kMaxUnsure = 1 << 16;
+struct Unsure {
+  unsigned int count, pad[3];
+  int4 at[kMaxUnsure];  // matrix, row, column
+};
+__device__ __forceinline__ void basis_store(const BasisOut &out, int w, int n, int r, int c, float x) {
+  if (out.f32[w]) out.f32[w][(size_t)r * n + c] = x;
+  if (out.split[w]) {
+    const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+    out.split[w][(size_t)r * 2 * n + c] = hi;
+    out.split[w][(size_t)r * 2 * n + n + c] = __float2bfloat16_rn(x - __bfloat162float(hi));
+  }
+}
+__global__ void __launch_bounds__(256) k_basis(int nx, int ny, BasisOut out, Unsure *unsure) {
+  const int w = blockIdx.z;
+  const bool x_side = w == B_CXTS || w == B_SX || w == B_CX;
+  const int n = x_side ? nx : ny;
+  const int r = blockIdx.y;
+  if (r >= n) return;
+  for (int c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
+    const bool fwd = w == B_CYTS || w == B_CXTS;
+    const int k = fwd ? r : c, j = fwd ? c : r;
+    const double a = __ddiv_rn(__dmul_rn(__dmul_rn(M_PI, (double)k), __dadd_rn((double)j, 0.5)), (double)n);
+    double v;
+    if (w == B_SY || w == B_SX)
+      v = k == 0 ? ((j & 1) ? -1.0 : 1.0) : sin(a);
+    else
+      v = cos(a);
+    if (fwd) v = __dmul_rn(__ddiv_rn(__dmul_rn(r == 0 ? 0.5 : 1.0, 2.0), (double)n), v);
+    const double e = fabs(v) * 0x1p-49;
+    const float x = __double2float_rn(v);
+    if (__double2float_rn(v - e) != x || __double2float_rn(v + e) != x) {
+      const unsigned q = atomicAdd(&unsure->count, 1u);
+      if (q < kMaxUnsure) unsure->at[q] = make_int4(w, r, c, 0);
+    }
+    basis_store(out, w, n, r, c, x);
+  }
+}
+__global__ void k_basis_patch(int nx, int ny, BasisOut out, const Unsure *unsure, const float *x, unsigned count) {
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= count) return;
+  const int4 at = unsure->at[q];
+  const bool x_side = at.x == B_CXTS || at.x == B_SX || at.x == B_CX;
+  basis_store(out, at.x, x_side ? nx : ny, at.y, at.z, x[q]);
+}
+
+cudaError_t device_basis(int nx, int ny, const BasisOut &out, cudaStream_t s) {
+  if (std::max(nx, ny) > 65535) return cudaErrorInvalidValue;  // a row a block; the form's matrices would take 100 GB
+  Scratch buf(sizeof(Unsure), s);
+  cudaError_t e = buf.error();
   if (e != cudaSuccess) return e;
-  return pool_upload(*d, f.data(), f.size() * sizeof(float));
+  Unsure *u = static_cast<Unsure *>(buf.get());
+  if ((e = cudaMemsetAsync(u, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
+  const int n = std::max(nx, ny);
+  k_basis<<<dim3((unsigned)std::min((n + 255) / 256, 8), (unsigned)n, B_COUNT), 256, 0, s>>>(nx, ny, out, u);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  unsigned count = 0;
+  if ((e = cudaMemcpyAsync(&count, u, sizeof count, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+  if (count == 0) return cudaSuccess;
+  if (count > (unsigned)kMaxUnsure) return cudaErrorUnknown;  // cannot happen: one entry in 10^7
+  std::vector<int4> at(count);
+  if ((e = cudaMemcpyAsync(at.data(), u->at, count * sizeof(int4), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+  std::vector<float> x(count);
+  for (unsigned q = 0; q < count; q++) x[q] = (float)basis_entry(at[q].x, at[q].y, at[q].z, basis_of_x(at[q].x) ? nx : ny);
+  Scratch dx(count * sizeof(float), s);
+  if ((e = dx.error()) != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(dx.get(), x.data(), count * sizeof(float), cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
+  k_basis_patch<<<(count + 255) / 256, 256, 0, s>>>(nx, ny, out, u, static_cast<const float *>(dx.get()), count);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return cudaStreamSynchronize(s);  // the host values have been read
 }
 
 size_t poisson_workspace_bytes(int nx, int ny) {
@@ -392,7 +458,10 @@ size_t poisson_workspace_bytes(int nx, int ny) {
   return (basis + 5 * n) * sizeof(float) + 2 * (size_t)(nx + ny) * sizeof(float);
 }
 
-PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const float *wy_host, int mode, cudaError_t *err) {
+// One arena holds the plan: from the device's default pool (an engine's plans: kept warm by its
+// release threshold), ordered on the legacy stream and complete when the create returns; or
+// (scratch) from the entry points' own pool, ordered on the call's stream.
+PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const float *wy_host, int mode, cudaError_t *err, bool scratch, cudaStream_t s) {
   PoissonPlan *p = new PoissonPlan();
   p->nx = nx;
   p->ny = ny;
@@ -400,78 +469,79 @@ PoissonPlan *poisson_plan_create(int nx, int ny, const float *wx_host, const flo
   // multiples of 128 (small or odd -bin_grid_count grids) is solved with the FP32 GEMMs
   if (mode == 1 && (nx % 128 != 0 || ny % 128 != 0)) mode = 0;
   p->mode = mode;
+  p->scratch = scratch;
+  p->stream = s;
   *err = cudaSuccess;
-  std::vector<float> w2((size_t)nx + ny);
-  BasisHost b;
-  build_basis(nx, ny, b);
-  if (nx >= 512) progress("    plan: bases built");
-  size_t n = (size_t)nx * ny;
-#define TRY(x)              \
-  do {                      \
-    cudaError_t e_ = (x);   \
-    if (e_ != cudaSuccess) { \
-      *err = e_;            \
-      poisson_plan_destroy(p); \
-      return nullptr;       \
-    }                       \
-  } while (0)
-  TRY(pool_alloc((void **)&p->wx, nx * sizeof(float)));
-  TRY(pool_alloc((void **)&p->wx2, nx * sizeof(float)));
-  TRY(pool_alloc((void **)&p->wy, ny * sizeof(float)));
-  TRY(pool_alloc((void **)&p->wy2, ny * sizeof(float)));
-  std::vector<float> sq(std::max(nx, ny));
-  for (int i = 0; i < nx; i++) sq[i] = wx_host[i] * wx_host[i];
-  TRY(pool_upload(p->wx, wx_host, nx * sizeof(float)));
-  TRY(pool_upload(p->wx2, sq.data(), nx * sizeof(float)));
-  for (int i = 0; i < ny; i++) sq[i] = wy_host[i] * wy_host[i];
-  TRY(pool_upload(p->wy, wy_host, ny * sizeof(float)));
-  TRY(pool_upload(p->wy2, sq.data(), ny * sizeof(float)));
-  if (mode == 2) {
-    const std::vector<double> *mats[6] = {&b.CyTs, &b.CxTs, &b.Cy, &b.Sy, &b.Sx, &b.Cx};
-    for (int k = 0; k < 6; k++) {
-      TRY(pool_alloc((void **)&p->d_basis[k], mats[k]->size() * sizeof(double)));
-      TRY(pool_upload(p->d_basis[k], mats[k]->data(), mats[k]->size() * sizeof(double)));
+  const size_t n = (size_t)nx * ny, xx = (size_t)nx * nx, yy = (size_t)ny * ny;
+  auto side2 = [&](int w) { return basis_of_x(w) ? xx : yy; };
+  // the arena's layout, twice: its size, then the pointers
+  char *base = nullptr;
+  size_t at = 0;
+  auto take = [&](auto **ptr, size_t count) {
+    using E = typename std::remove_pointer<typename std::remove_reference<decltype(*ptr)>::type>::type;
+    if (base) *ptr = reinterpret_cast<E *>(base + at);
+    at += (count * sizeof(E) + 255) / 256 * 256;
+  };
+  float *w_all = nullptr;
+  BasisOut out{};
+  auto layout = [&]() {
+    at = 0;
+    take(&w_all, 2 * (size_t)(nx + ny));
+    if (mode == 2) {
+      for (int k = 0; k < B_COUNT; k++) take(&p->d_basis[k], side2(k));
+      for (int k = 0; k < 8; k++) take(&p->d_buf[k], n);
+    } else if (mode == 0) {
+      for (int k = 0; k < B_COUNT; k++) take(&out.f32[k], side2(k));
+      for (float **b : {&p->t1, &p->exh, &p->eyh, &p->t2, &p->t3}) take(b, n);
+    } else {
+      char *tc = nullptr;
+      take(&tc, tc_plan_bytes(nx, ny));
+      if (tc) *err = tc_plan_init(p, tc, out);
     }
-    for (int k = 0; k < 8; k++) TRY(pool_alloc((void **)&p->d_buf[k], n * sizeof(double)));
-  } else if (mode == 0) {
-    TRY(upload_f32(b.CyTs, &p->CyTs));
-    TRY(upload_f32(b.CxTs, &p->CxTs));
-    TRY(upload_f32(b.Cy, &p->Cy));
-    TRY(upload_f32(b.Sy, &p->Sy));
-    TRY(upload_f32(b.Sx, &p->Sx));
-    TRY(upload_f32(b.Cx, &p->Cx));
-    TRY(pool_alloc((void **)&p->t1, n * sizeof(float)));
-    TRY(pool_alloc((void **)&p->exh, n * sizeof(float)));
-    TRY(pool_alloc((void **)&p->eyh, n * sizeof(float)));
-    TRY(pool_alloc((void **)&p->t2, n * sizeof(float)));
-    TRY(pool_alloc((void **)&p->t3, n * sizeof(float)));
-  } else {
-    if (nx >= 512) progress("    plan: wavenumbers uploaded");
-    cudaError_t e = tc_plan_init(p, b);
-    if (e != cudaSuccess) {
-      *err = e;
-      poisson_plan_destroy(p);
-      return nullptr;
-    }
-  }
-#undef TRY
-  if ((*err = cudaStreamSynchronize(0)) != cudaSuccess) {
+  };
+  auto fail = [&]() -> PoissonPlan * {
     poisson_plan_destroy(p);
     return nullptr;
+  };
+  layout();
+  *err = scratch ? scratch_alloc(&p->arena, at, s) : cudaMallocAsync(&p->arena, at, s);
+  if (*err != cudaSuccess) return fail();
+  base = static_cast<char *>(p->arena);
+  layout();
+  if (*err != cudaSuccess) return fail();
+  p->wx = w_all;
+  p->wx2 = w_all + nx;
+  p->wy = w_all + 2 * (size_t)nx;
+  p->wy2 = p->wy + ny;
+  std::vector<float> w((size_t)2 * (nx + ny));
+  for (int i = 0; i < nx; i++) w[i] = wx_host[i], w[nx + i] = wx_host[i] * wx_host[i];
+  for (int i = 0; i < ny; i++) w[2 * nx + i] = wy_host[i], w[2 * nx + ny + i] = wy_host[i] * wy_host[i];
+  *err = cudaMemcpyAsync(w_all, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice, s);
+  if (*err == cudaSuccess && mode == 2) {
+    BasisHost b;
+    build_basis(nx, ny, b);
+    for (int k = 0; k < B_COUNT && *err == cudaSuccess; k++) *err = cudaMemcpyAsync(p->d_basis[k], b.m[k].data(), b.m[k].size() * sizeof(double), cudaMemcpyHostToDevice, s);
+    if (*err == cudaSuccess) *err = cudaStreamSynchronize(s);
+  } else if (*err == cudaSuccess) {
+    *err = device_basis(nx, ny, out, s);  // synchronises: the copies above have been read
   }
+  if (*err != cudaSuccess) return fail();
+  p->CyTs = out.f32[B_CYTS];
+  p->CxTs = out.f32[B_CXTS];
+  p->Cy = out.f32[B_CY];
+  p->Sy = out.f32[B_SY];
+  p->Sx = out.f32[B_SX];
+  p->Cx = out.f32[B_CX];
   return p;
 }
 
 void poisson_plan_destroy(PoissonPlan *p) {
   if (!p) return;
-  cudaDeviceSynchronize();
-  float *bufs[] = {p->wx, p->wx2, p->wy, p->wy2, p->CyTs, p->CxTs, p->Cy, p->Sy, p->Sx, p->Cx, p->t1, p->exh, p->eyh, p->t2, p->t3};
-  for (float *b : bufs)
-    pool_free(b);
-  for (double *b : p->d_basis)
-    pool_free(b);
-  for (double *b : p->d_buf)
-    pool_free(b);
+  if (p->arena) {
+    // an engine's plan may have been used on any of its streams
+    if (!p->scratch) cudaDeviceSynchronize();
+    cudaFreeAsync(p->arena, p->stream);
+  }
   tc_plan_free(p);
   delete p;
 }
@@ -645,3 +715,23 @@ void load_module_poisson() {
 }
 
 }  // namespace gpl
+
+// Test-only: the six matrices the device makes, in float, one after the other into host memory
+// (sides ny, nx, ny, ny, nx, nx).
+extern "C" int gpl_rules_basis(int32_t nx, int32_t ny, float *out) {
+  using namespace gpl;
+  if (nx <= 0 || ny <= 0) return (int)cudaErrorInvalidValue;
+  const size_t xx = (size_t)nx * nx, yy = (size_t)ny * ny;
+  Scratch buf(3 * (xx + yy) * sizeof(float), 0);
+  cudaError_t e = buf.error();
+  if (e != cudaSuccess) return (int)e;
+  BasisOut o{};
+  size_t at = 0;
+  for (int k = 0; k < B_COUNT; k++) {
+    o.f32[k] = static_cast<float *>(buf.get()) + at;
+    at += basis_of_x(k) ? xx : yy;
+  }
+  e = device_basis(nx, ny, o, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(out, buf.get(), at * sizeof(float), cudaMemcpyDeviceToHost);
+  return (int)e;
+}

@@ -320,23 +320,12 @@ struct TcState {
   CUtensorMap mExh, mEyh, mT2, mT3;              // B operands of the batched pairs (128-row boxes)
 };
 
-static cudaError_t upload_split(const std::vector<double> &h, int rows, int k, __nv_bfloat16 **d) {
-  std::vector<__nv_bfloat16> v((size_t)rows * 2 * k);
-  parallel_for((size_t)rows, [&](size_t r0, size_t r1) {
-    for (size_t r = r0; r < r1; r++)
-      for (int c = 0; c < k; c++) {
-        float x = (float)h[r * k + c];
-        __nv_bfloat16 hi = __float2bfloat16_rn(x);
-        v[r * 2 * k + c] = hi;
-        v[r * 2 * k + k + c] = __float2bfloat16_rn(x - __bfloat162float(hi));
-      }
-  }, 16);
-  cudaError_t e = pool_alloc((void **)d, v.size() * sizeof(__nv_bfloat16));
-  if (e != cudaSuccess) return e;
-  return pool_upload(*d, v.data(), v.size() * sizeof(__nv_bfloat16));
+size_t tc_plan_bytes(int nx, int ny) {
+  // three split matrices a side, six split operands of the grid, the error word
+  return (3 * ((size_t)nx * nx + (size_t)ny * ny) + 6 * (size_t)nx * ny) * 2 * sizeof(__nv_bfloat16) + 256;
 }
 
-cudaError_t tc_plan_init(PoissonPlan *p, const BasisHost &b) {
+cudaError_t tc_plan_init(PoissonPlan *p, char *base, BasisOut &out) {
   int nx = p->nx, ny = p->ny;
   if (nx % 128 != 0 || ny % 128 != 0) return cudaErrorNotSupported;
   TcState *t = new TcState();
@@ -346,22 +335,28 @@ cudaError_t tc_plan_init(PoissonPlan *p, const BasisHost &b) {
   do {                                    \
     if ((e = (x)) != cudaSuccess) return e; \
   } while (0)
-  TRY(upload_split(b.CyTs, ny, ny, &t->CyTs));
-  TRY(upload_split(b.CxTs, nx, nx, &t->CxTs));
-  TRY(upload_split(b.Cy, ny, ny, &t->Cy));
-  TRY(upload_split(b.Sy, ny, ny, &t->Sy));
-  TRY(upload_split(b.Sx, nx, nx, &t->Sx));
-  TRY(upload_split(b.Cx, nx, nx, &t->Cx));
-  size_t n = (size_t)nx * ny * 2;
-  TRY(pool_alloc((void **)&p->tc_dens, n * sizeof(__nv_bfloat16)));
-  TRY(pool_alloc((void **)&t->t1, n * sizeof(__nv_bfloat16)));
-  TRY(pool_alloc((void **)&t->exh, n * sizeof(__nv_bfloat16)));
-  TRY(pool_alloc((void **)&t->eyh, n * sizeof(__nv_bfloat16)));
-  TRY(pool_alloc((void **)&t->t2, n * sizeof(__nv_bfloat16)));
-  TRY(pool_alloc((void **)&t->t3, n * sizeof(__nv_bfloat16)));
-  TRY(cudaMemsetAsync(p->tc_dens, 0, n * sizeof(__nv_bfloat16), 0));
-  TRY(pool_alloc((void **)&t->err, sizeof(int)));
-  TRY(cudaMemsetAsync(t->err, 0, sizeof(int), 0));
+  // sides of multiples of 128: every part is a multiple of 256 bytes
+  auto take = [&](size_t elems) {
+    __nv_bfloat16 *q = reinterpret_cast<__nv_bfloat16 *>(base);
+    base += elems * 2 * sizeof(__nv_bfloat16);
+    return q;
+  };
+  const size_t xx = (size_t)nx * nx, yy = (size_t)ny * ny, n = (size_t)nx * ny;
+  out.split[B_CYTS] = t->CyTs = take(yy);
+  out.split[B_CXTS] = t->CxTs = take(xx);
+  out.split[B_CY] = t->Cy = take(yy);
+  out.split[B_SY] = t->Sy = take(yy);
+  out.split[B_SX] = t->Sx = take(xx);
+  out.split[B_CX] = t->Cx = take(xx);
+  p->tc_dens = take(n);
+  t->t1 = take(n);
+  t->exh = take(n);
+  t->eyh = take(n);
+  t->t2 = take(n);
+  t->t3 = take(n);
+  t->err = reinterpret_cast<int *>(base);
+  TRY(cudaMemsetAsync(p->tc_dens, 0, n * 2 * sizeof(__nv_bfloat16), p->stream));
+  TRY(cudaMemsetAsync(t->err, 0, sizeof(int), p->stream));
   // A operands [M][2K]: 128-row boxes
   TRY(make_map(&t->mCyTs, t->CyTs, ny, ny, BM));
   TRY(make_map(&t->mCxTs, t->CxTs, nx, nx, BM));
@@ -389,14 +384,7 @@ cudaError_t tc_plan_init(PoissonPlan *p, const BasisHost &b) {
 }
 
 void tc_plan_free(PoissonPlan *p) {
-  pool_free(p->tc_dens);
-  p->tc_dens = nullptr;
-  TcState *t = p->tc;
-  if (!t) return;
-  void *bufs[] = {t->CyTs, t->CxTs, t->Cy, t->Sy, t->Sx, t->Cx, t->t1, t->exh, t->eyh, t->t2, t->t3, t->err};
-  for (void *b : bufs)
-    pool_free(b);
-  delete t;
+  delete p->tc;
   p->tc = nullptr;
 }
 
