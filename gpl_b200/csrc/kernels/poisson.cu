@@ -31,82 +31,6 @@
 
 namespace gpl {
 
-// ---------------------------------------------------------------- FP32 SIMT GEMM
-// 128 x 64 output tile per block, K-step 8, 256 threads with 8 x 4 outputs each.
-constexpr int SG_BM = 128, SG_BN = 64, SG_BK = 8;
-
-// One 128 x 64 output tile of D = A B^T from (m0, n0).
-template <typename T>
-__device__ __forceinline__ void gemm_tile(const GemmProblemT<T> &P, const int m0, const int n0) {
-  __shared__ __align__(16) T As[SG_BK][SG_BM + 4];
-  __shared__ __align__(16) T Bs[SG_BK][SG_BN + 4];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int ar = tid >> 1, ak = (tid & 1) * 4;  // A loader: row, first k
-  const int br = tid >> 2, bk = (tid & 3) * 2;  // B loader
-  T acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = (T)0;
-  T ra[4], rb[2];
-  auto load = [&](int k0) {
-    int gm = m0 + ar;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      int gk = k0 + ak + q;
-      ra[q] = (gm < P.M && gk < P.K) ? P.A[(size_t)gm * P.lda + gk] : (T)0;
-    }
-    int gn = n0 + br;
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      int gk = k0 + bk + q;
-      rb[q] = (gn < P.N && gk < P.K) ? P.B[(size_t)gn * P.ldb + gk] : (T)0;
-    }
-  };
-  load(0);
-  for (int k0 = 0; k0 < P.K; k0 += SG_BK) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) As[ak + q][ar] = ra[q];
-#pragma unroll
-    for (int q = 0; q < 2; q++) Bs[bk + q][br] = rb[q];
-    __syncthreads();
-    if (k0 + SG_BK < P.K) load(k0 + SG_BK);
-#pragma unroll
-    for (int kk = 0; kk < SG_BK; kk++) {
-      T a[8], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        a[q] = As[kk][ty * 4 + q];
-        a[4 + q] = As[kk][64 + ty * 4 + q];
-        b[q] = Bs[kk][tx * 4 + q];
-      }
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-    if (gm >= P.M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      int gn = n0 + tx * 4 + j;
-      if (gn < P.N) P.D[(size_t)gm * P.ldd + gn] = acc[i][j];
-    }
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_gemm_tn(GemmBatchT<T> gb) {
-  const GemmProblemT<T> P = gb.p[blockIdx.z];
-  const int m0 = blockIdx.y * SG_BM, n0 = blockIdx.x * SG_BN;
-  if (m0 >= P.M || n0 >= P.N) return;
-  gemm_tile<T>(P, m0, n0);
-}
-
 // ---------------------------------------------------------------- FP32, spread over the SMs
 // BM x BN output tile per block, K in chunks of 32 through two shared buffers (the next chunk's
 // loads in flight beside the current one's products), TM x 4 outputs a thread, pairs of rows in
@@ -293,15 +217,100 @@ __global__ void __launch_bounds__((BM / TM) * (BN / 4)) k_gemm_grouped(const Gem
   gemm_tile_f32<BM, BN, TM>(P, E, (t / tn) * BM, (t % tn) * BN);
 }
 
-template <typename T>
-cudaError_t gemm_tn(const GemmBatchT<T> &gb, int count, cudaStream_t s) {
+// ---------------------------------------------------------------- FP64
+// The same in double (the check paths: the FP64 solve, the density objective) on the double
+// tensor path (mma m8n8k4), whose result is the chain of fused multiply-adds over k in order bit
+// for bit: 64 x 32 tiles, a warp 32 x 16 of it, K in chunks of 16 through a ring of three
+// asynchronous copies (two chunks in flight cover the round trip to L2). Rows are padded to 20
+// values, so a fragment's 8 x 4 reads meet no bank conflict.
+// 512 x 512 x 512: 21 us (94 in 32 tiles of 128 x 64 with eight-wide steps; 30 with these
+// tiles in scalar multiply-adds); the chip's double rate bounds it at 7.
+constexpr int DG_BM = 64, DG_BN = 32, DG_BK = 16, DG_NT = 128, DG_LD = DG_BK + 4, DG_STAGES = 3;
+
+// One chunk of an operand into shared memory: asynchronously in pairs, or (an odd K or a base
+// off 16 bytes) value by value.
+template <int R>
+__device__ __forceinline__ void dg_fetch(double *s, const double *__restrict__ A, int lda, int r0, int rows, int k0, int K, bool vec) {
+  constexpr int PAIRS = R * DG_BK / 2;
+#pragma unroll
+  for (int i = 0; i < (PAIRS + DG_NT - 1) / DG_NT; i++) {
+    const int e = threadIdx.x + i * DG_NT, r = e / (DG_BK / 2), k = e % (DG_BK / 2) * 2;
+    if (PAIRS % DG_NT != 0 && e >= PAIRS) break;
+    double *d = s + r * DG_LD + k;
+    const bool in = r0 + r < rows;
+    const double *p = A + (size_t)(in ? r0 + r : 0) * lda + k0 + k;
+    if (vec) {
+      const int bytes = in && k0 + k < K ? 16 : 0;  // the rest of the 16 is zero-filled
+      if (!bytes) p = A;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(p), "r"(bytes) : "memory");
+    } else {
+      d[0] = in && k0 + k < K ? p[0] : 0.0;
+      d[1] = in && k0 + k + 1 < K ? p[1] : 0.0;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(DG_NT) k_dgemm_tn(GemmBatchT<double> gb) {
+  __shared__ __align__(16) double As[DG_STAGES][DG_BM * DG_LD];
+  __shared__ __align__(16) double Bs[DG_STAGES][DG_BN * DG_LD];
+  const GemmProblemT<double> P = gb.p[blockIdx.z];
+  const int m0 = blockIdx.y * DG_BM, n0 = blockIdx.x * DG_BN;
+  if (m0 >= P.M || n0 >= P.N) return;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int wm = (warp / 2) * 32, wn = (warp % 2) * 16;  // the warp's part of the tile
+  const bool vec = ((P.K | P.lda | P.ldb) & 1) == 0 && (((uintptr_t)P.A | (uintptr_t)P.B) & 15) == 0;
+  double acc[4][2][2] = {};
+  const int chunks = (P.K + DG_BK - 1) / DG_BK;
+  auto fetch = [&](int q) {
+    if (q < chunks) {
+      dg_fetch<DG_BM>(As[q % DG_STAGES], P.A, P.lda, m0, P.M, q * DG_BK, P.K, vec);
+      dg_fetch<DG_BN>(Bs[q % DG_STAGES], P.B, P.ldb, n0, P.N, q * DG_BK, P.K, vec);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0);
+  fetch(1);
+  for (int q = 0; q < chunks; q++) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // chunk q is there for every thread, and chunk q - 1's buffer is free
+    fetch(q + 2);
+    const double *as = As[q % DG_STAGES] + (wm + lane / 4) * DG_LD + lane % 4, *bs = Bs[q % DG_STAGES] + (wn + lane / 4) * DG_LD + lane % 4;
+#pragma unroll
+    for (int k = 0; k < DG_BK; k += 4) {
+      double a[4], b[2];
+#pragma unroll
+      for (int i = 0; i < 4; i++) a[i] = as[i * 8 * DG_LD + k];
+#pragma unroll
+      for (int j = 0; j < 2; j++) b[j] = bs[j * 8 * DG_LD + k];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]) : "d"(a[i]), "d"(b[j]));
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int m = m0 + wm + i * 8 + lane / 4;
+    if (m >= P.M) continue;
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int n = n0 + wn + j * 8 + 2 * (lane % 4) + h;
+        if (n < P.N) P.D[(size_t)m * P.ldd + n] = acc[i][j][h];
+      }
+  }
+}
+
+cudaError_t dgemm_tn(const GemmBatchT<double> &gb, int count, cudaStream_t s) {
   int M = 0, N = 0;
   for (int i = 0; i < count; i++) {
-    M = M > gb.p[i].M ? M : gb.p[i].M;
-    N = N > gb.p[i].N ? N : gb.p[i].N;
+    M = std::max(M, gb.p[i].M);
+    N = std::max(N, gb.p[i].N);
   }
-  dim3 grid((N + SG_BN - 1) / SG_BN, (M + SG_BM - 1) / SG_BM, count);
-  k_gemm_tn<T><<<grid, 256, 0, s>>>(gb);
+  k_dgemm_tn<<<dim3((N + DG_BN - 1) / DG_BN, (M + DG_BM - 1) / DG_BM, count), DG_NT, 0, s>>>(gb);
   return cudaGetLastError();
 }
 
@@ -324,7 +333,6 @@ static cudaError_t gemm_f32(const GemmBatch &gb, int count, const GemmEpi &E, cu
   if ((int64_t)((P.M + 127) / 128) * ((P.N + 63) / 64) >= 128) return gemm_f32_launch<128, 64, 8>(gb, count, E, s);
   return gemm_f32_launch<64, 32, 4>(gb, count, E, s);
 }
-cudaError_t dgemm_tn(const GemmBatchT<double> &gb, int count, cudaStream_t s) { return gemm_tn<double>(gb, count, s); }
 
 // The FP64 yardstick's spectral step: the same in double (wavenumbers widened from float).
 __global__ void k_spectral_d(int nx, int ny, const double *__restrict__ ah, const float *__restrict__ wx, const float *__restrict__ wy, double *__restrict__ exh, double *__restrict__ eyh) {
@@ -587,19 +595,19 @@ static cudaError_t solve_fp64(PoissonPlan *p, const float *density, float *field
   k_convert<float, double><<<blocks, 256, 0, s>>>(n, density, rho);
   GemmBatchT<double> g{};
   g.p[0] = GemmProblemT<double>{ny, nx, ny, B[0], ny, rho, ny, t1, nx};
-  cudaError_t e = gemm_tn<double>(g, 1, s);
+  cudaError_t e = dgemm_tn(g, 1, s);
   if (e != cudaSuccess) return e;
   g.p[0] = GemmProblemT<double>{nx, ny, nx, B[1], nx, t1, nx, ah, ny};
-  if ((e = gemm_tn<double>(g, 1, s)) != cudaSuccess) return e;
+  if ((e = dgemm_tn(g, 1, s)) != cudaSuccess) return e;
   k_spectral_d<<<blocks, 256, 0, s>>>(nx, ny, ah, p->wx, p->wy, exh, eyh);
   g.p[0] = GemmProblemT<double>{ny, nx, ny, B[2], ny, exh, ny, t2, nx};
   g.p[1] = GemmProblemT<double>{ny, nx, ny, B[3], ny, eyh, ny, t3, nx};
-  if ((e = gemm_tn<double>(g, 2, s)) != cudaSuccess) return e;
+  if ((e = dgemm_tn(g, 2, s)) != cudaSuccess) return e;
   g.p[0] = GemmProblemT<double>{nx, ny, nx, B[4], nx, t2, nx, f, ny};
-  if ((e = gemm_tn<double>(g, 1, s)) != cudaSuccess) return e;
+  if ((e = dgemm_tn(g, 1, s)) != cudaSuccess) return e;
   k_convert<double, float><<<blocks, 256, 0, s>>>(n, f, field_x);
   g.p[0] = GemmProblemT<double>{nx, ny, nx, B[5], nx, t3, nx, f, ny};
-  if ((e = gemm_tn<double>(g, 1, s)) != cudaSuccess) return e;
+  if ((e = dgemm_tn(g, 1, s)) != cudaSuccess) return e;
   k_convert<double, float><<<blocks, 256, 0, s>>>(n, f, field_y);
   return cudaGetLastError();
 }
