@@ -240,88 +240,88 @@ __global__ void k_bucket(int64_t nt, const int32_t *row, const int32_t *col, con
 // Per row: keys sorted (column, then position; the keys are distinct), each column's run
 // summed in position order (the first value, then the rest added to it), the distinct columns
 // compacted. Tiers by the row's length: a warp per row with its keys in registers (R per
-// lane, bitonic-sorted across the warp) for rows of up to 32, then 64, then 256 keys; a block
-// per row (bitonic sort in shared memory) up to 8192; a block per row merging sorted chunks
-// beyond. Every tier gives the same result.
+// lane, bitonic-sorted across the warp) for rows of up to 32, then 64, then 256 keys; a
+// block per row (sorted in shared memory) up to 8192; a block per row merging
+// sorted chunks beyond. Every tier gives the same result.
 constexpr int kRowTiny = 32, kRowShort = 64, kRowMid = 256;
+constexpr int kTiers = 4;  // after the first
 
 // One column's run [p, end) of a sorted row summed in position order: the first value, then
-// the rest added to it; the values' loads go four at a time ahead of the adds.
-__device__ __forceinline__ float run_sum(const unsigned long long *sk, int p, int end, const float *val) {
-  float s = val[(uint32_t)sk[p]];
+// the rest added to it; v(q) is the value at sorted position q, eight read ahead of the adds.
+// Half of a row's triplets are its diagonal's, so the longest run is half the row: its values
+// are gathered beforehand, every lane at once (see the tiers), or each add would wait for a
+// load.
+template <class V>
+__device__ __forceinline__ float run_sum(V v, int p, int end) {
+  float s = v(p);
   int q = p + 1;
-  for (; q + 4 <= end; q += 4) {
-    float t0 = val[(uint32_t)sk[q]], t1 = val[(uint32_t)sk[q + 1]], t2 = val[(uint32_t)sk[q + 2]], t3 = val[(uint32_t)sk[q + 3]];
-    s = __fadd_rn(s, t0);
-    s = __fadd_rn(s, t1);
-    s = __fadd_rn(s, t2);
-    s = __fadd_rn(s, t3);
+  for (; q + 8 <= end; q += 8) {
+    float t[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) t[u] = v(q + u);
+#pragma unroll
+    for (int u = 0; u < 8; u++) s = __fadd_rn(s, t[u]);
   }
-  for (; q < end; q++) s = __fadd_rn(s, val[(uint32_t)sk[q]]);
+  for (; q < end; q++) s = __fadd_rn(s, v(q));
   return s;
 }
 
-// Sums and compacts a sorted row held in shared memory (sk: m keys), a warp's lanes taking
-// the run starts; returns the row's distinct columns.
-__device__ __forceinline__ int64_t warp_runs(const unsigned long long *sk, int m, int64_t b, const float *val, int32_t *ucol, float *uval) {
+// Sums and compacts a sorted row held in shared memory (m keys sk, their values sv): the warp
+// first lists where the columns' runs start (st), then a lane a run; returns the row's distinct
+// columns. (A lane looking for its run's end key by key waited a load for each.)
+__device__ __forceinline__ int64_t warp_runs(const unsigned long long *sk, const float *sv, uint16_t *st, int m, int64_t b, int32_t *ucol, float *uval) {
   const int lane = threadIdx.x & 31;
-  int64_t base = 0;
+  int n = 0;
   for (int p0 = 0; p0 < m; p0 += 32) {
-    int p = p0 + lane;
-    bool start = p < m && (p == 0 || (uint32_t)(sk[p] >> 32) != (uint32_t)(sk[p - 1] >> 32));
-    unsigned mask = __ballot_sync(0xffffffffu, start);
-    if (start) {
-      unsigned long long key = sk[p];
-      uint32_t c = (uint32_t)(key >> 32);
-      int end = p + 1;
-      while (end < m && (uint32_t)(sk[end] >> 32) == c) end++;
-      float s = run_sum(sk, p, end, val);
-      int64_t u = base + __popc(mask & ((1u << lane) - 1u));
-      ucol[b + u] = (int32_t)c;
-      uval[b + u] = s;
-    }
-    base += __popc(mask);
+    const int p = p0 + lane;
+    const bool start = p < m && (p == 0 || (uint32_t)(sk[p] >> 32) != (uint32_t)(sk[p - 1] >> 32));
+    const unsigned mask = __ballot_sync(0xffffffffu, start);
+    if (start) st[n + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)p;
+    n += __popc(mask);
   }
-  return base;
+  __syncwarp();
+  for (int u = lane; u < n; u += 32) {
+    const int p = st[u], end = u + 1 < n ? st[u + 1] : m;
+    ucol[b + u] = (int32_t)(sk[p] >> 32);
+    uval[b + u] = run_sum([&](int q) { return sv[q]; }, p, end);
+  }
+  return n;
 }
 
-// The same for a block's warps at once (rows of the block tiers): the sorted positions cut
-// into one contiguous section of whole 32-position steps per warp, each warp counting the runs
-// that start in its section, a scan of those counts, then each warp summing and writing its
-// runs (a run that starts in a section may end in the next) from its offset. The distinct
-// columns come out in position order, as warp_runs writes them. Every thread of the block
-// calls it; returns the row's distinct columns.
-__device__ __forceinline__ int64_t block_runs(const unsigned long long *sk, int m, int64_t b, const float *val, int32_t *ucol, float *uval) {
-  __shared__ int64_t counts[kThreads / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// The same by a block of NT threads: its warps each list the starts of a contiguous section
+// (st, after a count and a scan of the sections), then a thread a run. v(q): the value at sorted
+// position q. Every thread of the block calls it; returns the row's distinct columns.
+template <int NT, class V>
+__device__ __forceinline__ int64_t block_runs(const unsigned long long *sk, V v, int32_t *st, int m, int64_t b, int32_t *ucol, float *uval) {
+  __shared__ int32_t counts[NT / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = NT / 32;
   const int steps = (m + 31) / 32, per = (steps + nw - 1) / nw;
-  const int lo = w * per * 32, hi = min(m, (w + 1) * per * 32);
+  const int lo = min(m, w * per * 32), hi = min(m, (w + 1) * per * 32);
   auto starts_at = [&](int p) { return p < hi && (p == 0 || (uint32_t)(sk[p] >> 32) != (uint32_t)(sk[p - 1] >> 32)); };
-  int64_t cnt = 0;
+  int cnt = 0;
   for (int p0 = lo; p0 < hi; p0 += 32) cnt += __popc(__ballot_sync(0xffffffffu, starts_at(p0 + lane)));
   if (lane == 0) counts[w] = cnt;
   __syncthreads();
-  int64_t base = 0, total = 0;
+  int base = 0, n = 0;
   for (int k = 0; k < nw; k++) {
     if (k < w) base += counts[k];
-    total += counts[k];
+    n += counts[k];
   }
   for (int p0 = lo; p0 < hi; p0 += 32) {
     const int p = p0 + lane;
     const bool start = starts_at(p);
     const unsigned mask = __ballot_sync(0xffffffffu, start);
-    if (start) {
-      const uint32_t c = (uint32_t)(sk[p] >> 32);
-      int end = p + 1;
-      while (end < m && (uint32_t)(sk[end] >> 32) == c) end++;
-      const int64_t u = base + __popc(mask & ((1u << lane) - 1u));
-      ucol[b + u] = (int32_t)c;
-      uval[b + u] = run_sum(sk, p, end, val);
-    }
+    if (start) st[base + __popc(mask & ((1u << lane) - 1u))] = p;
     base += __popc(mask);
   }
-  __syncthreads();  // counts free for the block's next row
-  return total;
+  __syncthreads();
+  for (int u = threadIdx.x; u < n; u += NT) {
+    const int p = st[u], end = u + 1 < n ? st[u + 1] : m;
+    ucol[b + u] = (int32_t)(sk[p] >> 32);
+    uval[b + u] = run_sum(v, p, end);
+  }
+  __syncthreads();  // the shared arrays free for the block's next row
+  return n;
 }
 
 // A warp per row of at most 32 R keys: element i = j * 32 + lane lives in register j.
@@ -364,11 +364,14 @@ __device__ __forceinline__ void warp_bitonic(unsigned long long (&v)[R]) {
 // rows of `list`; longer rows go to `next` (with `next_count`) for the next tier.
 template <int R>
 __global__ void __launch_bounds__(kThreads) k_row_collapse_warp(int64_t n, const int32_t *list, const int *count, const int64_t *row_off, const unsigned long long *bucket, const float *val, int32_t *ucol, float *uval, int64_t *ucount, int32_t *next, int *next_count) {
-  __shared__ unsigned long long sk[kThreads / 32][32 * R];
+  constexpr int W = kThreads / 32;
+  __shared__ unsigned long long sk[W][32 * R];
+  __shared__ float sv[W][32 * R];
+  __shared__ uint16_t st[W][32 * R];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t total = list ? (int64_t)*count : n;
-  const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
-  for (int64_t w = blockIdx.x * (int64_t)(kThreads / 32) + wib; w < total; w += warps) {
+  const int64_t warps = (int64_t)gridDim.x * W;
+  for (int64_t w = blockIdx.x * (int64_t)W + wib; w < total; w += warps) {
     const int64_t r = list ? (int64_t)list[w] : w;
     const int64_t b = row_off[r], e = row_off[r + 1];
     const int64_t m = e - b;
@@ -395,18 +398,44 @@ __global__ void __launch_bounds__(kThreads) k_row_collapse_warp(int64_t n, const
     }
     warp_bitonic<R>(v);
 #pragma unroll
-    for (int a = 0; a < R; a++) sk[wib][a * 32 + lane] = v[a];
+    for (int a = 0; a < R; a++) {
+      const int i = a * 32 + lane;
+      sk[wib][i] = v[a];
+      if (i < m) sv[wib][i] = val[(uint32_t)v[a]];
+    }
     __syncwarp();
-    int64_t u = warp_runs(sk[wib], (int)m, b, val, ucol, uval);
+    int64_t u = warp_runs(sk[wib], sv[wib], st[wib], (int)m, b, ucol, uval);
     if (lane == 0) ucount[r] = u;
     __syncwarp();
   }
 }
 
-// Rows of up to kRowLong keys, a block each: the keys bitonic-sorted in shared memory
-// (padded to a power of two), then the block's warps walk the runs. Longer rows go to `next`.
+// N keys (a power of two) in shared memory bitonic-sorted by the block, a thread a pair: a
+// stage is one barrier up to 2048 keys.
+constexpr int kSortThreads = 1024;
+__device__ __forceinline__ void block_sort(unsigned long long *s, int N) {
+  for (int k = 2; k <= N; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int q = threadIdx.x; q < N / 2; q += kSortThreads) {
+        const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1)), o = i | j;
+        const unsigned long long x = s[i], y = s[o];
+        if (((i & k) == 0) ? (x > y) : (x < y)) {
+          s[i] = y;
+          s[o] = x;
+        }
+      }
+      __syncthreads();
+    }
+}
+
+// Rows of up to kRowLong keys, a block each: the keys sorted in shared memory (padded to a
+// power of two), their values gathered beside them, then the block's warps walk the runs.
+// Longer rows go to `next`. Few rows are this long, and the longest one's time is the launch's
+// (400k cells, rows of up to 6700 keys, half of them one column: 520 us a launch with 256
+// threads, the runs' ends searched and their values read one add at a time; 140 now).
 constexpr int kRowLong = 8192;
-__global__ void __launch_bounds__(kThreads) k_row_collapse_block(const int32_t *list, const int *count, const int64_t *row_off, const unsigned long long *bucket, const float *val, int32_t *ucol, float *uval, int64_t *ucount, int32_t *next, int *next_count) {
+constexpr int kRowLongBytes = kRowLong * (int)(sizeof(unsigned long long) + sizeof(float) + sizeof(int32_t));
+__global__ void __launch_bounds__(kSortThreads, 1) k_row_collapse_block(const int32_t *list, const int *count, const int64_t *row_off, const unsigned long long *bucket, const float *val, int32_t *ucol, float *uval, int64_t *ucount, int32_t *next, int *next_count) {
   extern __shared__ unsigned long long skb[];
   const int64_t total = *count;
   for (int64_t w = blockIdx.x; w < total; w += gridDim.x) {
@@ -417,26 +446,15 @@ __global__ void __launch_bounds__(kThreads) k_row_collapse_block(const int32_t *
       if (threadIdx.x == 0) next[atomicAdd(next_count, 1)] = (int32_t)r;
       continue;
     }
-    int N = 1;
+    int N = 2;
     while (N < m) N <<= 1;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) skb[i] = i < m ? bucket[b + i] : ~0ull;
+    for (int i = threadIdx.x; i < N; i += kSortThreads) skb[i] = i < m ? bucket[b + i] : ~0ull;
     __syncthreads();
-    for (int k = 2; k <= N; k <<= 1)
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        for (int i = threadIdx.x; i < N; i += blockDim.x) {
-          const int o = i ^ j;
-          if (o > i) {
-            const bool up = (i & k) == 0;
-            unsigned long long x = skb[i], y = skb[o];
-            if (up ? (x > y) : (x < y)) {
-              skb[i] = y;
-              skb[o] = x;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    const int64_t u = block_runs(skb, (int)m, b, val, ucol, uval);
+    block_sort(skb, N);
+    float *svb = reinterpret_cast<float *>(skb + kRowLong);
+    for (int i = threadIdx.x; i < m; i += kSortThreads) svb[i] = val[(uint32_t)skb[i]];
+    __syncthreads();
+    const int64_t u = block_runs<kSortThreads>(skb, [&](int q) { return svb[q]; }, reinterpret_cast<int32_t *>(svb + kRowLong), (int)m, b, ucol, uval);
     if (threadIdx.x == 0) ucount[r] = u;
     __syncthreads();
   }
@@ -461,7 +479,7 @@ __device__ __forceinline__ void merge_share(const unsigned long long *A, int64_t
   for (int64_t k = d; k < end; k++) out[k] = (j >= lb || (i < la && A[i] < B[j])) ? A[i++] : B[j++];
 }
 
-__global__ void __launch_bounds__(kThreads) k_row_collapse_long(const int32_t *list, const int *count, const int64_t *row_off, unsigned long long *bucket, unsigned long long *scratch, const float *val, int32_t *ucol, float *uval, int64_t *ucount) {
+__global__ void __launch_bounds__(kSortThreads, 1) k_row_collapse_long(const int32_t *list, const int *count, const int64_t *row_off, unsigned long long *bucket, unsigned long long *scratch, const float *val, int32_t *ucol, float *uval, int64_t *ucount) {
   extern __shared__ unsigned long long skl[];
   const int64_t total = *count;
   for (int64_t w = blockIdx.x; w < total; w += gridDim.x) {
@@ -470,26 +488,12 @@ __global__ void __launch_bounds__(kThreads) k_row_collapse_long(const int32_t *l
     unsigned long long *keys = bucket + b, *tmp = scratch + b;
     for (int64_t c0 = 0; c0 < m; c0 += kRowLong) {
       const int cm = (int)(m - c0 < kRowLong ? m - c0 : kRowLong);
-      int N = 1;
+      int N = 2;
       while (N < cm) N <<= 1;
-      for (int i = threadIdx.x; i < N; i += blockDim.x) skl[i] = i < cm ? keys[c0 + i] : ~0ull;
+      for (int i = threadIdx.x; i < N; i += kSortThreads) skl[i] = i < cm ? keys[c0 + i] : ~0ull;
       __syncthreads();
-      for (int k = 2; k <= N; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int i = threadIdx.x; i < N; i += blockDim.x) {
-            const int o = i ^ j;
-            if (o > i) {
-              const bool up = (i & k) == 0;
-              unsigned long long x = skl[i], y = skl[o];
-              if (up ? (x > y) : (x < y)) {
-                skl[i] = y;
-                skl[o] = x;
-              }
-            }
-          }
-          __syncthreads();
-        }
-      for (int i = threadIdx.x; i < cm; i += blockDim.x) keys[c0 + i] = skl[i];
+      block_sort(skl, N);
+      for (int i = threadIdx.x; i < cm; i += kSortThreads) keys[c0 + i] = skl[i];
       __syncthreads();
     }
     unsigned long long *src = keys, *dst = tmp;
@@ -508,7 +512,8 @@ __global__ void __launch_bounds__(kThreads) k_row_collapse_long(const int32_t *l
       for (int64_t i = threadIdx.x; i < m; i += blockDim.x) keys[i] = src[i];
       __syncthreads();
     }
-    const int64_t u = block_runs(keys, (int)m, b, val, ucol, uval);
+    // the merge scratch takes the runs' starts
+    const int64_t u = block_runs<kSortThreads>(keys, [&](int q) { return val[(uint32_t)keys[q]]; }, reinterpret_cast<int32_t *>(tmp), (int)m, b, ucol, uval);
     if (threadIdx.x == 0) ucount[r] = u;
     __syncthreads();
   }
@@ -566,28 +571,37 @@ __global__ void k_scan_block(int64_t *data, int64_t n, int64_t *totals) {
   if (threadIdx.x == kScanBlock - 1) totals[blockIdx.x] = before + x;
 }
 
-// The block totals' exclusive scan: one block of 1024 threads, a chunk of totals each.
+// The block totals' exclusive scan: one block of 1024 threads, a run of totals each, the runs'
+// sums scanned by warps (one thread adding the 1024 of them took 7 us of each scan's 10).
 __global__ void k_scan_totals(int64_t *totals, int64_t nb) {
-  __shared__ int64_t part[kScanBlock];
+  __shared__ int64_t warp_sum[kScanBlock / 32];
   const int64_t per = (nb + kScanBlock - 1) / kScanBlock;
-  const int64_t lo = threadIdx.x * per, hi = min(nb, lo + per);
+  const int64_t lo = min(nb, (int64_t)threadIdx.x * per), hi = min(nb, lo + per);
   int64_t s = 0;
   for (int64_t b = lo; b < hi; b++) s += totals[b];
-  part[threadIdx.x] = s;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int64_t x = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sum[w] = x;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t run = 0;
-    for (int t = 0; t < kScanBlock; t++) {
-      int64_t q = part[t];
-      part[t] = run;
-      run += q;
+  if (w == 0) {
+    int64_t q = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, q, o);
+      if (lane >= o) q += y;
     }
-    totals[nb] = run;
+    warp_sum[lane] = q;
   }
   __syncthreads();
-  int64_t run = part[threadIdx.x];
+  int64_t run = (w ? warp_sum[w - 1] : 0) + x - s;
+  if (threadIdx.x == kScanBlock - 1) totals[nb] = run + s;
   for (int64_t b = lo; b < hi; b++) {
-    int64_t q = totals[b];
+    const int64_t q = totals[b];
     totals[b] = run;
     run += q;
   }
@@ -806,10 +820,10 @@ cudaError_t IpDevice::upload(const IpSetup &s) {
   CK(alloc(&cnt_, 4 * ((size_t)n_nets_ + 1), s_));
   CK(alloc(&row_off_, n_ + 1, s_));
   CK(alloc(&ucount_, n_ + 1, s_));
-  CK(cudaFuncSetAttribute(k_row_collapse_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLong * (int)sizeof(unsigned long long)));
+  CK(cudaFuncSetAttribute(k_row_collapse_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLongBytes));
   CK(cudaFuncSetAttribute(k_row_collapse_long, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLong * (int)sizeof(unsigned long long)));
-  CK(alloc(&tier_rows_, 4 * std::max<int64_t>(n_, 1), s_));
-  CK(alloc(&tier_n_, 4, s_));
+  CK(alloc(&tier_rows_, kTiers * std::max<int64_t>(n_, 1), s_));
+  CK(alloc(&tier_n_, kTiers, s_));
   CK(alloc(&fill_, n_, s_));
   CK(alloc(&hpwl_acc_, 1, s_));
   for (auto &a : ax_) {
@@ -860,13 +874,14 @@ cudaError_t IpDevice::collapse(int64_t n_trip, const int32_t *row, const int32_t
   if (n_) {
     // tiers: a warp per row up to 32 keys, then up to 64, then up to 256, a block per row up
     // to 8192, then a block per row merging sorted chunks
-    CK(cudaMemsetAsync(tier_n_, 0, 4 * sizeof(int), s_));
+    CK(cudaMemsetAsync(tier_n_, 0, kTiers * sizeof(int), s_));
     const int wblocks = (int)std::min<int64_t>((n_ + kThreads / 32 - 1) / (kThreads / 32), 148 * 64);
-    k_row_collapse_warp<kRowTiny / 32><<<wblocks, kThreads, 0, s_>>>(n_, nullptr, nullptr, row_off_, bucket_, val, ucol_, uval_, ucount_, tier_rows_, tier_n_);
-    k_row_collapse_warp<kRowShort / 32><<<148 * 16, kThreads, 0, s_>>>(n_, tier_rows_, tier_n_, row_off_, bucket_, val, ucol_, uval_, ucount_, tier_rows_ + n_, tier_n_ + 1);
-    k_row_collapse_warp<kRowMid / 32><<<148 * 4, kThreads, 0, s_>>>(n_, tier_rows_ + n_, tier_n_ + 1, row_off_, bucket_, val, ucol_, uval_, ucount_, tier_rows_ + 2 * n_, tier_n_ + 2);
-    k_row_collapse_block<<<148 * 2, kThreads, kRowLong * sizeof(unsigned long long), s_>>>(tier_rows_ + 2 * n_, tier_n_ + 2, row_off_, bucket_, val, ucol_, uval_, ucount_, tier_rows_ + 3 * n_, tier_n_ + 3);
-    k_row_collapse_long<<<148 * 2, kThreads, kRowLong * sizeof(unsigned long long), s_>>>(tier_rows_ + 3 * n_, tier_n_ + 3, row_off_, bucket_, bucket2_, val, ucol_, uval_, ucount_);
+    auto rows = [&](int tier) { return tier_rows_ + tier * n_; };
+    k_row_collapse_warp<kRowTiny / 32><<<wblocks, kThreads, 0, s_>>>(n_, nullptr, nullptr, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(0), tier_n_);
+    k_row_collapse_warp<kRowShort / 32><<<148 * 16, kThreads, 0, s_>>>(n_, rows(0), tier_n_, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(1), tier_n_ + 1);
+    k_row_collapse_warp<kRowMid / 32><<<148 * 4, kThreads, 0, s_>>>(n_, rows(1), tier_n_ + 1, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(2), tier_n_ + 2);
+    k_row_collapse_block<<<148, kSortThreads, kRowLongBytes, s_>>>(rows(2), tier_n_ + 2, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(3), tier_n_ + 3);
+    k_row_collapse_long<<<148, kSortThreads, kRowLong * sizeof(unsigned long long), s_>>>(rows(3), tier_n_ + 3, row_off_, bucket_, bucket2_, val, ucol_, uval_, ucount_);
     launches += 5;
   }
   launches += 2;
@@ -894,13 +909,13 @@ cudaError_t IpDevice::csr_from_triplets(int64_t n, int64_t nt, const int32_t *ro
   release();
   keep_pool_once();
   n_ = n;
-  CK(cudaFuncSetAttribute(k_row_collapse_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLong * (int)sizeof(unsigned long long)));
+  CK(cudaFuncSetAttribute(k_row_collapse_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLongBytes));
   CK(cudaFuncSetAttribute(k_row_collapse_long, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLong * (int)sizeof(unsigned long long)));
   CK(alloc(&row_off_, n_ + 1, s_));
   CK(alloc(&ucount_, n_ + 1, s_));
   CK(alloc(&fill_, n_, s_));
-  CK(alloc(&tier_rows_, 4 * std::max<int64_t>(n_, 1), s_));
-  CK(alloc(&tier_n_, 4, s_));
+  CK(alloc(&tier_rows_, kTiers * std::max<int64_t>(n_, 1), s_));
+  CK(alloc(&tier_n_, kTiers, s_));
   CK(grow(s_, (size_t)std::max<int64_t>(nt, 1), w_cap_, &bucket_, &bucket2_, &ucol_, &uval_));
   size_t cap = (size_t)std::max<int64_t>(nt, 1);  // nnz <= nt: the caller's buffers suffice
   int32_t *c = cols;

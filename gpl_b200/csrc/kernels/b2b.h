@@ -102,7 +102,7 @@ class IpDevice {
   unsigned long long *bucket2_ = nullptr; // the longest rows' merge scratch, as long
   int32_t *fill_ = nullptr;
   int64_t *row_off_ = nullptr, *ucount_ = nullptr;
-  int32_t *tier_rows_ = nullptr;  // [3][n]: rows handed to the collapse's later tiers
+  int32_t *tier_rows_ = nullptr;  // [tiers][n]: rows handed to the collapse's later tiers
   int *tier_n_ = nullptr;         // their counts
   int32_t *ucol_ = nullptr;
   float *uval_ = nullptr;
