@@ -3,7 +3,7 @@
 // src/bicgstab.rs:501-541), BiCGSTAB, `updateCoordi` and the report's HPWL.
 //
 // Bit-exact with the host restatement: every triplet and right-hand-side term is written at
-// the position the host's net loop would append it (per-net counts, an exclusive scan, then
+// the position the host's net loop would append it (per-pin counts, an exclusive scan, then
 // the same loop writing), and each row's duplicates are summed in that order (a row's
 // entries sorted by (column, position)), the first occurrence first, as the reference sums
 // them into the first.
@@ -31,6 +31,8 @@ struct IpArgs {
   const uint8_t *pin_mio;
   const int2 *pin_xy;
   uint8_t *pin_flag;
+  const int32_t *pin_net;
+  int4 *net_ext;
   const int4 *box;
   const uint8_t *locked;
   int32_t max_fanout, min_diff;
@@ -38,171 +40,171 @@ struct IpArgs {
 };
 
 // Where one axis's terms go: triplets (row, col, value) and right-hand-side terms (row,
-// value), each net's run starting at its scanned offset.
+// value), each pin's run starting at its scanned offset.
 struct AxisOut {
   int32_t *t_row, *t_col;
   float *t_val;
   int32_t *r_row;
   float *r_val;
-  const int64_t *t_off, *r_off;  // per net
+  const int64_t *t_off, *r_off;  // per pin
   int64_t t_base;                // the locked diagonal precedes the nets' triplets
 };
 
-// `updatePinInfo` (src/initial_place.rs:203-252): per net, the first strict extreme per side.
+__device__ __forceinline__ int32_t centre(const int4 &b, int axis) { return axis == 0 ? (b.x + b.z) / 2 : (b.y + b.w) / 2; }
+
+// `updatePinInfo` (src/initial_place.rs:203-252): per net, the first strict extreme per side
+// among its solve pins. Each pin's flags, and the net's extreme pins (at most four, from its
+// first pin, in index order, -1 for none).
 __global__ void k_pin_info(IpArgs a) {
   int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.n_nets) return;
-  int64_t b = a.net_start[n], e = a.net_start[n + 1];
+  const int64_t b = a.net_start[n];
+  const int32_t deg = (int32_t)(a.net_start[n + 1] - b);
   int32_t lx = INT32_MAX, ly = INT32_MAX, ux = INT32_MIN, uy = INT32_MIN;
-  int64_t pminx = -1, pmaxx = -1, pminy = -1, pmaxy = -1;
-  for (int64_t k = b; k < e; k++) a.pin_flag[k] = 0;
-  for (int64_t k = b; k < e; k++) {
-    if (a.pin_mio[k]) continue;
-    int2 q = a.pin_xy[k];
-    if (lx > q.x) {
-      if (pminx >= 0) a.pin_flag[pminx] &= (uint8_t)~F_MIN_X;
-      lx = q.x;
-      pminx = k;
-      a.pin_flag[k] |= F_MIN_X;
-    }
-    if (ux < q.x) {
-      if (pmaxx >= 0) a.pin_flag[pmaxx] &= (uint8_t)~F_MAX_X;
-      ux = q.x;
-      pmaxx = k;
-      a.pin_flag[k] |= F_MAX_X;
-    }
-    if (ly > q.y) {
-      if (pminy >= 0) a.pin_flag[pminy] &= (uint8_t)~F_MIN_Y;
-      ly = q.y;
-      pminy = k;
-      a.pin_flag[k] |= F_MIN_Y;
-    }
-    if (uy < q.y) {
-      if (pmaxy >= 0) a.pin_flag[pmaxy] &= (uint8_t)~F_MAX_Y;
-      uy = q.y;
-      pmaxy = k;
-      a.pin_flag[k] |= F_MAX_Y;
-    }
+  int32_t p[4] = {-1, -1, -1, -1};  // min x, max x, min y, max y
+  for (int32_t k = 0; k < deg; k++) {
+    a.pin_flag[b + k] = 0;
+    if (a.pin_mio[b + k]) continue;
+    const int2 q = a.pin_xy[b + k];
+    if (lx > q.x) lx = q.x, p[0] = k;
+    if (ux < q.x) ux = q.x, p[1] = k;
+    if (ly > q.y) ly = q.y, p[2] = k;
+    if (uy < q.y) uy = q.y, p[3] = k;
   }
+  // the distinct extremes in index order, each with its sides
+  int32_t ext[4] = {-1, -1, -1, -1};
+  int32_t last = -1;
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    int32_t next = INT32_MAX;
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+      if (p[s] > last) next = min(next, p[s]);
+    if (next == INT32_MAX) break;
+    uint8_t f = 0;
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+      if (p[s] == next) f |= (uint8_t)(1 << s);
+    a.pin_flag[b + next] = f;
+    ext[e] = last = next;
+  }
+  a.net_ext[n] = make_int4(ext[0], ext[1], ext[2], ext[3]);
 }
 
-__device__ __forceinline__ int32_t centre(const int4 &b, int axis) { return axis == 0 ? (b.x + b.z) / 2 : (b.y + b.w) / 2; }
-
-// One net's pairs in the host's order (the second pin from the second solve pin on, the first
-// below it; x then y): counted (EMIT false) or written at the net's offsets (EMIT true).
-// A pair counts on an axis only when one of its pins is that axis's extreme, so a second pin
-// that is no extreme pairs only with the net's extreme pins: for it the first pin runs over
-// the (at most four) extremes below it, in index order, instead of every pin below it; the
-// pairs visited, and their order, are the reference's, in O(degree) per net.
+// One second pin's pairs in the host's order (the first pin below it, ascending; x then y):
+// counted (EMIT false) or written from the pin's offsets (EMIT true). The host runs over a
+// net's second pins in order, so the pins' runs, one after the other, are its list: a thread a
+// pin. (A thread a net took 0.8 ms to write 400k cells' triplets, its largest net's 64 pins
+// one after the other; 0.3 ms now.) A pair counts on an axis only when one of its pins is that
+// axis's extreme, so a second pin that is no extreme pairs only with the net's extreme pins
+// below it instead of every pin: the pairs visited, and their order, are the reference's, in
+// O(degree) per net.
 template <bool EMIT>
-__device__ void net_pairs(const IpArgs &a, int n, int64_t *cnt, int64_t stride, const AxisOut *out) {
-  int64_t b = a.net_start[n], e = a.net_start[n + 1];
-  int64_t deg = e - b;
+__device__ __forceinline__ void pin_pairs(const IpArgs &a, int64_t k1, int64_t *cnt, int64_t stride, const AxisOut *out) {
   int64_t tpos[2] = {0, 0}, rpos[2] = {0, 0};
-  if (EMIT) {
+  const int32_t n = a.pin_net[k1];
+  const int64_t b = a.net_start[n], deg = a.net_start[n + 1] - b;
+  if (deg > 1 && deg < a.max_fanout && !a.pin_mio[k1]) {
+    if (EMIT) {
 #pragma unroll
-    for (int ax = 0; ax < 2; ax++) {
-      tpos[ax] = out[ax].t_base + out[ax].t_off[n];
-      rpos[ax] = out[ax].r_off[n];
+      for (int ax = 0; ax < 2; ax++) {
+        tpos[ax] = out[ax].t_base + out[ax].t_off[k1];
+        rpos[ax] = out[ax].r_off[k1];
+      }
     }
-  }
-  int64_t tc[2] = {0, 0}, rc[2] = {0, 0};
-  if (deg > 1 && deg < a.max_fanout) {
-    float net_weight = __fdiv_rn(a.weight_scale, (float)(deg - 1));
-    // the net's extreme pins (a pin flagged on any side), in index order; at most four
-    int64_t ext[4];
-    int n_ext = 0;
-    for (int64_t k = b; k < e && n_ext < 4; k++)
-      if (a.pin_flag[k]) ext[n_ext++] = k;
-    for (int64_t k1 = b; k1 < e; k1++) {
-      if (a.pin_mio[k1]) continue;
-      const bool k1_ext = a.pin_flag[k1] != 0;
-      const int64_t n2 = k1_ext ? k1 - b : (int64_t)n_ext;
-      for (int64_t j = 0; j < n2; j++) {
-        const int64_t k2 = k1_ext ? b + j : ext[j];
-        if (k2 >= k1) break;  // the extremes are in index order
-        if (a.pin_mio[k2]) continue;
-        if (a.pin_inst[k1] == a.pin_inst[k2]) continue;
-        uint8_t f = a.pin_flag[k1] | a.pin_flag[k2];
-        int2 q1 = a.pin_xy[k1], q2 = a.pin_xy[k2];
-        int32_t ea = a.pin_e[k1], eb = a.pin_e[k2];
+    const float net_weight = __fdiv_rn(a.weight_scale, (float)(deg - 1));
+    const uint8_t f1 = a.pin_flag[k1];
+    const int2 q1 = a.pin_xy[k1];
+    const int32_t ea = a.pin_e[k1], inst1 = a.pin_inst[k1];
+    const bool la = ea >= 0 && a.locked[ea];
+    const int4 box1 = ea >= 0 ? a.box[ea] : make_int4(0, 0, 0, 0);
+    const int32_t i1 = (int32_t)(k1 - b);
+    const int4 ext = a.net_ext[n];
+    const int32_t n2 = f1 ? i1 : 4;
+    for (int32_t j = 0; j < n2; j++) {
+      int32_t i2 = j;
+      if (!f1) i2 = j == 0 ? ext.x : j == 1 ? ext.y : j == 2 ? ext.z : ext.w;
+      if (i2 < 0 || i2 >= i1) break;  // the extremes are in index order
+      const int64_t k2 = b + i2;
+      if (a.pin_mio[k2]) continue;
+      if (inst1 == a.pin_inst[k2]) continue;
+      const uint8_t f = f1 | a.pin_flag[k2];
+      const int32_t eb = a.pin_e[k2];
+      const bool lb = eb >= 0 && a.locked[eb];
+      const bool fa = ea >= 0 && !la, fb = eb >= 0 && !lb;  // a moving row on that side
+      if (!EMIT) {
+        // two moving rows: four triplets and two terms; a moving row opposite a locked one, or
+        // any row opposite a port: one of each; else none
+        const int nt = fa && fb ? 4 : (fa && lb) || (la && fb) || ((ea < 0) != (eb < 0)) ? 1 : 0;
+        const int nr = nt == 4 ? 2 : nt;
 #pragma unroll
-        for (int axis = 0; axis < 2; axis++) {
-          uint8_t mask = axis == 0 ? (F_MIN_X | F_MAX_X) : (F_MIN_Y | F_MAX_Y);
-          if (!(f & mask)) continue;
-          int32_t c1 = axis == 0 ? q1.x : q1.y, c2 = axis == 0 ? q2.x : q2.y;
-          int32_t diff = abs(c1 - c2);
-          float weight = diff > a.min_diff ? __fdiv_rn(net_weight, (float)diff) : __fdiv_rn(net_weight, (float)a.min_diff);
-          int nt = 0, nr = 0;
-          int32_t rows[4], cols[4], rr[2];
-          float vals[4], rv[2];
-          if (ea >= 0 && eb >= 0) {
-            bool la = a.locked[ea], lb = a.locked[eb];
-            if (!la && !lb) {
-              int32_t ca = centre(a.box[ea], axis), cb = centre(a.box[eb], axis);
-              rows[0] = ea, cols[0] = ea, vals[0] = weight;
-              rows[1] = eb, cols[1] = eb, vals[1] = weight;
-              rows[2] = ea, cols[2] = eb, vals[2] = -weight;
-              rows[3] = eb, cols[3] = ea, vals[3] = -weight;
-              nt = 4;
-              rr[0] = ea, rv[0] = __fmul_rn(-weight, (float)((c1 - ca) - (c2 - cb)));
-              rr[1] = eb, rv[1] = __fmul_rn(-weight, (float)((c2 - cb) - (c1 - ca)));
-              nr = 2;
-            } else if (la && !lb) {
-              int32_t cb = centre(a.box[eb], axis);
-              rows[0] = eb, cols[0] = eb, vals[0] = weight, nt = 1;
-              rr[0] = eb, rv[0] = __fmul_rn(weight, (float)(c1 - (c2 - cb))), nr = 1;
-            } else if (!la && lb) {
-              int32_t ca = centre(a.box[ea], axis);
-              rows[0] = ea, cols[0] = ea, vals[0] = weight, nt = 1;
-              rr[0] = ea, rv[0] = __fmul_rn(weight, (float)(c2 - (c1 - ca))), nr = 1;
-            }
-          } else if (ea < 0 && eb >= 0) {
-            int32_t cb = centre(a.box[eb], axis);
-            rows[0] = eb, cols[0] = eb, vals[0] = weight, nt = 1;
-            rr[0] = eb, rv[0] = __fmul_rn(weight, (float)(c1 - (c2 - cb))), nr = 1;
-          } else if (ea >= 0 && eb < 0) {
-            int32_t ca = centre(a.box[ea], axis);
-            rows[0] = ea, cols[0] = ea, vals[0] = weight, nt = 1;
-            rr[0] = ea, rv[0] = __fmul_rn(weight, (float)(c2 - (c1 - ca))), nr = 1;
-          }
-          if (EMIT) {
-            const AxisOut &o = out[axis];
-            for (int q = 0; q < nt; q++) {
-              int64_t at = tpos[axis]++;
-              o.t_row[at] = rows[q];
-              o.t_col[at] = cols[q];
-              o.t_val[at] = vals[q];
-            }
-            for (int q = 0; q < nr; q++) {
-              int64_t at = rpos[axis]++;
-              o.r_row[at] = rr[q];
-              o.r_val[at] = rv[q];
-            }
-          }
-          tc[axis] += nt;
-          rc[axis] += nr;
+        for (int axis = 0; axis < 2; axis++)
+          if (f & (axis == 0 ? (F_MIN_X | F_MAX_X) : (F_MIN_Y | F_MAX_Y))) tpos[axis] += nt, rpos[axis] += nr;
+        continue;
+      }
+      const int2 q2 = a.pin_xy[k2];
+      const int4 box2 = eb >= 0 ? a.box[eb] : make_int4(0, 0, 0, 0);
+#pragma unroll
+      for (int axis = 0; axis < 2; axis++) {
+        const uint8_t mask = axis == 0 ? (F_MIN_X | F_MAX_X) : (F_MIN_Y | F_MAX_Y);
+        if (!(f & mask)) continue;
+        const int32_t c1 = axis == 0 ? q1.x : q1.y, c2 = axis == 0 ? q2.x : q2.y;
+        const int32_t diff = abs(c1 - c2);
+        const float weight = diff > a.min_diff ? __fdiv_rn(net_weight, (float)diff) : __fdiv_rn(net_weight, (float)a.min_diff);
+        const AxisOut &o = out[axis];
+        auto trip = [&](int32_t row, int32_t col, float v) {
+          const int64_t at = tpos[axis]++;
+          o.t_row[at] = row;
+          o.t_col[at] = col;
+          o.t_val[at] = v;
+        };
+        auto term = [&](int32_t row, float v) {
+          const int64_t at = rpos[axis]++;
+          o.r_row[at] = row;
+          o.r_val[at] = v;
+        };
+        const int32_t ca = centre(box1, axis), cb = centre(box2, axis);
+        if (fa && fb) {
+          trip(ea, ea, weight);
+          trip(eb, eb, weight);
+          trip(ea, eb, -weight);
+          trip(eb, ea, -weight);
+          term(ea, __fmul_rn(-weight, (float)((c1 - ca) - (c2 - cb))));
+          term(eb, __fmul_rn(-weight, (float)((c2 - cb) - (c1 - ca))));
+        } else if ((la && fb) || (ea < 0 && eb >= 0)) {
+          trip(eb, eb, weight);
+          term(eb, __fmul_rn(weight, (float)(c1 - (c2 - cb))));
+        } else if ((fa && lb) || (ea >= 0 && eb < 0)) {
+          trip(ea, ea, weight);
+          term(ea, __fmul_rn(weight, (float)(c2 - (c1 - ca))));
         }
       }
     }
   }
   if (!EMIT) {
-    cnt[n] = tc[0];
-    cnt[stride + n] = tc[1];
-    cnt[2 * stride + n] = rc[0];
-    cnt[3 * stride + n] = rc[1];
+    cnt[k1] = tpos[0];
+    cnt[stride + k1] = tpos[1];
+    cnt[2 * stride + k1] = rpos[0];
+    cnt[3 * stride + k1] = rpos[1];
   }
 }
 
-__global__ void k_count(IpArgs a, int64_t *cnt, int64_t stride) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n < a.n_nets) net_pairs<false>(a, n, cnt, stride, nullptr);
+__global__ void k_count(IpArgs a, int64_t n_pins, int64_t *cnt, int64_t stride) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k < n_pins) pin_pairs<false>(a, k, cnt, stride, nullptr);
 }
 
-__global__ void k_emit(IpArgs a, AxisOut x, AxisOut y) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  AxisOut out[2] = {x, y};
-  if (n < a.n_nets) net_pairs<true>(a, n, nullptr, 0, out);
+__global__ void k_emit(IpArgs a, int64_t n_pins, AxisOut x, AxisOut y) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const AxisOut out[2] = {x, y};
+  if (k < n_pins) pin_pairs<true>(a, k, nullptr, 0, out);
+}
+
+// Each pin's net.
+__global__ void k_pin_net(int32_t n_nets, const int64_t *__restrict__ net_start, int32_t *__restrict__ pin_net) {
+  const int32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= n_nets) return;
+  for (int64_t k = net_start[n]; k < net_start[n + 1]; k++) pin_net[k] = n;
 }
 
 // The locked instances' unit diagonal (first in the triplet list, in instance order), and
@@ -543,7 +545,10 @@ __global__ void k_rhs(int64_t n, int axis, const int4 *box, const uint8_t *locke
 }
 
 // ---- exclusive scan of int64 counts (in place; data[n] receives the total)
-__global__ void k_scan_block(int64_t *data, int64_t n, int64_t *totals) {
+// blockIdx.y: one of several arrays, `stride` apart (their block totals nb + 1 apart).
+__global__ void k_scan_block(int64_t *data, int64_t n, int64_t stride, int64_t *totals) {
+  data += blockIdx.y * stride;
+  totals += blockIdx.y * (int64_t)(gridDim.x + 1);
   __shared__ int64_t warp_sum[kScanBlock / 32];
   int64_t i = blockIdx.x * (int64_t)kScanBlock + threadIdx.x;
   int64_t v = i < n ? data[i] : 0;
@@ -574,6 +579,7 @@ __global__ void k_scan_block(int64_t *data, int64_t n, int64_t *totals) {
 // The block totals' exclusive scan: one block of 1024 threads, a run of totals each, the runs'
 // sums scanned by warps (one thread adding the 1024 of them took 7 us of each scan's 10).
 __global__ void k_scan_totals(int64_t *totals, int64_t nb) {
+  totals += blockIdx.y * (nb + 1);
   __shared__ int64_t warp_sum[kScanBlock / 32];
   const int64_t per = (nb + kScanBlock - 1) / kScanBlock;
   const int64_t lo = min(nb, (int64_t)threadIdx.x * per), hi = min(nb, lo + per);
@@ -607,7 +613,9 @@ __global__ void k_scan_totals(int64_t *totals, int64_t nb) {
   }
 }
 
-__global__ void k_scan_add(int64_t *data, int64_t n, const int64_t *totals, int64_t nb) {
+__global__ void k_scan_add(int64_t *data, int64_t n, int64_t stride, const int64_t *totals, int64_t nb) {
+  data += blockIdx.y * stride;
+  totals += blockIdx.y * (nb + 1);
   int64_t i = blockIdx.x * (int64_t)kScanBlock + threadIdx.x;
   if (i < n) data[i] += totals[blockIdx.x];
   if (i == 0) data[n] = totals[nb];
@@ -757,7 +765,7 @@ IpDevice::~IpDevice() { release(); }
 
 void IpDevice::release() {
   void *ptrs[] = {box_, clamp_, db_box_, pin_static_, db_size_, pin_off_, pin_xy_, locked_, grouped_, pin_mio_, pin_hp_, pin_flag_, pin_e_, pin_inst_, locked_rank_,
-                  net_start_, cnt_, scan_tmp_, t_row_, t_col_, t_val_, r_row_, r_val_, bucket_, bucket2_, fill_, row_off_, ucount_, ucol_, uval_, scratch_, hpwl_acc_, tier_rows_, tier_n_};
+                  net_start_, pin_net_, net_ext_, cnt_, scan_tmp_, t_row_, t_col_, t_val_, r_row_, r_val_, bucket_, bucket2_, fill_, row_off_, ucount_, ucol_, uval_, scratch_, hpwl_acc_, tier_rows_, tier_n_};
   for (void *p : ptrs)
     if (p) cudaFreeAsync(p, s_);
   for (void *p : {(void *)perm_, (void *)inv_, (void *)ord_idx_, (void *)ord_hist_, (void *)ord_key0_, (void *)ord_key1_})
@@ -775,6 +783,8 @@ void IpDevice::release() {
   db_size_ = pin_off_ = pin_xy_ = nullptr;
   locked_ = grouped_ = pin_mio_ = pin_hp_ = pin_flag_ = nullptr;
   pin_e_ = pin_inst_ = locked_rank_ = nullptr;
+  pin_net_ = nullptr;
+  net_ext_ = nullptr;
   net_start_ = cnt_ = scan_tmp_ = row_off_ = ucount_ = nullptr;
   t_row_ = t_col_ = r_row_ = fill_ = ucol_ = nullptr;
   t_val_ = r_val_ = uval_ = nullptr;
@@ -817,7 +827,10 @@ cudaError_t IpDevice::upload(const IpSetup &s) {
   CK(put(&pin_static_, s.pin_static, s_, b));
   CK(put(&net_start_, s.net_start, s_, b));
   CK(alloc(&pin_flag_, n_pins_, s_));
-  CK(alloc(&cnt_, 4 * ((size_t)n_nets_ + 1), s_));
+  CK(alloc(&cnt_, 4 * ((size_t)n_pins_ + 1), s_));
+  CK(alloc(&pin_net_, n_pins_, s_));
+  CK(alloc(&net_ext_, n_nets_, s_));
+  if (n_nets_) k_pin_net<<<grid(n_nets_), kThreads, 0, s_>>>(n_nets_, net_start_, pin_net_);
   CK(alloc(&row_off_, n_ + 1, s_));
   CK(alloc(&ucount_, n_ + 1, s_));
   CK(cudaFuncSetAttribute(k_row_collapse_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowLongBytes));
@@ -842,23 +855,28 @@ size_t scan_i64_tmp(int64_t n) { return (size_t)((n + kScanBlock - 1) / kScanBlo
 cudaError_t scan_i64(int64_t *data, int64_t n, int64_t *tmp, cudaStream_t s) {
   const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
   if (nb == 0) return cudaMemsetAsync(data, 0, sizeof(int64_t), s);
-  k_scan_block<<<(unsigned)nb, kScanBlock, 0, s>>>(data, n, tmp);
+  k_scan_block<<<(unsigned)nb, kScanBlock, 0, s>>>(data, n, 0, tmp);
   k_scan_totals<<<1, kScanBlock, 0, s>>>(tmp, nb);
-  k_scan_add<<<(unsigned)nb, kScanBlock, 0, s>>>(data, n, tmp, nb);
+  k_scan_add<<<(unsigned)nb, kScanBlock, 0, s>>>(data, n, 0, tmp, nb);
   return cudaGetLastError();
 }
 
-cudaError_t IpDevice::scan(int64_t *data, int64_t n) {
+// `arrays` scans at once, the arrays `stride` apart.
+cudaError_t IpDevice::scan(int64_t *data, int64_t n, int arrays, int64_t stride) {
   int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-  if ((size_t)(nb + 1) > scan_tmp_n_) {
+  const size_t need = (size_t)arrays * (size_t)(nb + 1);
+  if (need > scan_tmp_n_) {
     if (scan_tmp_) cudaFreeAsync(scan_tmp_, s_);
-    scan_tmp_n_ = (size_t)(nb + 1);
+    scan_tmp_n_ = need;
     CK(alloc(&scan_tmp_, scan_tmp_n_, s_));
   }
-  if (nb == 0) return cudaMemsetAsync(data, 0, sizeof(int64_t), s_);
-  k_scan_block<<<(unsigned)nb, kScanBlock, 0, s_>>>(data, n, scan_tmp_);
-  k_scan_totals<<<1, kScanBlock, 0, s_>>>(scan_tmp_, nb);
-  k_scan_add<<<(unsigned)nb, kScanBlock, 0, s_>>>(data, n, scan_tmp_, nb);
+  if (nb == 0) {
+    for (int q = 0; q < arrays; q++) CK(cudaMemsetAsync(data + q * stride, 0, sizeof(int64_t), s_));
+    return cudaSuccess;
+  }
+  k_scan_block<<<dim3((unsigned)nb, arrays), kScanBlock, 0, s_>>>(data, n, stride, scan_tmp_);
+  k_scan_totals<<<dim3(1, arrays), kScanBlock, 0, s_>>>(scan_tmp_, nb);
+  k_scan_add<<<dim3((unsigned)nb, arrays), kScanBlock, 0, s_>>>(data, n, stride, scan_tmp_, nb);
   launches += 3;
   return cudaGetLastError();
 }
@@ -934,20 +952,22 @@ cudaError_t IpDevice::assemble(IpAxisResult out[2]) {
   a.pin_mio = pin_mio_;
   a.pin_xy = pin_xy_;
   a.pin_flag = pin_flag_;
+  a.pin_net = pin_net_;
+  a.net_ext = net_ext_;
   a.box = box_;
   a.locked = locked_;
   a.max_fanout = cfg_.max_fanout;
   a.min_diff = cfg_.min_diff;
   a.weight_scale = cfg_.weight_scale;
-  const int64_t stride = (int64_t)n_nets_ + 1;
+  const int64_t stride = n_pins_ + 1;
   if (n_nets_) {
     k_pin_info<<<grid(n_nets_), kThreads, 0, s_>>>(a);
-    k_count<<<grid(n_nets_), kThreads, 0, s_>>>(a, cnt_, stride);
+    if (n_pins_) k_count<<<grid(n_pins_), kThreads, 0, s_>>>(a, n_pins_, cnt_, stride);
     launches += 2;
   }
-  for (int q = 0; q < 4; q++) CK(scan(cnt_ + q * stride, n_nets_));
+  CK(scan(cnt_, n_pins_, 4, stride));
   int64_t tot[4];
-  for (int q = 0; q < 4; q++) CK(cudaMemcpyAsync(&tot[q], cnt_ + q * stride + n_nets_, sizeof(int64_t), cudaMemcpyDeviceToHost, s_));
+  CK(cudaMemcpy2DAsync(tot, sizeof(int64_t), cnt_ + n_pins_, stride * sizeof(int64_t), sizeof(int64_t), 4, cudaMemcpyDeviceToHost, s_));
   CK(cudaStreamSynchronize(s_));
   d2h_bytes += 32;
   const bool first = t_cap_ == 0;
@@ -971,7 +991,7 @@ cudaError_t IpDevice::assemble(IpAxisResult out[2]) {
   oy.r_row = r_row_ + nr[0], oy.r_val = r_val_ + nr[0];
   ox.r_off = cnt_ + 2 * stride, oy.r_off = cnt_ + 3 * stride;
   if (n_) k_locked_and_x0<<<grid(n_), kThreads, 0, s_>>>(n_, box_, locked_, locked_rank_, ox, oy, ax_[0].x, ax_[1].x);
-  if (n_nets_) k_emit<<<grid(n_nets_), kThreads, 0, s_>>>(a, ox, oy);
+  if (n_pins_) k_emit<<<grid(n_pins_), kThreads, 0, s_>>>(a, n_pins_, ox, oy);
   launches += 2;
   CK(cudaGetLastError());
   if (first) {

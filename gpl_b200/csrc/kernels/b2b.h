@@ -92,7 +92,9 @@ class IpDevice {
   int32_t *pin_e_ = nullptr, *pin_inst_ = nullptr, *locked_rank_ = nullptr;
   int64_t *net_start_ = nullptr;
   // counts and offsets, triplets and right-hand-side terms of both axes, the collapse's work
-  int64_t *cnt_ = nullptr;       // [4][n_nets + 1]: triplets x, triplets y, rhs x, rhs y
+  int32_t *pin_net_ = nullptr;   // each pin's net
+  int4 *net_ext_ = nullptr;      // each net's extreme pins
+  int64_t *cnt_ = nullptr;       // [4][n_pins + 1]: triplets x, triplets y, rhs x, rhs y
   int64_t *scan_tmp_ = nullptr;
   size_t scan_tmp_n_ = 0;
   int32_t *t_row_ = nullptr, *t_col_ = nullptr, *r_row_ = nullptr;
@@ -138,7 +140,7 @@ class IpDevice {
   int64_t *hpwl_acc_ = nullptr;
   void release();
   cudaError_t collapse(int64_t n_trip, const int32_t *row, const int32_t *col, const float *val, int64_t *starts_out, int32_t **cols, float **vals, size_t *cap, int64_t *nnz);
-  cudaError_t scan(int64_t *data, int64_t n);
+  cudaError_t scan(int64_t *data, int64_t n, int arrays = 1, int64_t stride = 0);
   cudaError_t slice(Axis &A, CsrDev m);  // the axis's sliced copy of m (its CSR, as solved)
 };
 
