@@ -774,7 +774,7 @@ void IpDevice::release() {
   ord_key0_ = ord_key1_ = nullptr;
   solves_ = 0;
   for (auto &a : ax_) {
-    void *q[] = {a.starts, a.cols, a.vals, a.rhs, a.x, a.sl_row, a.sl_len, a.sl_count, a.sl_start, a.sl_ent, a.p_starts, a.p_cols, a.p_vals, a.p_rhs, a.p_x};
+    void *q[] = {a.row_off, a.ucount, a.ucol, a.uval, a.starts, a.cols, a.vals, a.rhs, a.x, a.sl_row, a.sl_len, a.sl_count, a.sl_start, a.sl_ent, a.p_starts, a.p_cols, a.p_vals, a.p_rhs, a.p_x};
     for (void *p : q)
       if (p) cudaFreeAsync(p, s_);
     a = Axis{};
@@ -793,7 +793,7 @@ void IpDevice::release() {
   hpwl_acc_ = nullptr;
   tier_rows_ = nullptr;
   tier_n_ = nullptr;
-  t_cap_ = r_cap_ = w_cap_ = scan_tmp_n_ = 0;
+  t_cap_ = r_cap_ = w_cap_ = u_cap_ = scan_tmp_n_ = 0;
 }
 
 cudaError_t IpDevice::upload(const IpSetup &s) {
@@ -839,8 +839,11 @@ cudaError_t IpDevice::upload(const IpSetup &s) {
   CK(alloc(&tier_n_, kTiers, s_));
   CK(alloc(&fill_, n_, s_));
   CK(alloc(&hpwl_acc_, 1, s_));
+  read_options();
   for (auto &a : ax_) {
     CK(alloc(&a.starts, n_ + 1, s_));
+    CK(alloc(&a.row_off, n_ + 1, s_));
+    CK(alloc(&a.ucount, n_ + 1, s_));
     CK(alloc(&a.rhs, n_, s_));
     CK(alloc(&a.x, n_, s_));
   }
@@ -881,30 +884,32 @@ cudaError_t IpDevice::scan(int64_t *data, int64_t n, int arrays, int64_t stride)
   return cudaGetLastError();
 }
 
-// Collapses triplets (row, col or one column, val) [0, n_trip) into CSR rows; with no
-// output arrays it stops at the per-row sums (row_off_, ucount_, uval_).
-cudaError_t IpDevice::collapse(int64_t n_trip, const int32_t *row, const int32_t *col, const float *val, int64_t *starts_out, int32_t **cols, float **vals, size_t *cap, int64_t *nnz) {
-  CK(cudaMemsetAsync(row_off_, 0, (n_ + 1) * sizeof(int64_t), s_));
+// Collapses triplets (row, col or one column, val) [0, n_trip) into rows.
+cudaError_t IpDevice::collapse(int64_t n_trip, const int32_t *row, const int32_t *col, const float *val, const Rows &to) {
+  CK(cudaMemsetAsync(to.row_off, 0, (n_ + 1) * sizeof(int64_t), s_));
   CK(cudaMemsetAsync(fill_, 0, std::max<int64_t>(n_, 1) * sizeof(int32_t), s_));
-  if (n_trip) k_row_count<<<grid(n_trip), kThreads, 0, s_>>>(n_trip, row, (unsigned long long *)row_off_);
-  CK(scan(row_off_, n_));
-  if (n_trip) k_bucket<<<grid(n_trip), kThreads, 0, s_>>>(n_trip, row, col, row_off_, fill_, bucket_);
+  if (n_trip) k_row_count<<<grid(n_trip), kThreads, 0, s_>>>(n_trip, row, (unsigned long long *)to.row_off);
+  CK(scan(to.row_off, n_));
+  if (n_trip) k_bucket<<<grid(n_trip), kThreads, 0, s_>>>(n_trip, row, col, to.row_off, fill_, bucket_);
   if (n_) {
     // tiers: a warp per row up to 32 keys, then up to 64, then up to 256, a block per row up
     // to 8192, then a block per row merging sorted chunks
     CK(cudaMemsetAsync(tier_n_, 0, kTiers * sizeof(int), s_));
     const int wblocks = (int)std::min<int64_t>((n_ + kThreads / 32 - 1) / (kThreads / 32), 148 * 64);
     auto rows = [&](int tier) { return tier_rows_ + tier * n_; };
-    k_row_collapse_warp<kRowTiny / 32><<<wblocks, kThreads, 0, s_>>>(n_, nullptr, nullptr, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(0), tier_n_);
-    k_row_collapse_warp<kRowShort / 32><<<148 * 16, kThreads, 0, s_>>>(n_, rows(0), tier_n_, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(1), tier_n_ + 1);
-    k_row_collapse_warp<kRowMid / 32><<<148 * 4, kThreads, 0, s_>>>(n_, rows(1), tier_n_ + 1, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(2), tier_n_ + 2);
-    k_row_collapse_block<<<148, kSortThreads, kRowLongBytes, s_>>>(rows(2), tier_n_ + 2, row_off_, bucket_, val, ucol_, uval_, ucount_, rows(3), tier_n_ + 3);
-    k_row_collapse_long<<<148, kSortThreads, kRowLong * sizeof(unsigned long long), s_>>>(rows(3), tier_n_ + 3, row_off_, bucket_, bucket2_, val, ucol_, uval_, ucount_);
+    k_row_collapse_warp<kRowTiny / 32><<<wblocks, kThreads, 0, s_>>>(n_, nullptr, nullptr, to.row_off, bucket_, val, to.ucol, to.uval, to.ucount, rows(0), tier_n_);
+    k_row_collapse_warp<kRowShort / 32><<<148 * 16, kThreads, 0, s_>>>(n_, rows(0), tier_n_, to.row_off, bucket_, val, to.ucol, to.uval, to.ucount, rows(1), tier_n_ + 1);
+    k_row_collapse_warp<kRowMid / 32><<<148 * 4, kThreads, 0, s_>>>(n_, rows(1), tier_n_ + 1, to.row_off, bucket_, val, to.ucol, to.uval, to.ucount, rows(2), tier_n_ + 2);
+    k_row_collapse_block<<<148, kSortThreads, kRowLongBytes, s_>>>(rows(2), tier_n_ + 2, to.row_off, bucket_, val, to.ucol, to.uval, to.ucount, rows(3), tier_n_ + 3);
+    k_row_collapse_long<<<148, kSortThreads, kRowLong * sizeof(unsigned long long), s_>>>(rows(3), tier_n_ + 3, to.row_off, bucket_, bucket2_, val, to.ucol, to.uval, to.ucount);
     launches += 5;
   }
   launches += 2;
-  if (!cols) return cudaGetLastError();
-  CK(cudaMemcpyAsync(starts_out, ucount_, n_ * sizeof(int64_t), cudaMemcpyDeviceToDevice, s_));
+  return cudaGetLastError();
+}
+
+cudaError_t IpDevice::pack(const Rows &r, int64_t *starts_out, int32_t **cols, float **vals, size_t *cap, int64_t *nnz) {
+  CK(cudaMemcpyAsync(starts_out, r.ucount, n_ * sizeof(int64_t), cudaMemcpyDeviceToDevice, s_));
   CK(scan(starts_out, n_));
   CK(cudaMemcpyAsync(nnz, starts_out + n_, sizeof(int64_t), cudaMemcpyDeviceToHost, s_));
   CK(cudaStreamSynchronize(s_));
@@ -918,7 +923,7 @@ cudaError_t IpDevice::collapse(int64_t n_trip, const int32_t *row, const int32_t
     CK(alloc(cols, *cap, s_));
     CK(alloc(vals, *cap, s_));
   }
-  if (n_) k_row_fill<<<grid(n_), kThreads, 0, s_>>>(n_, row_off_, starts_out, ucol_, uval_, *cols, *vals);
+  if (n_) k_row_fill<<<grid(n_), kThreads, 0, s_>>>(n_, r.row_off, starts_out, r.ucol, r.uval, *cols, *vals);
   launches += 1;
   return cudaGetLastError();
 }
@@ -934,11 +939,14 @@ cudaError_t IpDevice::csr_from_triplets(int64_t n, int64_t nt, const int32_t *ro
   CK(alloc(&fill_, n_, s_));
   CK(alloc(&tier_rows_, kTiers * std::max<int64_t>(n_, 1), s_));
   CK(alloc(&tier_n_, kTiers, s_));
-  CK(grow(s_, (size_t)std::max<int64_t>(nt, 1), w_cap_, &bucket_, &bucket2_, &ucol_, &uval_));
+  CK(grow(s_, (size_t)std::max<int64_t>(nt, 1), w_cap_, &bucket_, &bucket2_));
+  CK(grow(s_, (size_t)std::max<int64_t>(nt, 1), u_cap_, &ucol_, &uval_));
   size_t cap = (size_t)std::max<int64_t>(nt, 1);  // nnz <= nt: the caller's buffers suffice
   int32_t *c = cols;
   float *v = vals;
-  CK(collapse(nt, row, col, val, starts, &c, &v, &cap, nnz));
+  const Rows to{row_off_, ucount_, ucol_, uval_};
+  CK(collapse(nt, row, col, val, to));
+  CK(pack(to, starts, &c, &v, &cap, nnz));
   if (c != cols || v != vals) return cudaErrorUnknown;  // cannot happen: nnz <= nt
   return cudaStreamSynchronize(s_);
 }
@@ -977,7 +985,8 @@ cudaError_t IpDevice::assemble(IpAxisResult out[2]) {
   const int64_t nt[2] = {n_locked_ + tot[0], n_locked_ + tot[1]}, nr[2] = {tot[2], tot[3]};
   CK(grow(s_, (size_t)(nt[0] + nt[1]), t_cap_, &t_row_, &t_col_, &t_val_));
   CK(grow(s_, (size_t)(nr[0] + nr[1]), r_cap_, &r_row_, &r_val_));
-  CK(grow(s_, (size_t)std::max({nt[0], nt[1], nr[0], nr[1]}), w_cap_, &bucket_, &bucket2_, &ucol_, &uval_));
+  CK(grow(s_, (size_t)std::max({nt[0], nt[1], nr[0], nr[1]}), w_cap_, &bucket_, &bucket2_));
+  CK(grow(s_, (size_t)std::max<int64_t>({nr[0], nr[1], 1}), u_cap_, &ucol_, &uval_));
   if (first) {
     CK(cudaStreamSynchronize(s_));
     progress("    round 1: triplet buffers allocated");
@@ -1001,7 +1010,12 @@ cudaError_t IpDevice::assemble(IpAxisResult out[2]) {
   for (int ax = 0; ax < 2; ax++) {
     Axis &A = ax_[ax];
     int64_t o = ax ? nt[0] : 0;
-    CK(collapse(nt[ax], t_row_ + o, t_col_ + o, t_val_ + o, A.starts, &A.cols, &A.vals, &A.cap, &A.nnz));
+    CK(grow(s_, (size_t)std::max<int64_t>(nt[ax], 1), A.u_cap, &A.ucol, &A.uval));
+    const Rows to{A.row_off, A.ucount, A.ucol, A.uval};
+    CK(collapse(nt[ax], t_row_ + o, t_col_ + o, t_val_ + o, to));
+    // the sliced copies are made from the rows as they are; packing them took 0.27 ms an axis
+    // and round at 400k cells and a read-back of their total
+    if (spmv_form_ != kSpmvSliced || ip_order_) CK(pack(to, A.starts, &A.cols, &A.vals, &A.cap, &A.nnz));
     if (first) {
       CK(cudaStreamSynchronize(s_));
       progress("    round 1: axis %d collapsed", ax);
@@ -1009,7 +1023,7 @@ cudaError_t IpDevice::assemble(IpAxisResult out[2]) {
     out[ax].triplets = nt[ax];
     // the right-hand side: this axis's terms as one-column triplets, summed per row in order
     int64_t r = ax ? nr[0] : 0;
-    CK(collapse(nr[ax], r_row_ + r, nullptr, r_val_ + r, nullptr, nullptr, nullptr, nullptr, nullptr));
+    CK(collapse(nr[ax], r_row_ + r, nullptr, r_val_ + r, Rows{row_off_, ucount_, ucol_, uval_}));
     if (n_) {
       k_rhs<<<grid(n_), kThreads, 0, s_>>>(n_, ax, box_, locked_, row_off_, ucount_, uval_, A.rhs);
       launches += 1;
@@ -1019,32 +1033,42 @@ cudaError_t IpDevice::assemble(IpAxisResult out[2]) {
   return cudaStreamSynchronize(s_);
 }
 
-// The sliced copy: the rows in order of length and the count of long rows read back, the
-// slice widths of the rest, their scan (the starts), the total read back to size the
-// entries, then the entries.
-cudaError_t IpDevice::slice(Axis &A, CsrDev m) {
-  CK(grow(s_, (size_t)std::max<int64_t>(n_, 1), A.sl_row_cap, &A.sl_row, &A.sl_len));
-  CK(grow(s_, (size_t)kSliceLenCap + 1, A.sl_count_cap, &A.sl_count));
-  CK(csr_slice_order(m, A.sl_row, A.sl_len, A.sl_count, s_));
-  int32_t n_long = 0;
-  CK(cudaMemcpyAsync(&n_long, A.sl_count + kSliceLongRow + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s_));
+// The sliced copies: the rows in order of length and the counts of long rows read back, the
+// slice widths of the rest, their scans (the starts), the totals read back to size the entries,
+// then the entries; both axes at each step, so a round waits twice.
+cudaError_t IpDevice::slice(CsrDev m[2]) {
+  int32_t n_long[2] = {0, 0};
+  int64_t ns[2], total[2] = {0, 0};
+  for (int a = 0; a < 2; a++) {
+    Axis &A = ax_[a];
+    CK(grow(s_, (size_t)std::max<int64_t>(n_, 1), A.sl_row_cap, &A.sl_row, &A.sl_len));
+    CK(grow(s_, (size_t)kSliceLenCap + 1, A.sl_count_cap, &A.sl_count));
+    CK(csr_slice_order(m[a], A.sl_row, A.sl_len, A.sl_count, s_));
+    CK(cudaMemcpyAsync(&n_long[a], A.sl_count + kSliceLongRow + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s_));
+  }
   CK(cudaStreamSynchronize(s_));
-  A.sl_long = n_long;
-  const int64_t ns = (n_ - n_long + kSliceRows - 1) / kSliceRows;
-  CK(grow(s_, (size_t)ns + 1, A.sl_start_cap, &A.sl_start));
-  CK(csr_slice_widths(n_, n_long, A.sl_len, A.sl_start, s_));
-  CK(scan(A.sl_start, ns));
-  int64_t total = 0;
-  CK(cudaMemcpyAsync(&total, A.sl_start + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s_));
+  for (int a = 0; a < 2; a++) {
+    Axis &A = ax_[a];
+    A.sl_long = n_long[a];
+    ns[a] = (n_ - n_long[a] + kSliceRows - 1) / kSliceRows;
+    CK(grow(s_, (size_t)ns[a] + 1, A.sl_start_cap, &A.sl_start));
+    CK(csr_slice_widths(n_, n_long[a], A.sl_len, A.sl_start, s_));
+    CK(scan(A.sl_start, ns[a]));
+    CK(cudaMemcpyAsync(&total[a], A.sl_start + ns[a], sizeof(int64_t), cudaMemcpyDeviceToHost, s_));
+  }
   CK(cudaStreamSynchronize(s_));
-  d2h_bytes += sizeof(int64_t) + sizeof(int32_t);
-  CK(grow(s_, (size_t)std::max<int64_t>(total, 1), A.sl_cap, &A.sl_ent));
-  m.sl_long = n_long;
-  m.sl_row = A.sl_row;
-  m.sl_len = A.sl_len;
-  m.sl_start = A.sl_start;
-  CK(csr_slice_fill(m, A.sl_ent, s_));
-  launches += 8;
+  d2h_bytes += 2 * (sizeof(int64_t) + sizeof(int32_t));
+  for (int a = 0; a < 2; a++) {
+    Axis &A = ax_[a];
+    CK(grow(s_, (size_t)std::max<int64_t>(total[a], 1), A.sl_cap, &A.sl_ent));
+    m[a].sl_long = A.sl_long;
+    m[a].sl_row = A.sl_row;
+    m[a].sl_len = A.sl_len;
+    m[a].sl_start = A.sl_start;
+    m[a].sl_ent = A.sl_ent;
+    CK(csr_slice_fill(m[a], A.sl_ent, s_));
+    launches += 5;
+  }
   return cudaSuccess;
 }
 
@@ -1083,7 +1107,7 @@ cudaError_t IpDevice::solver_order() {
   return cudaGetLastError();
 }
 
-cudaError_t IpDevice::solve(int max_iters, IpAxisResult out[2]) {
+void IpDevice::read_options() {
   // The forms give the same products bit for bit, so the choice changes only the speed:
   // GPL_SPMV_FORM=0|1|2 (a thread per row, tiled, sliced), else the sliced form, the faster at
   // every size measured (eight iterations, sliced against tiled: 300 cells 255 / 242 us, level;
@@ -1099,30 +1123,30 @@ cudaError_t IpDevice::solve(int max_iters, IpAxisResult out[2]) {
     const char *f = std::getenv("GPL_IP_ORDER");
     ip_order_ = f && f[0] == '1' ? 1 : 0;
   }
+}
+
+cudaError_t IpDevice::solve(int max_iters, IpAxisResult out[2]) {
   // the first solve starts every row at one point (the core centre): no order to take yet
   const bool ordered = ip_order_ && solves_ > 0 && n_ > 0;
   solves_++;
   if (ordered) CK(solver_order());
-  const bool sliced = spmv_form_ == kSpmvSliced;  // it reads copies of its own
   CsrDev m[2];
   const float *b[2];
   float *x[2];
   void *scratch[2];
   for (int a = 0; a < 2; a++) {
     Axis &A = ax_[a];
-    m[a] = ordered ? CsrDev{n_, A.p_starts, A.p_cols, A.p_vals} : CsrDev{n_, A.starts, A.cols, A.vals};
-    if (sliced) {
-      CK(slice(A, m[a]));
-      m[a].sl_long = A.sl_long;
-      m[a].sl_row = A.sl_row;
-      m[a].sl_len = A.sl_len;
-      m[a].sl_start = A.sl_start;
-      m[a].sl_ent = A.sl_ent;
-    }
+    if (ordered)
+      m[a] = CsrDev{n_, A.p_starts, A.p_cols, A.p_vals};
+    else if (spmv_form_ == kSpmvSliced)
+      m[a] = CsrDev{n_, A.row_off, A.ucol, A.uval, A.ucount};
+    else
+      m[a] = CsrDev{n_, A.starts, A.cols, A.vals};
     b[a] = ordered ? A.p_rhs : A.rhs;
     x[a] = ordered ? A.p_x : A.x;
     scratch[a] = (char *)scratch_ + a * scratch_bytes_;
   }
+  if (spmv_form_ == kSpmvSliced) CK(slice(m));
   BicgResult r[2]{};
   cudaError_t e = bicgstab_solve_pair(m, b, x, max_iters, scratch, s_, r, spmv_form_);
   // the starts' launches and a persistent loop (one more for each restart)

@@ -76,12 +76,12 @@ class IpDevice {
   // cols and vals (device buffers of at least nt entries). For a device that holds no design.
   cudaError_t csr_from_triplets(int64_t n, int64_t nt, const int32_t *row, const int32_t *col, const float *val, int64_t *starts, int32_t *cols, float *vals, int64_t *nnz);
   int64_t launches = 0, h2d_bytes = 0, d2h_bytes = 0;
-  // The solver's SpMV form ("" before the first solve).
+  // The solver's SpMV form ("" before the upload).
   std::string tuning() const { return spmv_form_ < 0 ? std::string() : std::string("initial placement SpMV: ") + (spmv_form_ == 2 ? "sliced" : spmv_form_ == 1 ? "tiled" : "rows"); }
 
  private:
   cudaStream_t s_;
-  int spmv_form_ = -1;  // the solver's SpMV form (SpmvForm), set at the first solve
+  int spmv_form_ = -1;  // the solver's SpMV form (SpmvForm), set at the upload
   int64_t n_ = 0, n_pins_ = 0, n_locked_ = 0;
   int32_t n_nets_ = 0;
   IpSetup cfg_;
@@ -99,7 +99,7 @@ class IpDevice {
   size_t scan_tmp_n_ = 0;
   int32_t *t_row_ = nullptr, *t_col_ = nullptr, *r_row_ = nullptr;
   float *t_val_ = nullptr, *r_val_ = nullptr;
-  size_t t_cap_ = 0, r_cap_ = 0, w_cap_ = 0;
+  size_t t_cap_ = 0, r_cap_ = 0, w_cap_ = 0, u_cap_ = 0;
   unsigned long long *bucket_ = nullptr;  // (column << 32 | position) per triplet, by row
   unsigned long long *bucket2_ = nullptr; // the longest rows' merge scratch, as long
   int32_t *fill_ = nullptr;
@@ -109,6 +109,13 @@ class IpDevice {
   int32_t *ucol_ = nullptr;
   float *uval_ = nullptr;
   struct Axis {
+    // the collapsed rows where the collapse leaves them (each row's distinct columns first in
+    // its triplets' span), as the sliced copy reads them; or, for the other forms and the
+    // solver's row order, packed
+    int64_t *row_off = nullptr, *ucount = nullptr;
+    int32_t *ucol = nullptr;
+    float *uval = nullptr;
+    size_t u_cap = 0;
     int64_t *starts = nullptr;
     int32_t *cols = nullptr;
     float *vals = nullptr, *rhs = nullptr, *x = nullptr;
@@ -139,9 +146,18 @@ class IpDevice {
   size_t scratch_bytes_ = 0;
   int64_t *hpwl_acc_ = nullptr;
   void release();
-  cudaError_t collapse(int64_t n_trip, const int32_t *row, const int32_t *col, const float *val, int64_t *starts_out, int32_t **cols, float **vals, size_t *cap, int64_t *nnz);
+  // Where a collapse leaves its rows: row i's [row_off[i], row_off[i] + ucount[i]).
+  struct Rows {
+    int64_t *row_off, *ucount;
+    int32_t *ucol;
+    float *uval;
+  };
+  cudaError_t collapse(int64_t n_trip, const int32_t *row, const int32_t *col, const float *val, const Rows &to);
+  // The rows packed into CSR arrays (grown as needed); *nnz read back.
+  cudaError_t pack(const Rows &r, int64_t *starts_out, int32_t **cols, float **vals, size_t *cap, int64_t *nnz);
+  void read_options();
   cudaError_t scan(int64_t *data, int64_t n, int arrays = 1, int64_t stride = 0);
-  cudaError_t slice(Axis &A, CsrDev m);  // the axis's sliced copy of m (its CSR, as solved)
+  cudaError_t slice(CsrDev m[2]);  // both axes' sliced copies of m (their rows, as solved)
 };
 
 }  // namespace gpl

@@ -41,6 +41,8 @@ __device__ __forceinline__ double loop_state(const double *S) {
 constexpr int kSpmvTile = 6144;
 constexpr int kSpmvUnroll = 8;
 
+__device__ __forceinline__ int64_t row_end(const int64_t *__restrict__ rs, const int64_t *__restrict__ cnt, int64_t i) { return cnt ? rs[i] + cnt[i] : rs[i + 1]; }
+
 // Each form hands every row it forms to emit(row, value), at most one row per thread, and
 // returns nowhere early, so a block-wide step may follow.
 template <class Emit>
@@ -119,14 +121,14 @@ constexpr int kLongChunks = 4;
 __host__ __device__ __forceinline__ int64_t sliced_long_blocks(int64_t n_long) { return (n_long + kThreads / 32 - 1) / (kThreads / 32); }
 __host__ __device__ __forceinline__ int64_t sliced_blocks(int64_t n, int64_t n_long) { return sliced_long_blocks(n_long) + (n - n_long + kThreads - 1) / kThreads; }
 template <class Emit>
-__device__ __forceinline__ void spmv_sliced_rows(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, Emit emit) {
+__device__ __forceinline__ void spmv_sliced_rows(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int64_t *__restrict__ cnt, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, Emit emit) {
   const int64_t lb = sliced_long_blocks(n_long);
   if (blockIdx.x < lb) {
     const int64_t w = blockIdx.x * (int64_t)(kThreads / 32) + (threadIdx.x >> 5);
     if (w >= n_long) return;  // the whole warp; such a warp forms no row
     const int lane = threadIdx.x & 31;
     const int32_t row = sl_row[w];
-    const int64_t b = rs[row], e = rs[row + 1];
+    const int64_t b = rs[row], e = row_end(rs, cnt, row);
     float sum = 0.0f;
     for (int64_t m = b; m < e; m += 32 * kLongChunks) {
       float p[kLongChunks];
@@ -175,19 +177,19 @@ __device__ __forceinline__ void spmv_sliced_rows(int64_t n, int64_t n_long, cons
   }
   emit(row, __fadd_rn(0.0f, __fmul_rn(1.0f, tmp)));
 }
-__global__ void __launch_bounds__(kThreads) k_spmv_sliced(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, float *__restrict__ y) {
-  spmv_sliced_rows(n, n_long, rs, cols, vals, sl_row, sl_len, sl_start, sl_ent, x, [&](int64_t r, float v) { y[r] = v; });
+__global__ void __launch_bounds__(kThreads) k_spmv_sliced(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int64_t *__restrict__ cnt, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, float *__restrict__ y) {
+  spmv_sliced_rows(n, n_long, rs, cnt, cols, vals, sl_row, sl_len, sl_start, sl_ent, x, [&](int64_t r, float v) { y[r] = v; });
 }
 
 // The order by length: a histogram of the (capped) lengths per block in shared memory, the
 // buckets' starts longest first, then each row's position from its bucket's cursor (a warp's
 // rows of one bucket take one atomic between them).
-__global__ void __launch_bounds__(kThreads) k_len_hist(int64_t n, const int64_t *__restrict__ rs, int32_t *__restrict__ count) {
+__global__ void __launch_bounds__(kThreads) k_len_hist(int64_t n, const int64_t *__restrict__ rs, const int64_t *__restrict__ cnt, int32_t *__restrict__ count) {
   __shared__ int32_t h[kSliceLenCap + 1];
   for (int b = threadIdx.x; b <= kSliceLenCap; b += kThreads) h[b] = 0;
   __syncthreads();
   const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
-  if (i < n) atomicAdd(&h[(int)min(rs[i + 1] - rs[i], (int64_t)kSliceLenCap)], 1);
+  if (i < n) atomicAdd(&h[(int)min(row_end(rs, cnt, i) - rs[i], (int64_t)kSliceLenCap)], 1);
   __syncthreads();
   for (int b = threadIdx.x; b <= kSliceLenCap; b += kThreads)
     if (h[b]) atomicAdd(&count[b], h[b]);
@@ -219,10 +221,10 @@ __global__ void k_len_starts(int32_t *count) {
     run += c[q];
   }
 }
-__global__ void __launch_bounds__(kThreads) k_len_scatter(int64_t n, const int64_t *__restrict__ rs, int32_t *__restrict__ cursor, int32_t *__restrict__ row, int32_t *__restrict__ len) {
+__global__ void __launch_bounds__(kThreads) k_len_scatter(int64_t n, const int64_t *__restrict__ rs, const int64_t *__restrict__ cnt, int32_t *__restrict__ cursor, int32_t *__restrict__ row, int32_t *__restrict__ len) {
   const int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;
   const bool live = i < n;
-  const int64_t l = live ? rs[i + 1] - rs[i] : 0;
+  const int64_t l = live ? row_end(rs, cnt, i) - rs[i] : 0;
   const int b = live ? (int)min(l, (int64_t)kSliceLenCap) : -1;
   const unsigned peers = __match_any_sync(0xffffffffu, b);
   const int leader = __ffs(peers) - 1, lane = threadIdx.x & 31;
@@ -256,7 +258,7 @@ static void spmv_launch(int form, cudaStream_t st, const CsrDev &A, const float 
   if (A.n <= 0) return;
   const unsigned eb = (unsigned)((A.n + kThreads - 1) / kThreads);
   if (form == kSpmvSliced)
-    k_spmv_sliced<<<(unsigned)std::max<int64_t>(sliced_blocks(A.n, A.sl_long), 1), kThreads, 0, st>>>(A.n, A.sl_long, A.rs, A.cols, A.vals, A.sl_row, A.sl_len, A.sl_start, A.sl_ent, in, o);
+    k_spmv_sliced<<<(unsigned)std::max<int64_t>(sliced_blocks(A.n, A.sl_long), 1), kThreads, 0, st>>>(A.n, A.sl_long, A.rs, A.cnt, A.cols, A.vals, A.sl_row, A.sl_len, A.sl_start, A.sl_ent, in, o);
   else if (form == kSpmvTiled)
     k_spmv_tiled<<<eb, kThreads, 0, st>>>(A.n, A.rs, A.cols, A.vals, in, o);
   else
@@ -361,7 +363,7 @@ constexpr unsigned long long kWaitNs = 2000000000ull;
 
 struct SysDev {
   int64_t n;
-  const int64_t *rs;
+  const int64_t *rs, *cnt;
   const int32_t *cols;
   const float *vals;
   int64_t sl_long;
@@ -661,7 +663,7 @@ __device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, floa
     for (int64_t w = (int64_t)(threadIdx.x >> 5) * blocks + c; w < items; w += warps) {
       if (w < q.sl_long) {
         const int32_t row = __ldg(q.sl_row + w);
-        const int64_t b = __ldg(q.rs + row), e = __ldg(q.rs + row + 1);
+        const int64_t b = __ldg(q.rs + row), e = row_end(q.rs, q.cnt, row);
         float sum = 0.0f;
         for (int64_t m = b; m < e; m += 32 * kLongChunks) {
           float pr[kLongChunks];
@@ -824,9 +826,9 @@ cudaError_t csr_slice_order(const CsrDev &A, int32_t *row, int32_t *len, int32_t
   const unsigned g = (unsigned)((A.n + kThreads - 1) / kThreads);
   cudaError_t e = cudaMemsetAsync(count, 0, (kSliceLenCap + 1) * sizeof(int32_t), st);
   if (e != cudaSuccess) return e;
-  k_len_hist<<<g, kThreads, 0, st>>>(A.n, A.rs, count);
+  k_len_hist<<<g, kThreads, 0, st>>>(A.n, A.rs, A.cnt, count);
   k_len_starts<<<1, 32, 0, st>>>(count);
-  k_len_scatter<<<g, kThreads, 0, st>>>(A.n, A.rs, count, row, len);
+  k_len_scatter<<<g, kThreads, 0, st>>>(A.n, A.rs, A.cnt, count, row, len);
   return cudaGetLastError();
 }
 
@@ -844,7 +846,7 @@ cudaError_t csr_slice_fill(const CsrDev &A, int2 *sl_ent, cudaStream_t st) {
 
 cudaError_t spmv(const CsrDev &A, const float *x, float *y, int form, cudaStream_t st) {
   if (form != kSpmvRows && form != kSpmvTiled && form != kSpmvSliced) return cudaErrorInvalidValue;
-  if (form == kSpmvSliced && (!A.sl_start || !A.sl_row || !A.sl_len)) return cudaErrorInvalidValue;
+  if (form == kSpmvSliced ? !A.sl_start || !A.sl_row || !A.sl_len : A.cnt != nullptr) return cudaErrorInvalidValue;
   if (A.n <= 0) return cudaSuccess;
   spmv_launch(form, st, A, x, y);
   return cudaGetLastError();
@@ -880,11 +882,12 @@ static cudaError_t solve_systems(int nsys, const CsrDev *A, const float *const *
   SysPair P{};
   for (int a = 0; a < nsys; a++) {
     if (A[a].n != n) return cudaErrorInvalidValue;
-    if (form == kSpmvSliced && (!A[a].sl_start || !A[a].sl_row || !A[a].sl_len)) return cudaErrorInvalidValue;
+    if (form == kSpmvSliced ? !A[a].sl_start || !A[a].sl_row || !A[a].sl_len : A[a].cnt != nullptr) return cudaErrorInvalidValue;
     char *base = (char *)scratch[a];
     SysDev &q = P.a[a];
     q.n = n;
     q.rs = A[a].rs;
+    q.cnt = A[a].cnt;
     q.cols = A[a].cols;
     q.vals = A[a].vals;
     q.sl_long = A[a].sl_long;

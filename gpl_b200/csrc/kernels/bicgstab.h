@@ -16,6 +16,9 @@ struct CsrDev {
   const int64_t *rs;
   const int32_t *cols;
   const float *vals;
+  // Rows that are not packed: row i's entries are [rs[i], rs[i] + cnt[i]) (NULL: packed, up to
+  // rs[i + 1]). The sliced form only.
+  const int64_t *cnt = nullptr;
   // Optional: the rows in order of length (longest first; the order within a length does
   // not matter): the row at position j is sl_row[j], of sl_len[j] entries. The first sl_long
   // positions (rows over kSliceLongRow entries) are read from the CSR arrays, a warp per row;
