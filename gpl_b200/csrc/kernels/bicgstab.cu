@@ -111,46 +111,81 @@ __global__ void __launch_bounds__(kThreads) k_spmv_tiled(int64_t n, const int64_
 }
 
 //  sliced: over the sliced copy (rows in order of length). The long rows first, a warp per
-//         row: the lanes form 32 products at a time from the CSR arrays (coalesced, several
-//         chunks in flight) and every lane adds them in column order through shuffles. Then
+//         row (long_row). Then
 //         a thread per short row: at step k a warp's rows read one coalesced run of entries
 //         (the slice's column k), each row summed in column order and stopping at its own
 //         length. y is written at the row's own index. Blocks [0, long_blocks) take the long
 //         rows, kThreads / 32 rows each.
-constexpr int kLongChunks = 4;
+// A long row by a warp: the lanes form kLongChunk products at a time from the CSR arrays into
+// buf (that many floats of the warp's own, 16-byte aligned), from where every lane adds them in
+// column order, four a load; the next chunk's x and the entries of the one after are in flight
+// meanwhile. The longest row bounds a product (a bound pin's cell ties to all its nets' pins:
+// 2500 entries at 400k cells): adding through shuffles took 20 ns an entry, this 4.
+constexpr int kLongPer = 4, kLongChunk = 32 * kLongPer;
+template <class Load>
+__device__ __forceinline__ float long_row(int64_t b, int64_t e, const int32_t *__restrict__ cols, const float *__restrict__ vals, float *buf, Load x) {
+  const int lane = threadIdx.x & 31;
+  int32_t c[kLongPer];
+  float v[kLongPer], xv[kLongPer], vx[kLongPer];
+  auto entries = [&](int64_t m) {
+#pragma unroll
+    for (int u = 0; u < kLongPer; u++) {
+      const int64_t k = m + 32 * u + lane;
+      c[u] = k < e ? __ldg(cols + k) : -1;
+      v[u] = k < e ? __ldg(vals + k) : 0.0f;
+    }
+  };
+  auto gather = [&]() {
+#pragma unroll
+    for (int u = 0; u < kLongPer; u++) {
+      xv[u] = c[u] >= 0 ? x(c[u]) : 0.0f;
+      vx[u] = v[u];
+    }
+  };
+  entries(b);
+  gather();
+  entries(b + kLongChunk);
+  float sum = 0.0f;
+  for (int64_t m = b; m < e; m += kLongChunk) {
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kLongPer; u++) buf[32 * u + lane] = __fmul_rn(vx[u], xv[u]);
+    __syncwarp();
+    gather();
+    entries(m + 2 * kLongChunk);
+    const float4 *q = reinterpret_cast<const float4 *>(buf);
+    if (e - m >= kLongChunk) {
+#pragma unroll
+      for (int t = 0; t < kLongChunk / 4; t++) {
+        const float4 z = q[t];
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, z.x), z.y), z.z), z.w);
+      }
+    } else {
+      const int cnt = (int)(e - m);
+      int t = 0;
+#pragma unroll 4
+      for (; t + 4 <= cnt; t += 4) {
+        const float4 z = q[t / 4];
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, z.x), z.y), z.z), z.w);
+      }
+      for (; t < cnt; t++) sum = __fadd_rn(sum, buf[t]);
+    }
+  }
+  __syncwarp();
+  return __fadd_rn(0.0f, __fmul_rn(1.0f, sum));
+}
 __host__ __device__ __forceinline__ int64_t sliced_long_blocks(int64_t n_long) { return (n_long + kThreads / 32 - 1) / (kThreads / 32); }
 __host__ __device__ __forceinline__ int64_t sliced_blocks(int64_t n, int64_t n_long) { return sliced_long_blocks(n_long) + (n - n_long + kThreads - 1) / kThreads; }
 template <class Emit>
 __device__ __forceinline__ void spmv_sliced_rows(int64_t n, int64_t n_long, const int64_t *__restrict__ rs, const int64_t *__restrict__ cnt, const int32_t *__restrict__ cols, const float *__restrict__ vals, const int32_t *__restrict__ sl_row, const int32_t *__restrict__ sl_len, const int64_t *__restrict__ sl_start, const int2 *__restrict__ sl_ent, const float *__restrict__ x, Emit emit) {
+  __shared__ __align__(16) float buf[kThreads / 32][kLongChunk];
   const int64_t lb = sliced_long_blocks(n_long);
   if (blockIdx.x < lb) {
     const int64_t w = blockIdx.x * (int64_t)(kThreads / 32) + (threadIdx.x >> 5);
     if (w >= n_long) return;  // the whole warp; such a warp forms no row
-    const int lane = threadIdx.x & 31;
     const int32_t row = sl_row[w];
-    const int64_t b = rs[row], e = row_end(rs, cnt, row);
-    float sum = 0.0f;
-    for (int64_t m = b; m < e; m += 32 * kLongChunks) {
-      float p[kLongChunks];
-#pragma unroll
-      for (int u = 0; u < kLongChunks; u++) {
-        const int64_t k = m + 32 * u + lane;
-        p[u] = k < e ? __fmul_rn(__ldg(vals + k), __ldg(x + __ldg(cols + k))) : 0.0f;
-      }
-#pragma unroll
-      for (int u = 0; u < kLongChunks; u++) {
-        const int64_t c0 = m + 32 * u;
-        if (c0 >= e) break;  // uniform across the warp
-        if (e - c0 >= 32) {
-#pragma unroll
-          for (int t = 0; t < 32; t++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, p[u], t));
-        } else {
-          const int cnt = (int)(e - c0);
-          for (int t = 0; t < cnt; t++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, p[u], t));
-        }
-      }
-    }
-    if (lane == 0) emit(row, __fadd_rn(0.0f, __fmul_rn(1.0f, sum)));
+    const float v = long_row(rs[row], row_end(rs, cnt, row), cols, vals, buf[threadIdx.x >> 5], [&](int32_t c) { return __ldg(x + c); });
+    if ((threadIdx.x & 31) == 0) emit(row, v);
     return;
   }
   const int64_t i = (blockIdx.x - lb) * (int64_t)kThreads + threadIdx.x;  // short position
@@ -579,14 +614,22 @@ __device__ __forceinline__ void each4(int64_t n, bool aligned, int c, int blocks
   for (int64_t i = 4 * n4 + tid; i < n; i += stride) f(i, false);
 }
 
+// The sliced form's items taken in the block so far; a product's first is left_base, the fetches
+// of the ones before it (a barrier apart).
+struct Left {
+  int taken;
+};
+
 // y = A x over the system's blocks, each row's products summed in column order (the forms of
 // SpmvForm, bit for bit the same y). x and y are written in this kernel: plain loads.
 //  rows:   a thread per row straight from memory;
 //  tiled:  a block's run of rows, its entries' products formed by all its threads into shared
 //          memory (coalesced, eight gathers a thread in flight), then a thread per row;
-//  sliced: a warp per long row (products through shuffles), then per slice of 32 rows.
+//  sliced: a warp per long row, then per slice of 32 rows. The gathers bound it: 0.8 a cycle
+//          and SM at 400k rows, near the one L1 looks up a cycle (the same loads without them
+//          took a third of the time).
 template <int FORM>
-__device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, float *y, int c, int blocks, float *prod) {
+__device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, float *y, int c, int blocks, float *prod, Left &left, int &left_base) {
   const int64_t n = q.n;
   if (FORM == kSpmvRows) {
     for (int64_t i = (int64_t)c * kSolveThreads + threadIdx.x; i < n; i += (int64_t)blocks * kSolveThreads) {
@@ -656,56 +699,52 @@ __device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, floa
       if (i < r1) y[i] = __fadd_rn(0.0f, __fmul_rn(1.0f, tmp));
     }
   } else {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warps = kSolveThreads / 32;
     const int64_t ns = (n - q.sl_long + kSliceRows - 1) / kSliceRows, items = q.sl_long + ns;
-    const int64_t warps = (int64_t)blocks * (kSolveThreads / 32);
-    // neighbouring items on different blocks: the longest rows spread over the SMs
-    for (int64_t w = (int64_t)(threadIdx.x >> 5) * blocks + c; w < items; w += warps) {
+    // the block's items are c, c + blocks, ...: neighbours lie on different blocks, so the
+    // longest rows spread over the SMs. With more of them than warps each warp takes the next
+    // one left when it is done: a fetch an item and one a warp past the end. 400k rows, two
+    // systems, an iteration: 149 us with fixed items and shuffled sums, 130 with the long rows'
+    // sums from shared memory, 107 with items taken too (112 to 117 taken one ahead, with or
+    // without the next one's loads in flight); 100k: 38 for all.
+    const int mine = (int)((items - c + blocks - 1) / blocks);
+    const bool shared = mine > warps;
+    int it = threadIdx.x >> 5;
+    auto next = [&](int now) {
+      if (!shared) return now + warps;
+      int z = 0;
+      if (lane == 0) z = atomicAdd(&left.taken, 1);
+      return __shfl_sync(0xffffffffu, z, 0) - left_base;
+    };
+    if (shared) it = next(it);
+    for (; it >= 0 && it < mine; it = next(it)) {
+      const int64_t w = (int64_t)it * blocks + c;
       if (w < q.sl_long) {
         const int32_t row = __ldg(q.sl_row + w);
-        const int64_t b = __ldg(q.rs + row), e = row_end(q.rs, q.cnt, row);
-        float sum = 0.0f;
-        for (int64_t m = b; m < e; m += 32 * kLongChunks) {
-          float pr[kLongChunks];
+        const float v = long_row(__ldg(q.rs + row), row_end(q.rs, q.cnt, row), q.cols, q.vals, prod + (threadIdx.x >> 5) * kLongChunk, [&](int32_t i) { return x[i]; });
+        if (lane == 0) y[row] = v;
+      } else {
+        const int64_t slice = w - q.sl_long, j = q.sl_long + slice * kSliceRows + lane;
+        const bool has = j < n;
+        const int32_t len = has ? __ldg(q.sl_len + j) : 0, row = has ? __ldg(q.sl_row + j) : 0;
+        const int2 *e = q.sl_ent + __ldg(q.sl_start + slice) + lane;
+        float tmp = 0.0f;
+        for (int32_t k = 0; k < len; k += kSpmvUnroll) {
+          int2 cv[kSpmvUnroll];
+          float xv[kSpmvUnroll];
 #pragma unroll
-          for (int u = 0; u < kLongChunks; u++) {
-            const int64_t k = m + 32 * u + lane;
-            pr[u] = k < e ? __fmul_rn(__ldg(q.vals + k), x[__ldg(q.cols + k)]) : 0.0f;
-          }
+          for (int u = 0; u < kSpmvUnroll; u++) cv[u] = k + u < len ? __ldg(e + (int64_t)(k + u) * kSliceRows) : make_int2(0, 0);
 #pragma unroll
-          for (int u = 0; u < kLongChunks; u++) {
-            const int64_t c0 = m + 32 * u;
-            if (c0 >= e) break;  // uniform across the warp
-            if (e - c0 >= 32) {
+          for (int u = 0; u < kSpmvUnroll; u++) xv[u] = k + u < len ? x[cv[u].x] : 0.0f;
 #pragma unroll
-              for (int z = 0; z < 32; z++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, pr[u], z));
-            } else {
-              const int cnt = (int)(e - c0);
-              for (int z = 0; z < cnt; z++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, pr[u], z));
-            }
-          }
+          for (int u = 0; u < kSpmvUnroll; u++)
+            if (k + u < len) tmp = __fadd_rn(tmp, __fmul_rn(__int_as_float(cv[u].y), xv[u]));
         }
-        if (lane == 0) y[row] = __fadd_rn(0.0f, __fmul_rn(1.0f, sum));
-        continue;
+        if (has) y[row] = __fadd_rn(0.0f, __fmul_rn(1.0f, tmp));
       }
-      const int64_t slice = w - q.sl_long, j = q.sl_long + slice * kSliceRows + lane;
-      if (j >= n) continue;
-      const int32_t len = __ldg(q.sl_len + j), row = __ldg(q.sl_row + j);
-      const int2 *ent = q.sl_ent + __ldg(q.sl_start + slice) + lane;
-      float tmp = 0.0f;
-      for (int32_t k = 0; k < len; k += kSpmvUnroll) {
-        int2 cv[kSpmvUnroll];
-        float xv[kSpmvUnroll];
-#pragma unroll
-        for (int u = 0; u < kSpmvUnroll; u++) cv[u] = k + u < len ? __ldg(ent + (int64_t)(k + u) * kSliceRows) : make_int2(0, 0);
-#pragma unroll
-        for (int u = 0; u < kSpmvUnroll; u++) xv[u] = k + u < len ? x[cv[u].x] : 0.0f;
-#pragma unroll
-        for (int u = 0; u < kSpmvUnroll; u++)
-          if (k + u < len) tmp = __fadd_rn(tmp, __fmul_rn(__int_as_float(cv[u].y), xv[u]));
-      }
-      y[row] = __fadd_rn(0.0f, __fmul_rn(1.0f, tmp));
+      __syncwarp();
     }
+    if (shared) left_base += mine + warps;
   }
 }
 
@@ -714,8 +753,11 @@ __device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, floa
 template <int FORM>
 __global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys, int blocks) {
   __shared__ double shp[32], shs[32];  // the partials' sums, the scalar steps' sums
-  __shared__ __align__(16) float prod[FORM == kSpmvTiled ? kSolveTile : 4];
+  __shared__ __align__(16) float prod[FORM == kSpmvTiled ? kSolveTile : FORM == kSpmvSliced ? kSolveThreads / 32 * kLongChunk : 4];
   __shared__ Factors f;
+  __shared__ Left left;
+  int left_base = 0;
+  if (threadIdx.x == 0) left.taken = 0;
   const int sys = (int)(blockIdx.x % nsys), c = (int)(blockIdx.x / nsys);
   const SysDev q = sys ? P.a[1] : P.a[0];
   const int64_t n = q.n;
@@ -749,7 +791,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys,
       });
     }
     if (!meet(m)) return;
-    solve_spmv<FORM>(q, q.p, q.v, c, blocks, prod);
+    solve_spmv<FORM>(q, q.p, q.v, c, blocks, prod, left, left_base);
     if (!meet(m)) return;
     int live = loop_dots<0>(n, q.r0, q.v, q.part, 0, c, blocks, shp);
     if (!meet(m)) return;
@@ -773,7 +815,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys,
       });
     }
     if (!meet(m)) return;
-    solve_spmv<FORM>(q, q.s, q.t, c, blocks, prod);
+    solve_spmv<FORM>(q, q.s, q.t, c, blocks, prod, left, left_base);
     if (!meet(m)) return;
     live = loop_dots<1>(n, q.t, q.s, q.part, 0, c, blocks, shp);
     if (!meet(m)) return;
