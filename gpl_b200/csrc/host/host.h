@@ -4,9 +4,9 @@
 // the Nesterov loop run on the device (engine.h).
 #pragma once
 #include <array>
-#include <functional>
 #include <cmath>
 #include <cstdint>
+#include <functional>
 #include <tuple>
 #include <map>
 #include <string>
@@ -241,7 +241,14 @@ double normal(Mt19937 &eng, double mean, double sigma);
 std::pair<int32_t, int32_t> orient_point(int orient, int32_t x, int32_t y);
 Ip make_pins(const Design &d, const Common &c, const Vars &v);
 class IpDevice;
-Ip do_bicgstab_place_device(Log &log, const Design &d, Common &c, const Vars &v, const IpVars &vars, IpDevice &dev);
+// Work beside the device's rounds: `begin` before them (the instances, their sizes and the pins'
+// offsets stay as they are until `end`), `end` after them or on the way out of a failure, and
+// before the instances move. Neither is called where no round runs.
+struct IpRounds {
+  std::function<void(const Ip &)> begin;
+  std::function<void()> end;
+};
+Ip do_bicgstab_place_device(Log &log, const Design &d, Common &c, const Vars &v, const IpVars &vars, IpDevice &dev, const IpRounds &rounds);
 
 }  // namespace gpl
 

@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <stdexcept>
 #include <tuple>
@@ -779,7 +780,7 @@ static uint64_t fnv_f32(const std::vector<float> &v) {
 // `doBicgstabPlace` (src/initial_place.rs:420-446) with its matrices assembled, collapsed and
 // solved on the device (kernels/b2b.cu): the reference's rounds, report lines, probes and stop
 // rules; the host reads back the two solves' scalars and the report's HPWL per round.
-Ip do_bicgstab_place_device(Log &log, const Design &d, Common &c, const Vars &v, const IpVars &vars, IpDevice &dev) {
+Ip do_bicgstab_place_device(Log &log, const Design &d, Common &c, const Vars &v, const IpVars &vars, IpDevice &dev, const IpRounds &rounds) {
   log.info("GPL", 5, "---- Execute Conjugate Gradient Initial Placement.");
   Ip ip = make_pins(d, c, v);
   progress("pins made");
@@ -869,6 +870,14 @@ Ip do_bicgstab_place_device(Log &log, const Design &d, Common &c, const Vars &v,
   s.max_fanout = vars.max_fanout;
   s.min_diff = vars.min_diff_length;
   s.weight_scale = vars.net_weight_scale;
+  struct Beside {
+    const IpRounds &r;
+    ~Beside() {
+      if (r.end) r.end();
+    }
+  };
+  std::unique_ptr<Beside> beside(new Beside{rounds});
+  if (rounds.begin) rounds.begin(ip);
   device(dev.upload(s), "initial placement upload");
   progress("initial placement (device): %zu pins, %zu nets", ip.pins.size(), ip.net_pins.size());
   std::vector<float> xs, ys;
@@ -904,6 +913,8 @@ Ip do_bicgstab_place_device(Log &log, const Design &d, Common &c, const Vars &v,
   std::vector<int4> box, db_box;
   device(dev.download(box, db_box), "initial placement download");
   progress("initial placement downloaded");
+  beside.reset();
+  progress("set-up beside the rounds done");
   // each placed instance writes only itself, its database box and its own pins
   parallel_for(n, [&](size_t a, size_t b) {
     for (size_t e = a; e < b; e++) {
