@@ -12,10 +12,10 @@
 // stages; thread 32 issues tcgen05.mma (M=128, N=BN, K=16, kind::f16, bf16 in, f32
 // accumulate), three per K step, as the stages land, committing each stage back to the
 // producer; after the last K-block all four warps read their 32 TMEM lanes, 32 columns at a
-// time. The single GEMMs use BN = 64 (a 1024-point grid gives 128 tiles for the 148 SMs), the
-// batched pairs BN = 128 (the same 128 tiles over both). Every wait is bounded by the GPU's
-// global timer (1 s): a wait that runs out records an error word, and the CTA drains and
-// returns.
+// time. The single GEMMs use BN = 32 or 64 (a 1024-point grid gives 128 tiles of 64 for the 148
+// SMs), the batched pairs up to BN = 128 (the same 128 tiles over both). Every wait is bounded
+// by the GPU's global timer (1 s): a wait that runs out records an error word, and the CTA
+// drains and returns.
 //
 // The four launches of a solve (see poisson.cu for the algebra):
 //   1  T1t = CyTs rho^T                      split out
@@ -26,6 +26,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -46,9 +47,9 @@ constexpr int BM = 128, BK = 64;
 constexpr int A_TILE = BM * BK * 2;                    // 16 KB
 template <int BN>
 struct Tile {
-  static constexpr int B_TILE = BN * BK * 2;                   // 8 or 16 KB
-  static constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;  // 48 or 64 KB, multiples of 1 KB
-  static constexpr int STAGES = BN == 64 ? 4 : 3;
+  static constexpr int B_TILE = BN * BK * 2;                   // 4, 8 or 16 KB
+  static constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;  // 40, 48 or 64 KB, multiples of 1 KB
+  static constexpr int STAGES = BN == 32 ? 5 : BN == 64 ? 4 : 3;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
   static constexpr uint32_t TMEM_COLS = BN;                    // fp32 accumulator columns
   // kind::f16 instruction descriptor: D f32, A and B bf16, both K-major, M=BM, N=BN.
@@ -68,6 +69,7 @@ struct TcOut {
 struct TcArgs {
   int M, N, K;        // multiples of 128, 64, 64
   TcOut o[2];         // per batch entry (blockIdx.z)
+  int early;          // A (a basis matrix) may be read before the kernel before this one ends
   const float *wx, *wx2, *wy, *wy2;
   int *err;
 };
@@ -158,7 +160,6 @@ __device__ __forceinline__ void split_store(__nv_bfloat16 *row_hi, __nv_bfloat16
 template <int EPI, int BN>
 __global__ void __launch_bounds__(128, 1) k_tc_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUtensorMap tB0,
                                                    const __grid_constant__ CUtensorMap tA1, const __grid_constant__ CUtensorMap tB1, TcArgs args) {
-  chain_enter();
   using T = Tile<BN>;
   constexpr int STAGES = T::STAGES, STAGE_BYTES = T::STAGE_BYTES, B_TILE = T::B_TILE;
   constexpr uint32_t TMEM_COLS = T::TMEM_COLS, IDESC = T::IDESC;
@@ -194,6 +195,20 @@ __global__ void __launch_bounds__(128, 1) k_tc_gemm(const __grid_constant__ CUte
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
+  // The barriers and the accumulator were set up, and the first stages' A tiles (basis
+  // matrices, which no solve writes) are asked for, beside the end of the kernel before this
+  // one; nothing else is read or written until it has ended.
+  const int pre = args.early ? min(STAGES, nkb) : 0;
+  auto load_a = [&](int kb) {
+    uint8_t *st = smem + (kb % STAGES) * STAGE_BYTES;
+    mbar_expect_tx(&full[kb % STAGES], STAGE_BYTES);
+    tma_load(st, mA, &full[kb % STAGES], kb * BK, m0);
+    tma_load(st + A_TILE, mA, &full[kb % STAGES], args.K + kb * BK, m0);
+  };
+  if (threadIdx.x == 0)
+    for (int kb = 0; kb < pre; kb++) load_a(kb);
+  chain_enter();
+
   if (threadIdx.x == 0) {
     // producer: K-block kb brings A_hi, A_lo (columns k0 and K + k0 of A) and B_hi, B_lo
     for (int kb = 0; kb < nkb; kb++) {
@@ -201,9 +216,7 @@ __global__ void __launch_bounds__(128, 1) k_tc_gemm(const __grid_constant__ CUte
       if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, fail, args.err, 1)) break;
       int k0 = kb * BK;
       uint8_t *st = smem + s * STAGE_BYTES;
-      mbar_expect_tx(&full[s], STAGE_BYTES);
-      tma_load(st, mA, &full[s], k0, m0);
-      tma_load(st + A_TILE, mA, &full[s], args.K + k0, m0);
+      if (kb >= pre) load_a(kb);
       tma_load(st + 2 * A_TILE, mB, &full[s], k0, n0);
       tma_load(st + 2 * A_TILE + B_TILE, mB, &full[s], args.K + k0, n0);
     }
@@ -309,6 +322,15 @@ cudaError_t make_map(CUtensorMap *m, const __nv_bfloat16 *base, int rows, int k,
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+template <int EPI, int BN>
+void tc_allow() {
+  cudaFuncSetAttribute(k_tc_gemm<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::SMEM_BYTES);
+}
+template <int EPI, int BN>
+cudaError_t tc_gemm(const TcArgs &a, int batch, cudaStream_t s, const CUtensorMap &A0, const CUtensorMap &B0, const CUtensorMap &A1, const CUtensorMap &B1) {
+  return launch_chained(k_tc_gemm<EPI, BN>, dim3(a.N / BN, a.M / BM, batch), dim3(128), Tile<BN>::SMEM_BYTES, s, A0, B0, A1, B1, a);
+}
+
 }  // namespace
 
 struct TcState {
@@ -316,8 +338,9 @@ struct TcState {
   __nv_bfloat16 *t1 = nullptr, *exh = nullptr, *eyh = nullptr, *t2 = nullptr, *t3 = nullptr;
   int *err = nullptr;
   CUtensorMap mCyTs, mCxTs, mCy, mSy, mSx, mCx;  // A operands (BM-row boxes)
-  CUtensorMap mDens, mT1;                        // B operands of the single GEMMs (64-row boxes)
-  CUtensorMap mExh, mEyh, mT2, mT3;              // B operands of the batched pairs (128-row boxes)
+  CUtensorMap mDens, mT1;                        // B operands of the single GEMMs (bn1-row boxes)
+  CUtensorMap mExh, mEyh, mT2, mT3;              // B operands of the batched pairs (bn2-row boxes)
+  int bn1 = 0, bn2 = 0;                          // output tile widths
 };
 
 size_t tc_plan_bytes(int nx, int ny) {
@@ -364,20 +387,34 @@ cudaError_t tc_plan_init(PoissonPlan *p, char *base, BasisOut &out) {
   TRY(make_map(&t->mSy, t->Sy, ny, ny, BM));
   TRY(make_map(&t->mSx, t->Sx, nx, nx, BM));
   TRY(make_map(&t->mCx, t->Cx, nx, nx, BM));
+  // A block's loads bound a GEMM (0.38 MB for a 128 x 64 tile at 512 points), so while the
+  // grid leaves SMs idle the tiles are narrower; past one wave of blocks their total traffic
+  // counts and they are wide. The four kernels end to end, 64 and 128 wide throughout against
+  // this rule and the early A tiles: 512 points 38 / 31 us; 1024 (the same widths) 64 / 62.
+  int dev = 0, sms = 0;
+  TRY(cudaGetDevice(&dev));
+  TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t tiles32 = (int64_t)nx * ny / (32 * BM);  // of one GEMM of 128 x 32 tiles
+  t->bn1 = tiles32 <= sms ? 32 : 64;
+  t->bn2 = 2 * tiles32 <= sms ? 32 : tiles32 <= sms ? 64 : 128;
   // B operands [N][2K]: BN-row boxes
-  TRY(make_map(&t->mDens, p->tc_dens, nx, ny, 64));  // rows x, K = y
-  TRY(make_map(&t->mT1, t->t1, ny, nx, 64));         // rows v, K = x
-  TRY(make_map(&t->mExh, t->exh, nx, ny, 128));      // rows u, K = v
-  TRY(make_map(&t->mEyh, t->eyh, nx, ny, 128));
-  TRY(make_map(&t->mT2, t->t2, ny, nx, 128));        // rows y, K = u
-  TRY(make_map(&t->mT3, t->t3, ny, nx, 128));
+  TRY(make_map(&t->mDens, p->tc_dens, nx, ny, t->bn1));  // rows x, K = y
+  TRY(make_map(&t->mT1, t->t1, ny, nx, t->bn1));         // rows v, K = x
+  TRY(make_map(&t->mExh, t->exh, nx, ny, t->bn2));       // rows u, K = v
+  TRY(make_map(&t->mEyh, t->eyh, nx, ny, t->bn2));
+  TRY(make_map(&t->mT2, t->t2, ny, nx, t->bn2));         // rows y, K = u
+  TRY(make_map(&t->mT3, t->t3, ny, nx, t->bn2));
 #undef TRY
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_tc_gemm<EPI_SPLIT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<64>::SMEM_BYTES);
-    cudaFuncSetAttribute(k_tc_gemm<EPI_SPECTRAL, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<64>::SMEM_BYTES);
-    cudaFuncSetAttribute(k_tc_gemm<EPI_SPLIT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<128>::SMEM_BYTES);
-    cudaFuncSetAttribute(k_tc_gemm<EPI_F32, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<128>::SMEM_BYTES);
+    tc_allow<EPI_SPLIT, 32>();
+    tc_allow<EPI_SPLIT, 64>();
+    tc_allow<EPI_SPLIT, 128>();
+    tc_allow<EPI_SPECTRAL, 32>();
+    tc_allow<EPI_SPECTRAL, 64>();
+    tc_allow<EPI_F32, 32>();
+    tc_allow<EPI_F32, 64>();
+    tc_allow<EPI_F32, 128>();
     attr = true;
   }
   return cudaGetLastError();
@@ -402,22 +439,30 @@ cudaError_t tc_solve(PoissonPlan *p, float *field_x, float *field_y, cudaStream_
   // 1: T1t[v][x] = sum_y CyTs[v][y] rho[x][y]      M = ny, N = nx, K = ny
   a.M = ny, a.N = nx, a.K = ny;
   a.o[0] = TcOut{t->t1, nullptr, nx};
-  cudaError_t le = launch_chained(k_tc_gemm<EPI_SPLIT, 64>, dim3(nx / 64, ny / BM, 1), dim3(128), Tile<64>::SMEM_BYTES, s, t->mCyTs, t->mDens, t->mCyTs, t->mDens, a);
+  cudaError_t le = t->bn1 == 32 ? tc_gemm<EPI_SPLIT, 32>(a, 1, s, t->mCyTs, t->mDens, t->mCyTs, t->mDens) : tc_gemm<EPI_SPLIT, 64>(a, 1, s, t->mCyTs, t->mDens, t->mCyTs, t->mDens);
   if (le != cudaSuccess) return le;
   // 2: Ah[u][v] = sum_x CxTs[u][x] T1t[v][x]; spectral  M = nx, N = ny, K = nx
   a.M = nx, a.N = ny, a.K = nx;
   a.o[0] = TcOut{t->exh, t->eyh, ny};
-  if ((le = launch_chained(k_tc_gemm<EPI_SPECTRAL, 64>, dim3(ny / 64, nx / BM, 1), dim3(128), Tile<64>::SMEM_BYTES, s, t->mCxTs, t->mT1, t->mCxTs, t->mT1, a)) != cudaSuccess) return le;
+  a.early = 1;  // from here on the kernel before is one of these, which writes no basis matrix
+  le = t->bn1 == 32 ? tc_gemm<EPI_SPECTRAL, 32>(a, 1, s, t->mCxTs, t->mT1, t->mCxTs, t->mT1) : tc_gemm<EPI_SPECTRAL, 64>(a, 1, s, t->mCxTs, t->mT1, t->mCxTs, t->mT1);
+  if (le != cudaSuccess) return le;
   // 3: T2t[y][u] = sum_v Cy[y][v] Exh[u][v]; T3t = Sy Eyh^T   M = ny, N = nx, K = ny
   a.M = ny, a.N = nx, a.K = ny;
   a.o[0] = TcOut{t->t2, nullptr, nx};
   a.o[1] = TcOut{t->t3, nullptr, nx};
-  if ((le = launch_chained(k_tc_gemm<EPI_SPLIT, 128>, dim3(nx / 128, ny / BM, 2), dim3(128), Tile<128>::SMEM_BYTES, s, t->mCy, t->mExh, t->mSy, t->mEyh, a)) != cudaSuccess) return le;
+  le = t->bn2 == 32   ? tc_gemm<EPI_SPLIT, 32>(a, 2, s, t->mCy, t->mExh, t->mSy, t->mEyh)
+       : t->bn2 == 64 ? tc_gemm<EPI_SPLIT, 64>(a, 2, s, t->mCy, t->mExh, t->mSy, t->mEyh)
+                      : tc_gemm<EPI_SPLIT, 128>(a, 2, s, t->mCy, t->mExh, t->mSy, t->mEyh);
+  if (le != cudaSuccess) return le;
   // 4: Ex[x][y] = sum_u Sx[x][u] T2t[y][u]; Ey = Cx T3t^T     M = nx, N = ny, K = nx
   a.M = nx, a.N = ny, a.K = nx;
   a.o[0] = TcOut{field_x, nullptr, ny};
   a.o[1] = TcOut{field_y, nullptr, ny};
-  if ((le = launch_chained(k_tc_gemm<EPI_F32, 128>, dim3(ny / 128, nx / BM, 2), dim3(128), Tile<128>::SMEM_BYTES, s, t->mSx, t->mT2, t->mCx, t->mT3, a)) != cudaSuccess) return le;
+  le = t->bn2 == 32   ? tc_gemm<EPI_F32, 32>(a, 2, s, t->mSx, t->mT2, t->mCx, t->mT3)
+       : t->bn2 == 64 ? tc_gemm<EPI_F32, 64>(a, 2, s, t->mSx, t->mT2, t->mCx, t->mT3)
+                      : tc_gemm<EPI_F32, 128>(a, 2, s, t->mSx, t->mT2, t->mCx, t->mT3);
+  if (le != cudaSuccess) return le;
   return cudaGetLastError();
 }
 
