@@ -1114,8 +1114,12 @@ void launch_wa_tiles(const WaArgs &w, float cx, float cy, cudaStream_t s) {
 // of |wl|, |density| and the two step-length distances (getDistance :319-330):
 // |a1 - b1|^2 and |out - b2|^2.
 // A block's cells are consecutive, so their pins' forces (cell-major) are one run: staged in
-// shared memory with coalesced loads when the run fits kGradPinTile, then each cell sums its
-// own in order. A cell over at most 3 x 3 bins loads its bins' boundaries and fields before
+// shared memory by asynchronous copies when the run fits kGradPinTile, in flight beside the
+// density force, then each cell sums its own in order. The loads' latencies bound it (issue
+// slots half used, DRAM 30 %): 1.1M cells, stand-alone 103 us with the run staged first, 98 with
+// it beside the density force, 94 with the pins' range and the area loaded ahead too, which
+// takes 48 registers (108 at 40, spilled; 101 and 105 with the distances' points ahead as well,
+// at 64 and 48); in the loop 107 to 90. A cell over at most 3 x 3 bins loads its bins' boundaries and fields before
 // the ordered sums; larger cells walk their bins, the largest (kBigCell) by their warp.
 constexpr int kGradPinTile = 2048;
 
@@ -1199,6 +1203,9 @@ __device__ __forceinline__ void big_force(const RegionArgs &r, bool big, int32_t
   }
 }
 
+__device__ __forceinline__ void copy_async8(void *to, const void *from) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory"); }
+__device__ __forceinline__ void copy_async_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // One block (cells blk * 256 ..) of a region's gradient update over nblk blocks.
 __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellArgs &c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1,
                                                 const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, const Publish &pub, int blk, int nblk) {
@@ -1209,17 +1216,29 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
   const int i1 = min(r.n_cells, i0 + (int)blockDim.x);
   const int64_t p0 = c.pin_start[i0], p1 = c.pin_start[i1];
   const bool staged = p1 - p0 <= kGradPinTile;
-  if (staged)
-    for (int k = threadIdx.x; k < (int)(p1 - p0); k += blockDim.x) s_pg[k] = pin_grad[p0 + k];
-  __syncthreads();
   double s_wl = 0, s_den = 0, s_d1 = 0, s_d2 = 0;
   const bool valid = i < r.n_cells;
   int32_t dlx = 0, dux = 0, dly = 0, duy = 0, x0 = 0, x1 = 0, y0 = 0, y1 = 0;
   float scale = 0.0f, fx = 0.0f, fy = 0.0f;
+  int2 d = make_int2(0, 0);
+  int32_t hx = 0, hy = 0;
   if (valid) {
-    const int2 d = c.dc[i];
-    const int32_t hx = c.hx[i], hy = c.hy[i];
+    d = c.dc[i];
+    hx = c.hx[i];
+    hy = c.hy[i];
     scale = c.dscale[i];
+  }
+  int64_t pb = 0, pe = 0;
+  float area = 0.0f;
+  if (valid) {
+    pb = c.pin_start[i];
+    pe = c.pin_start[i + 1];
+    area = c.area[i];
+  }
+  // the pins' forces arrive beside the density force
+  if (staged)
+    for (int k = threadIdx.x; k < (int)(p1 - p0); k += blockDim.x) copy_async8(s_pg + k, pin_grad + p0 + k);
+  if (valid) {
     dlx = d.x - hx, dux = d.x + hx, dly = d.y - hy, duy = d.y + hy;
     bin_span(dlx, dux, r.lx, r.size_x, r.inv_size_x, r.nx, x0, x1);
     bin_span(dly, duy, r.ly, r.size_y, r.inv_size_y, r.ny, y0, y1);
@@ -1281,8 +1300,9 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
   }
   const bool big = x1 > x0 && y1 > y0 && (x1 - x0) * (y1 - y0) > kBigCell;
   if (__any_sync(0xffffffffu, big)) big_force(r, big, x0, x1, y0, y1, dlx, dux, dly, duy, scale, fx, fy);
+  copy_async_all();
+  __syncthreads();
   if (valid) {
-    const int64_t pb = c.pin_start[i], pe = c.pin_start[i + 1];
     float wlx = 0.0f, wly = 0.0f;
     if (staged) {
       for (int k = (int)(pb - p0); k < (int)(pe - p0); k++) {
@@ -1300,7 +1320,7 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
     float sx = __fadd_rn(wlx, __fmul_rn(penalty, fx));
     float sy = __fadd_rn(wly, __fmul_rn(penalty, fy));
     float wl_pre = (float)(pe - pb);
-    float pre = fmaxf(__fadd_rn(wl_pre, __fmul_rn(penalty, c.area[i])), 1.0f);
+    float pre = fmaxf(__fadd_rn(wl_pre, __fmul_rn(penalty, area)), 1.0f);
     sx = __fdiv_rn(sx, pre);
     sy = __fdiv_rn(sy, pre);
     out_sum[i] = make_float2(sx, sy);
@@ -1332,12 +1352,12 @@ __device__ __forceinline__ void gradients_block(const RegionArgs &r, const CellA
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 6) k_gradients(RegionArgs r, CellArgs c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1, const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, Publish pub) {
+__global__ void __launch_bounds__(kThreads, 5) k_gradients(RegionArgs r, CellArgs c, const float2 *__restrict__ pin_grad, float penalty, float2 *__restrict__ out_sum, const float2 *__restrict__ a1, const float2 *__restrict__ b1, const float2 *__restrict__ b2, double *__restrict__ partials, unsigned int *ticket, double *out, Publish pub) {
   chain_enter();
   gradients_block(r, c, pin_grad, penalty, out_sum, a1, b1, b2, partials, ticket, out, pub, blockIdx.x, gridDim.x);
 }
 
-__global__ void __launch_bounds__(kThreads, 6) k_gradients_packed(const PackedRegion *__restrict__ t, int n, Publish pub) {
+__global__ void __launch_bounds__(kThreads, 5) k_gradients_packed(const PackedRegion *__restrict__ t, int n, Publish pub) {
   __shared__ PackedRegion e;
   packed_entry(t, n, e);
   gradients_block(e.r, e.c, e.pin_grad, e.penalty, e.out_sum, e.a1, e.b1, e.b2, e.partials, e.ticket, e.out, pub, (int)blockIdx.x - e.first, e.blocks);
