@@ -62,6 +62,35 @@ __device__ __forceinline__ int64_t cell_bin_addend(const RegionArgs &r, int32_t 
   return small_f2l_rz(a);
 }
 
+// A tile's slots zeroed, 16 bytes a store (the slots in use, rounded up to a multiple of 16
+// bytes), and its nonzero ones added to the HBM accumulators.
+__device__ __forceinline__ void tile_clear(bool narrow, unsigned long long *s64, unsigned int *s32, int cap, int nt, int start, int stride) {
+  uint4 *c4 = reinterpret_cast<uint4 *>(narrow ? (void *)s32 : (void *)s64);
+  uint4 *f4 = reinterpret_cast<uint4 *>(narrow ? (void *)(s32 + cap) : (void *)(s64 + cap));
+  const int n4 = narrow ? (nt + 3) / 4 : (nt + 1) / 2;
+  for (int k = start; k < n4; k += stride) c4[k] = f4[k] = make_uint4(0u, 0u, 0u, 0u);
+}
+__device__ __forceinline__ void tile_flush(const RegionArgs &r, bool narrow, const unsigned long long *s64, const unsigned int *s32, int cap, int nt, int32_t tx0, int32_t ty0, int32_t th, int start, int stride) {
+  // the slot's bin (x, y) followed step by step (one division per thread, not per slot)
+  const int dxs = stride / th, dys = stride - dxs * th;
+  int xk = start / th, yk = start - xk * th;
+  for (int k = start; k < nt; k += stride) {
+    unsigned long long vi = narrow ? s32[k] : s64[k];
+    unsigned long long vf = narrow ? s32[cap + k] : s64[cap + k];
+    if (vi | vf) {
+      const size_t g = (size_t)(tx0 + xk) * r.ny + (ty0 + yk);
+      if (vi) atomicAdd((unsigned long long *)&r.acc_inst[g], vi);
+      if (vf) atomicAdd((unsigned long long *)&r.acc_fill[g], vf);
+    }
+    xk += dxs;
+    yk += dys;
+    if (yk >= th) {
+      yk -= th;
+      xk++;
+    }
+  }
+}
+
 // The lanes' addends summed in a shared tile of th x tw bins (y fastest) from bin (tx0, ty0):
 // slots [0, cap) for cells, [cap, 2 cap) for fillers, 32-bit when narrow; then every nonzero
 // slot added to the HBM accumulators once. BLOCK: the block's threads share the tile; else
@@ -74,13 +103,7 @@ __device__ __forceinline__ void tile_scatter(const RegionArgs &r, bool narrow, u
   const int lane = threadIdx.x & 31;
   const int start = BLOCK ? (int)threadIdx.x : lane, stride = BLOCK ? (int)blockDim.x : 32;
   const int nt = tw * th;
-  {
-    // zeroed 16 bytes a store (the slots this tile uses, rounded up to a multiple of 16 bytes)
-    uint4 *c4 = reinterpret_cast<uint4 *>(narrow ? (void *)s32 : (void *)s64);
-    uint4 *f4 = reinterpret_cast<uint4 *>(narrow ? (void *)(s32 + cap) : (void *)(s64 + cap));
-    const int n4 = narrow ? (nt + 3) / 4 : (nt + 1) / 2;
-    for (int k = start; k < n4; k += stride) c4[k] = f4[k] = make_uint4(0u, 0u, 0u, 0u);
-  }
+  tile_clear(narrow, s64, s32, cap, nt, start, stride);
   if (BLOCK)
     __syncthreads();
   else
@@ -123,24 +146,59 @@ __device__ __forceinline__ void tile_scatter(const RegionArgs &r, bool narrow, u
     __syncthreads();
   else
     __syncwarp();
-  // the slot's bin (x, y) followed step by step (one division per thread, not per slot)
-  const int dxs = stride / th, dys = stride - dxs * th;
-  int xk = start / th, yk = start - xk * th;
-  for (int k = start; k < nt; k += stride) {
-    unsigned long long vi = narrow ? s32[k] : s64[k];
-    unsigned long long vf = narrow ? s32[cap + k] : s64[cap + k];
-    if (vi | vf) {
-      const size_t g = (size_t)(tx0 + xk) * r.ny + (ty0 + yk);
-      if (vi) atomicAdd((unsigned long long *)&r.acc_inst[g], vi);
-      if (vf) atomicAdd((unsigned long long *)&r.acc_fill[g], vf);
+  tile_flush(r, narrow, s64, s32, cap, nt, tx0, ty0, th, start, stride);
+}
+
+// f(bin column, bin row, addend) for each of a cell's bins with one, x outer: up to 3 x 3 bins
+// with each edge read once (a cell is widened to sqrt(2) bins, so two or three an axis), more
+// of them one by one.
+template <class F>
+__device__ __forceinline__ void cell_addends(const RegionArgs &r, int32_t x0, int32_t x1, int32_t y0, int32_t y1, int32_t dlx, int32_t dux, int32_t dly, int32_t duy, float scale, uint8_t kind, F f) {
+  const int32_t w = x1 - x0, h = y1 - y0;
+  if (w <= 3 && h <= 3) {
+    float ox[3], oy[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      ox[q] = oy[q] = 0.0f;
+      if (q < w) {
+        const int32_t lo = r.bx[x0 + q], hi = r.bx[x0 + q + 1];
+        const int32_t o = (dux < hi ? dux : hi) - (dlx > lo ? dlx : lo);
+        if (o > 0) ox[q] = small_i2f(o);
+      }
+      if (q < h) {
+        const int32_t lo = r.by[y0 + q], hi = r.by[y0 + q + 1];
+        const int32_t o = (duy < hi ? duy : hi) - (dly > lo ? dly : lo);
+        if (o > 0) oy[q] = small_i2f(o);
+      }
     }
-    xk += dxs;
-    yk += dys;
-    if (yk >= th) {
-      yk -= th;
-      xk++;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+      float a = __fmul_rn(__fmul_rn(ox[q / 3], oy[q % 3]), scale);
+      if (kind == CELL_MACRO) a = __fmul_rn(a, r.target_density);
+      const int64_t v = small_f2l_rz(a);
+      if (v) f(q / 3, q % 3, v);
     }
+    return;
   }
+  for (int32_t x = x0; x < x1; x++)
+    for (int32_t y = y0; y < y1; y++) {
+      const int64_t v = cell_bin_addend(r, dlx, dux, dly, duy, x, y, scale, kind);
+      if (v) f(x - x0, y - y0, v);
+    }
+}
+
+// The block's addends summed in a shared tile as in tile_scatter, 32-bit slots, each lane
+// adding its cell's on its own.
+__device__ __forceinline__ void share_scatter(const RegionArgs &r, unsigned int *s32, int cap, int32_t tx0, int32_t ty0, int32_t th, int32_t tw, bool any, int32_t x0, int32_t x1, int32_t y0, int32_t y1, int32_t dlx, int32_t dux, int32_t dly, int32_t duy, float scale, uint8_t kind) {
+  const int nt = tw * th;
+  tile_clear(true, nullptr, s32, cap, nt, threadIdx.x, blockDim.x);
+  __syncthreads();
+  if (any) {
+    unsigned int *at = s32 + (kind == CELL_FILLER ? cap : 0) + (x0 - tx0) * th + (y0 - ty0);
+    cell_addends(r, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind, [&](int32_t x, int32_t y, int64_t v) { atomicAdd(at + x * th + y, (unsigned int)v); });
+  }
+  __syncthreads();
+  tile_flush(r, true, nullptr, s32, cap, nt, tx0, ty0, th, threadIdx.x, blockDim.x);
 }
 
 // Every addend straight to the HBM accumulators, the warp's lanes walking their cells' bins in
@@ -339,13 +397,20 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
   }
   unsigned int *t32 = reinterpret_cast<unsigned int *>(s_tile);
   const bool tiles = r.scatter_form == 0;
-  // A tile pays where its slots take many addends each: below kDense a slot the atomics on
-  // HBM's accumulators (in L2) seldom meet and the walk in step costs more than it saves.
-  // Measured on 1.1M cells, tiles against straight to HBM: spread evenly (8 addends a bin of a
-  // block's box) 226 against 72 us, 16 times as dense (51) 163 against 92, 100 times (120) 111
-  // against 155, 10^4 times 84 against 624.
-  constexpr int64_t kDense = 64;
-  if (tile && tiles && s_box[4] >= kDense * (int64_t)(s_box[1] - s_box[0]) * (s_box[3] - s_box[2])) {
+  // With 32-bit slots the block's cells add to its tile on their own where that leaves at least
+  // two addends a slot for one add to HBM's accumulators (in L2). 1.1M cells, shared so / straight
+  // to HBM: spread evenly (5 addends a bin of a block's box) level, 70 us; 4 times as dense 67 /
+  // 88, 10 times 66 / 147, 50 times 65 / 566, 200 times 59 / 1031; lanes pooling their addends in
+  // step came to 72 to 96 from 50 a slot on, 163 below. A 400k-cell command's updates: 58 to 30
+  // ms. Wider slots have no native add in shared memory: their lanes walk in step, which pays
+  // from kDense addends a slot (226 us against 72 spread evenly, 111 against 155 at 120).
+  constexpr int64_t kDense = 64, kShare = 2;
+  const int64_t slots = (int64_t)(s_box[1] - s_box[0]) * (s_box[3] - s_box[2]);
+  if (tile && tiles && narrow && s_box[4] >= kShare * slots) {
+    share_scatter(r, t32, bcap, s_box[0], s_box[2], s_box[3] - s_box[2], s_box[1] - s_box[0], any, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
+    return;
+  }
+  if (tile && tiles && s_box[4] >= kDense * slots) {
     tile_scatter<true>(r, narrow, s_tile, t32, s_red, bcap, s_box[0], s_box[2], s_box[3] - s_box[2], s_box[1] - s_box[0], any, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
     return;
   }
@@ -362,40 +427,8 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
     return;
   }
   if (any) {
-    unsigned long long *acc = (unsigned long long *)(kind == CELL_FILLER ? r.acc_fill : r.acc_inst);
-    const int32_t w = x1 - x0, h = y1 - y0;
-    if (w <= 3 && h <= 3) {
-      // two or three bins an axis (a cell is widened to sqrt(2) bins): each edge read once
-      float ox[3], oy[3];
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        ox[q] = oy[q] = 0.0f;
-        if (q < w) {
-          const int32_t lo = r.bx[x0 + q], hi = r.bx[x0 + q + 1];
-          const int32_t o = (dux < hi ? dux : hi) - (dlx > lo ? dlx : lo);
-          if (o > 0) ox[q] = small_i2f(o);
-        }
-        if (q < h) {
-          const int32_t lo = r.by[y0 + q], hi = r.by[y0 + q + 1];
-          const int32_t o = (duy < hi ? duy : hi) - (dly > lo ? dly : lo);
-          if (o > 0) oy[q] = small_i2f(o);
-        }
-      }
-      unsigned long long *at = acc + (size_t)x0 * r.ny + y0;
-#pragma unroll
-      for (int q = 0; q < 9; q++) {
-        float a = __fmul_rn(__fmul_rn(ox[q / 3], oy[q % 3]), scale);
-        if (kind == CELL_MACRO) a = __fmul_rn(a, r.target_density);
-        const int64_t v = small_f2l_rz(a);
-        if (v) atomicAdd(at + (size_t)(q / 3) * r.ny + q % 3, (unsigned long long)v);
-      }
-      return;
-    }
-    for (int32_t y = y0; y < y1; y++)
-      for (int32_t x = x0; x < x1; x++) {
-        int64_t v = cell_bin_addend(r, dlx, dux, dly, duy, x, y, scale, kind);
-        if (v) atomicAdd(&acc[(size_t)x * r.ny + y], (unsigned long long)v);
-      }
+    unsigned long long *at = (unsigned long long *)(kind == CELL_FILLER ? r.acc_fill : r.acc_inst) + (size_t)x0 * r.ny + y0;
+    cell_addends(r, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind, [&](int32_t x, int32_t y, int64_t v) { atomicAdd(at + (size_t)x * r.ny + y, (unsigned long long)v); });
   }
 }
 
