@@ -204,7 +204,6 @@ cudaError_t poisson_solve(PoissonPlan *p, const float *density, float *field_x, 
 __nv_bfloat16 *poisson_split_input(PoissonPlan *p, int *ld);
 // Fill the split-BF16 operand from a float density (when no bin finalize wrote it).
 cudaError_t poisson_split_density(PoissonPlan *p, const float *density, cudaStream_t s);
-size_t poisson_workspace_bytes(int nx, int ny);
 // Loads the modules of the engine's kernels (each translation unit's), which the driver
 // otherwise loads at their first launch.
 void load_kernel_modules();

@@ -460,12 +460,6 @@ cudaError_t device_basis(int nx, int ny, const BasisOut &out, cudaStream_t s) {
   return cudaStreamSynchronize(s);  // the host values have been read
 }
 
-size_t poisson_workspace_bytes(int nx, int ny) {
-  size_t n = (size_t)nx * ny;
-  size_t basis = 3 * (size_t)nx * nx + 3 * (size_t)ny * ny;
-  return (basis + 5 * n) * sizeof(float) + 2 * (size_t)(nx + ny) * sizeof(float);
-}
-
 // One arena holds the plan: from the device's default pool (an engine's plans: kept warm by its
 // release threshold), ordered on the legacy stream and complete when the create returns; or
 // (scratch) from the entry points' own pool, ordered on the call's stream.
