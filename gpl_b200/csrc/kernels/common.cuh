@@ -37,8 +37,9 @@ constexpr int kThreads = 256;
 
 // Rust `as i32` from f32/f64: round toward zero, saturating, NaN to 0 (PTX cvt.rzi clamps).
 __device__ __forceinline__ int32_t f2i_rz(float v) { return __float2int_rz(v); }
-__device__ __forceinline__ int64_t f2l_rz(float v) { return __float2ll_rz(v); }
 __device__ __forceinline__ int32_t d2i_rz(double v) { return __double2int_rz(v); }
+// Rust `as i64` from f32, except for NaN: INT64_MIN here, 0 there.
+__device__ __forceinline__ int64_t f2l_rz(float v) { return __float2ll_rz(v); }
 
 // `fastExp` (src/nesterov.rs:308-314): (1 + x/1024)^1024 by ten squarings, in float. x/1024
 // is taken as x * 2^-10: both are the one correctly rounded value of the same real number.

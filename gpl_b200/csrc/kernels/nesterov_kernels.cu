@@ -176,7 +176,10 @@ __device__ __forceinline__ void cell_addends(const RegionArgs &r, int32_t x0, in
       float a = __fmul_rn(__fmul_rn(ox[q / 3], oy[q % 3]), scale);
       if (kind == CELL_MACRO) a = __fmul_rn(a, r.target_density);
       const int64_t v = small_f2l_rz(a);
-      if (v) f(q / 3, q % 3, v);
+      // the span decides, not the product: outside it the overlap is 0, but 0 times a scale that
+      // is not finite is no 0, and its add would land in other cells' bins or past the grid (the
+      // test: 0.4 us of a 1.1M-cell step's 91)
+      if (v && q / 3 < w && q % 3 < h) f(q / 3, q % 3, v);
     }
     return;
   }
