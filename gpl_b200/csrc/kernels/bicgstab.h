@@ -62,8 +62,11 @@ cudaError_t csr_slice_fill(const CsrDev &A, int2 *sl_ent, cudaStream_t s);
 // Scratch the solve needs (seven vectors of n floats, the partials and the scalars).
 size_t bicgstab_scratch_bytes(int64_t n);
 // Solve A x = b from the start point in x; `scratch` holds bicgstab_scratch_bytes(n) bytes
-// (256-byte aligned). The tiled form: no copy of the matrix, any row length.
-cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t s, BicgResult *out);
+// (256-byte aligned). The tiled form: no copy of the matrix, any row length. The loop's blocks
+// wait for one another at most wait_ns nanoseconds at a time; past that the solve returns
+// cudaErrorLaunchTimeout, x then between two steps.
+constexpr unsigned long long kSolveWaitNs = 2000000000ull;
+cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t s, BicgResult *out, unsigned long long wait_ns = kSolveWaitNs);
 // y = A x in the given form (SpmvForm).
 cudaError_t spmv(const CsrDev &A, const float *x, float *y, int form, cudaStream_t s);
 // Two systems of the same size solved side by side (each launch carries both): each takes

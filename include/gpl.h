@@ -323,7 +323,10 @@ int gpl_kernel_spmv(int64_t n, const int64_t *row_start, const int32_t *cols, co
 
 /* The initial placement's solver `bicgstab` (src/bicgstab.rs:615-669) on a CSR matrix (device
  * pointers) with FP64 inner products; x is the start point and the result. Writes iterations
- * and error (host pointers). Allocates its scratch vectors per call. */
+ * and error (host pointers). Allocates its scratch vectors per call. The solver's blocks wait for
+ * one another on the device, each wait bounded: if one runs out, the call returns
+ * cudaErrorLaunchTimeout and x holds no solution. The launch is cooperative, so a kernel of
+ * another stream that holds the device delays the solve and does not count against the bound. */
 int gpl_kernel_bicgstab(int64_t n, const int64_t *row_start, const int32_t *cols,
                         const float *vals, const float *rhs, float *x, int32_t max_iters,
                         int32_t *iterations, float *error, void *stream);
