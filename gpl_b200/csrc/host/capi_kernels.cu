@@ -434,14 +434,14 @@ int gpl_kernel_spmv(int64_t n, const int64_t *row_start, const int32_t *cols, co
   return (int)(e != cudaSuccess ? e : e2);
 }
 
-static int bicgstab_call(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *rhs, float *x, int32_t max_iters, int32_t *iterations, float *error, unsigned long long wait_ns, void *stream) {
+static int bicgstab_call(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *rhs, float *x, int32_t max_iters, int32_t *iterations, float *error, SolveWait wait, void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   void *scratch = nullptr;
   cudaError_t e = cudaMalloc(&scratch, bicgstab_scratch_bytes(n));
   if (e != cudaSuccess) return (int)e;
   CsrDev A{n, row_start, cols, vals};
   BicgResult r{};
-  e = bicgstab_solve(A, rhs, x, max_iters, scratch, s, &r, wait_ns);
+  e = bicgstab_solve(A, rhs, x, max_iters, scratch, s, &r, wait);
   cudaError_t e2 = cudaStreamSynchronize(s);
   cudaFree(scratch);
   *iterations = r.iterations;
@@ -450,12 +450,12 @@ static int bicgstab_call(int64_t n, const int64_t *row_start, const int32_t *col
 }
 
 int gpl_kernel_bicgstab(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *rhs, float *x, int32_t max_iters, int32_t *iterations, float *error, void *stream) {
-  return bicgstab_call(n, row_start, cols, vals, rhs, x, max_iters, iterations, error, kSolveWaitNs, stream);
+  return bicgstab_call(n, row_start, cols, vals, rhs, x, max_iters, iterations, error, SolveWait{}, stream);
 }
 
-// Test-only (not in include/gpl.h): the same with the solver's wait limit given.
-int gpl_rules_bicgstab_wait(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *rhs, float *x, int32_t max_iters, int32_t *iterations, float *error, uint64_t wait_ns, void *stream) {
-  return bicgstab_call(n, row_start, cols, vals, rhs, x, max_iters, iterations, error, wait_ns, stream);
+// Test-only (not in include/gpl.h): the same with the limit of the solver's waits given.
+int gpl_rules_bicgstab_wait(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *rhs, float *x, int32_t max_iters, int32_t *iterations, float *error, uint64_t wait_ns, uint64_t entry_ns, void *stream) {
+  return bicgstab_call(n, row_start, cols, vals, rhs, x, max_iters, iterations, error, SolveWait{wait_ns, entry_ns}, stream);
 }
 
 int gpl_kernel_rudy(int64_t n_nets, const int32_t *boxes, int32_t die_lx, int32_t die_ly, int32_t die_ux, int32_t die_uy, int32_t cnt_x, int32_t cnt_y, int32_t tile_size, int32_t wire_width, float *demand, void *stream) {

@@ -751,7 +751,7 @@ __device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, floa
 // blocks: a system's blocks; block b belongs to system b % nsys (with an even count of SMs and
 // two blocks an SM, both of an SM's are one system's, so they share its vectors in L1).
 template <int FORM>
-__global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys, int blocks, unsigned long long wait_ns) {
+__global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys, int blocks, SolveWait wait) {
   __shared__ double shp[32], shs[32];  // the partials' sums, the scalar steps' sums
   __shared__ __align__(16) float prod[FORM == kSpmvTiled ? kSolveTile : FORM == kSpmvSliced ? kSolveThreads / 32 * kLongChunk : 4];
   __shared__ Factors f;
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve(SysPair P, int nsys,
   const SysDev q = sys ? P.a[1] : P.a[0];
   const int64_t n = q.n;
   double *S = q.S;
-  Meet m{reinterpret_cast<unsigned int *>(S + S_ARRIVE), reinterpret_cast<unsigned int *>(S + S_ERROR), (unsigned int)blocks, 0u, wait_ns};
+  Meet m{reinterpret_cast<unsigned int *>(S + S_ARRIVE), reinterpret_cast<unsigned int *>(S + S_ERROR), (unsigned int)blocks, 0u, wait.ns + wait.entry_ns * (unsigned long long)q.rs[n]};
   const bool al = aligned16(q.r, q.r);
   Scalars k{};
   double s0, s1;
@@ -900,7 +900,7 @@ cudaError_t spmv(const CsrDev &A, const float *x, float *y, int form, cudaStream
 // tiled form, whose threads share a run's entries, takes a block for every 128 rows (3000 rows:
 // 19.5 us against 22.4 with 512), the others a thread per row (10k rows, sliced, two systems:
 // 24 us against 25 with 128).
-static cudaError_t solve_launch(int form, SysPair P, int nsys, unsigned long long wait_ns, cudaStream_t st) {
+static cudaError_t solve_launch(int form, SysPair P, int nsys, SolveWait wait, cudaStream_t st) {
   const void *fn = form == kSpmvSliced ? (const void *)k_solve<kSpmvSliced> : form == kSpmvTiled ? (const void *)k_solve<kSpmvTiled> : (const void *)k_solve<kSpmvRows>;
   int dev = 0, sms = 0, per = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -912,12 +912,12 @@ static cudaError_t solve_launch(int form, SysPair P, int nsys, unsigned long lon
   int blocks = (int)std::min<int64_t>(most, std::max<int64_t>(1, (P.a[0].n + rows - 1) / rows));
   for (int a = 0; a < nsys; a++)
     if ((e = cudaMemsetAsync(P.a[a].S + S_ARRIVE, 0, (64 - S_ARRIVE) * sizeof(double), st)) != cudaSuccess) return e;
-  void *args[] = {&P, &nsys, &blocks, &wait_ns};
+  void *args[] = {&P, &nsys, &blocks, &wait};
   return cudaLaunchCooperativeKernel(fn, dim3((unsigned)(blocks * nsys)), dim3(kSolveThreads), args, 0, st);
 }
 
 // One or two systems of the same size, each with its own scalars and state.
-static cudaError_t solve_systems(int nsys, const CsrDev *A, const float *const *b, float *const *x, int max_iters, void *const *scratch, cudaStream_t st, BicgResult *out, int form, unsigned long long wait_ns) {
+static cudaError_t solve_systems(int nsys, const CsrDev *A, const float *const *b, float *const *x, int max_iters, void *const *scratch, cudaStream_t st, BicgResult *out, int form, SolveWait wait) {
   static_assert(S_END <= S_ARRIVE && S_ERROR < 64, "the scalars fit the scratch's 64 doubles");
   const int64_t n = A[0].n;
   const size_t vec = ((size_t)n * sizeof(float) + 255) / 256 * 256;
@@ -996,7 +996,7 @@ static cudaError_t solve_systems(int nsys, const CsrDev *A, const float *const *
   int64_t n_launches = 0;
   int restarts[2] = {0, 0};
   for (;;) {
-    if ((e = solve_launch(form, P, nsys, wait_ns, st)) != cudaSuccess) return e;
+    if ((e = solve_launch(form, P, nsys, wait, st)) != cudaSuccess) return e;
     if ((e = pull()) != cudaSuccess) return e;
     bool ended = true;
     for (int a = 0; a < nsys; a++) {
@@ -1030,9 +1030,9 @@ static cudaError_t solve_systems(int nsys, const CsrDev *A, const float *const *
   return cudaGetLastError();
 }
 
-cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t st, BicgResult *out, unsigned long long wait_ns) { return solve_systems(1, &A, &b, &x, max_iters, &scratch, st, out, kSpmvTiled, wait_ns); }
+cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t st, BicgResult *out, SolveWait wait) { return solve_systems(1, &A, &b, &x, max_iters, &scratch, st, out, kSpmvTiled, wait); }
 
-cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], float *const x[2], int max_iters, void *const scratch[2], cudaStream_t st, BicgResult out[2], int form) { return solve_systems(2, A, b, x, max_iters, scratch, st, out, form, kSolveWaitNs); }
+cudaError_t bicgstab_solve_pair(const CsrDev A[2], const float *const b[2], float *const x[2], int max_iters, void *const scratch[2], cudaStream_t st, BicgResult out[2], int form) { return solve_systems(2, A, b, x, max_iters, scratch, st, out, form, SolveWait{}); }
 
 // Loads this file's module (the driver loads a module at its first launch otherwise).
 void load_module_bicgstab() {

@@ -63,10 +63,14 @@ cudaError_t csr_slice_fill(const CsrDev &A, int2 *sl_ent, cudaStream_t s);
 size_t bicgstab_scratch_bytes(int64_t n);
 // Solve A x = b from the start point in x; `scratch` holds bicgstab_scratch_bytes(n) bytes
 // (256-byte aligned). The tiled form: no copy of the matrix, any row length. The loop's blocks
-// wait for one another at most wait_ns nanoseconds at a time; past that the solve returns
-// cudaErrorLaunchTimeout, x then between two steps.
-constexpr unsigned long long kSolveWaitNs = 2000000000ull;
-cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t s, BicgResult *out, unsigned long long wait_ns = kSolveWaitNs);
+// wait for one another; past the wait's limit the solve returns cudaErrorLaunchTimeout, x then
+// between two steps. A block may hold nearly every entry in one row, whose sum is one thread's
+// (4.5 ns an entry from shared memory, 50 straight from memory), so the limit grows with the
+// entries: at two seconds alone a row of 450M, or of 40M by rows, was taken for a block gone.
+struct SolveWait {
+  unsigned long long ns = 2000000000ull, entry_ns = 200;
+};
+cudaError_t bicgstab_solve(const CsrDev &A, const float *b, float *x, int max_iters, void *scratch, cudaStream_t s, BicgResult *out, SolveWait wait = SolveWait{});
 // y = A x in the given form (SpmvForm).
 cudaError_t spmv(const CsrDev &A, const float *x, float *y, int form, cudaStream_t s);
 // Two systems of the same size solved side by side (each launch carries both): each takes
