@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstring>
 #include <numeric>
+#include <system_error>
 
 #include "../kernels/b2b.h"
 #include "../kernels/bicgstab.h"
@@ -115,7 +116,7 @@ void Engine::join() {
 void Engine::prewarm(size_t bytes) {
   prewarm_join();
   const int dev = device_;
-  prewarm_ = new std::thread([dev, bytes] {
+  auto warm = [dev, bytes] {
     if (cudaSetDevice(dev) != cudaSuccess) return;
     cudaStream_t s = nullptr;
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return;
@@ -126,7 +127,11 @@ void Engine::prewarm(size_t bytes) {
     cudaStreamSynchronize(s);
     cudaStreamDestroy(s);
     cudaGetLastError();  // nothing of it is an error of the command's
-  });
+  };
+  try {
+    prewarm_ = new std::thread(warm);
+  } catch (const std::system_error &) {  // no thread to be had: the first uses map the memory
+  }
 }
 
 void Engine::prewarm_join() {

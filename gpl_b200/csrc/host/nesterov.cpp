@@ -2495,7 +2495,10 @@ struct gpl_ctx {
   void reap(std::unique_ptr<Run> run) {
     if (run) run->route.reset();
     settle();
-    reaper = std::thread([r = std::move(run)]() mutable { r.reset(); });
+    try {
+      reaper = std::thread([r = std::move(run)]() mutable { r.reset(); });
+    } catch (const std::system_error &) {  // no thread to be had: freed with the closure
+    }
   }
   void settle() {
     if (reaper.joinable()) reaper.join();
@@ -2873,6 +2876,23 @@ void gpl_rules_settle_wait_step(int start, int iter, int active, int settled, in
   out3[2] = extra;
 }
 float gpl_rules_fast_exp(float x) { return fast_exp(x); }
+// 0 + 1 + ... + (n - 1) over parallel_for's threads; -1 when the iteration `stop` was refused.
+int64_t gpl_rules_parallel_sum(int64_t n, int64_t stop) {
+  std::atomic<int64_t> sum{0};
+  try {
+    parallel_for((size_t)n, [&](size_t a, size_t b) {
+      int64_t s = 0;
+      for (size_t k = a; k < b; k++) {
+        if ((int64_t)k == stop) throw std::runtime_error("refused");
+        s += (int64_t)k;
+      }
+      sum += s;
+    }, 1);
+  } catch (const std::runtime_error &) {
+    return -1;
+  }
+  return sum;
+}
 float gpl_rules_wavenumber_x(int i, int nx) { return wavenumber_x(i, nx); }
 float gpl_rules_wavenumber_y(int i, int ny, float bx, float by) { return wavenumber_y(i, ny, bx, by); }
 uint32_t gpl_rules_round_down_pow2(uint32_t x) { return round_down_to_power_of_two(x); }

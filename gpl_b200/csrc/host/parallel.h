@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -48,7 +49,9 @@ inline unsigned host_threads() {
 }
 
 // f(begin, end) over [0, n) in contiguous chunks, one per thread (the calling thread takes
-// the first); ranges shorter than `grain` per thread run on fewer threads.
+// the first, and those for which no thread can be started); ranges shorter than `grain` per
+// thread run on fewer threads. An exception of f's reaches the caller, the first chunk's that
+// threw, once every thread has ended.
 template <class F>
 void parallel_for(size_t n, F &&f, size_t grain = 16384) {
   size_t t = std::min<size_t>(host_threads(), (n + grain - 1) / std::max<size_t>(grain, 1));
@@ -57,14 +60,27 @@ void parallel_for(size_t n, F &&f, size_t grain = 16384) {
     return;
   }
   const size_t chunk = (n + t - 1) / t;
+  std::vector<std::exception_ptr> thrown(t);
+  auto run = [&](size_t i) {
+    const size_t a = i * chunk, b = std::min(n, a + chunk);
+    try {
+      if (a < b) f(a, b);
+    } catch (...) {
+      thrown[i] = std::current_exception();
+    }
+  };
   std::vector<std::thread> pool;
   pool.reserve(t - 1);
-  for (size_t i = 1; i < t; i++) {
-    size_t a = i * chunk, b = std::min(n, a + chunk);
-    if (a < b) pool.emplace_back([&f, a, b] { f(a, b); });
+  size_t started = 1;
+  try {
+    for (; started < t; started++) pool.emplace_back(run, started);
+  } catch (const std::exception &) {  // no thread to be had, or no memory for its state
   }
-  f((size_t)0, std::min(n, chunk));
+  run(0);
+  for (size_t i = started; i < t; i++) run(i);
   for (auto &th : pool) th.join();
+  for (auto &e : thrown)
+    if (e) std::rethrow_exception(e);
 }
 
 }  // namespace gpl
