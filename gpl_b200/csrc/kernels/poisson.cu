@@ -403,26 +403,25 @@ __global__ void __launch_bounds__(256) k_basis(int nx, int ny, BasisOut out, Uns
   const int w = blockIdx.z;
   const bool x_side = w == B_CXTS || w == B_SX || w == B_CX;
   const int n = x_side ? nx : ny;
-  const int r = blockIdx.y;
-  if (r >= n) return;
-  for (int c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
-    const bool fwd = w == B_CYTS || w == B_CXTS;
-    const int k = fwd ? r : c, j = fwd ? c : r;
-    const double a = __ddiv_rn(__dmul_rn(__dmul_rn(M_PI, (double)k), __dadd_rn((double)j, 0.5)), (double)n);
-    double v;
-    if (w == B_SY || w == B_SX)
-      v = k == 0 ? ((j & 1) ? -1.0 : 1.0) : sin(a);
-    else
-      v = cos(a);
-    if (fwd) v = __dmul_rn(__ddiv_rn(__dmul_rn(r == 0 ? 0.5 : 1.0, 2.0), (double)n), v);
-    const double e = fabs(v) * 0x1p-49;
-    const float x = __double2float_rn(v);
-    if (__double2float_rn(v - e) != x || __double2float_rn(v + e) != x) {
-      const unsigned q = atomicAdd(&unsure->count, 1u);
-      if (q < kMaxUnsure) unsure->at[q] = make_int4(w, r, c, 0);
+  for (int r = blockIdx.y; r < n; r += gridDim.y)
+    for (int c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
+      const bool fwd = w == B_CYTS || w == B_CXTS;
+      const int k = fwd ? r : c, j = fwd ? c : r;
+      const double a = __ddiv_rn(__dmul_rn(__dmul_rn(M_PI, (double)k), __dadd_rn((double)j, 0.5)), (double)n);
+      double v;
+      if (w == B_SY || w == B_SX)
+        v = k == 0 ? ((j & 1) ? -1.0 : 1.0) : sin(a);
+      else
+        v = cos(a);
+      if (fwd) v = __dmul_rn(__ddiv_rn(__dmul_rn(r == 0 ? 0.5 : 1.0, 2.0), (double)n), v);
+      const double e = fabs(v) * 0x1p-49;
+      const float x = __double2float_rn(v);
+      if (__double2float_rn(v - e) != x || __double2float_rn(v + e) != x) {
+        const unsigned q = atomicAdd(&unsure->count, 1u);
+        if (q < kMaxUnsure) unsure->at[q] = make_int4(w, r, c, 0);
+      }
+      basis_store(out, w, n, r, c, x);
     }
-    basis_store(out, w, n, r, c, x);
-  }
 }
 __global__ void k_basis_patch(int nx, int ny, BasisOut out, const Unsure *unsure, const float *x, unsigned count) {
   const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -432,15 +431,15 @@ __global__ void k_basis_patch(int nx, int ny, BasisOut out, const Unsure *unsure
   basis_store(out, at.x, x_side ? nx : ny, at.y, at.z, x[q]);
 }
 
+constexpr int kMaxGridY = 65535;  // a row of blocks a matrix row, the rest of a longer side's in turn
 cudaError_t device_basis(int nx, int ny, const BasisOut &out, cudaStream_t s) {
-  if (std::max(nx, ny) > 65535) return cudaErrorInvalidValue;  // a row a block; the form's matrices would take 100 GB
   Scratch buf(sizeof(Unsure), s);
   cudaError_t e = buf.error();
   if (e != cudaSuccess) return e;
   Unsure *u = static_cast<Unsure *>(buf.get());
   if ((e = cudaMemsetAsync(u, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
   const int n = std::max(nx, ny);
-  k_basis<<<dim3((unsigned)std::min((n + 255) / 256, 8), (unsigned)n, B_COUNT), 256, 0, s>>>(nx, ny, out, u);
+  k_basis<<<dim3((unsigned)std::min((n + 255) / 256, 8), (unsigned)std::min(n, kMaxGridY), B_COUNT), 256, 0, s>>>(nx, ny, out, u);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   unsigned count = 0;
   if ((e = cudaMemcpyAsync(&count, u, sizeof count, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
