@@ -34,8 +34,8 @@ namespace {
 // pin order, and, for the gradient, a thread per pin its derivative:
 // dW/dx_p = w [ e+_p ((1 + c x_p) S+ - c A+) / S+^2 - e-_p ((1 - c x_p) S- + c A-) / S-^2 ].
 // A thread per net for all of it left a warp waiting for its largest net (250k nets of degree 2
-// to 64: value 86 us, gradient 179 us; now 50 and 49). A block whose pins do not fit takes a warp per
-// net straight from memory, the sums by strided lanes.
+// to 64: value 86 us, gradient 179 us; now 50 and 49). A block whose pins do not fit, or whose
+// starts do not ascend, takes a warp per net straight from memory, the sums by strided lanes.
 constexpr int kFnNets = 128;
 constexpr int kFnPins = 1024;
 
@@ -68,7 +68,10 @@ __global__ void __launch_bounds__(kThreads) k_wa_fn(int64_t n_nets, const int64_
   const int64_t p0 = net_start[n0], p1 = net_start[n0 + nn];
   const int j = threadIdx.x;
   double total = 0;  // this thread's nets' values
-  if (p1 - p0 <= kFnPins) {
+  // the staged form takes the nets' pins as one run cut at ascending starts; a net that ends
+  // before it starts (an empty one to the form below) would put its neighbours' outside the run
+  const int64_t qb = j < nn ? net_start[n0 + j] : 0, qe = j < nn ? net_start[n0 + j + 1] : 0;
+  if (__syncthreads_and(qe >= qb) && p1 - p0 <= kFnPins) {
     const int np = (int)(p1 - p0);
     for (int k = j; k < np; k += kThreads) {
       s_v[0][k] = xy[2 * (p0 + k)];
@@ -77,8 +80,8 @@ __global__ void __launch_bounds__(kThreads) k_wa_fn(int64_t n_nets, const int64_
     int b = 0, e = 0;
     double wt = 0;
     if (j < nn) {
-      b = (int)(net_start[n0 + j] - p0);
-      e = (int)(net_start[n0 + j + 1] - p0);
+      b = (int)(qb - p0);
+      e = (int)(qe - p0);
       wt = w ? (double)w[n0 + j] : 1.0;
       for (int k = b; k < e; k++) s_of[k] = (uint8_t)j;
     }
