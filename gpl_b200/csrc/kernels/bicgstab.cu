@@ -73,6 +73,7 @@ __device__ __forceinline__ void spmv_tiled_rows(int64_t n, const int64_t *__rest
     e = rs[i + 1];
   }
   const bool tiled = k1 - k0 <= kSpmvTile;
+  const bool inside = tiled && b >= k0 && e <= k1;  // not so where the starts do not ascend
   if (tiled) {
     const int cnt = (int)(k1 - k0);
     const int32_t *c = cols + k0;
@@ -98,7 +99,7 @@ __device__ __forceinline__ void spmv_tiled_rows(int64_t n, const int64_t *__rest
   __syncthreads();
   if (i < n) {
     float tmp = 0.0f;
-    if (tiled) {
+    if (inside) {
       const int lb = (int)(b - k0), le = (int)(e - k0);
       for (int k = lb; k < le; k++) tmp = __fadd_rn(tmp, prod[k]);
     } else {
@@ -651,6 +652,10 @@ __device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, floa
         e = __ldg(q.rs + i + 1);
       }
       float tmp = 0.0f;
+      if (at < k0 || e > k1) {  // starts that do not ascend: the row is no part of the run
+        for (int64_t k = at; k < e; k++) tmp = __fadd_rn(tmp, __fmul_rn(__ldg(q.vals + k), x[__ldg(q.cols + k)]));
+        at = e = k1;
+      }
       for (int64_t m0 = k0; m0 < k1; m0 += kSolveTile) {
         const int cnt = (int)min((int64_t)kSolveTile, k1 - m0);
         const int32_t *cc = q.cols + m0;
@@ -673,7 +678,8 @@ __device__ __forceinline__ void solve_spmv(const SysDev &q, const float *x, floa
           }
         }
         __syncthreads();
-        const int lb = (int)(at - m0), le = (int)(min(e, m0 + cnt) - m0);
+        const int64_t m1 = m0 + cnt;
+        const int lb = (int)(min(at, m1) - m0), le = (int)(min(e, m1) - m0);
         int k = lb;
         if (le - lb >= 4 * kSpmvUnroll) {
           // a long row: 16-byte loads, the next eight products beside the eight dependent adds
