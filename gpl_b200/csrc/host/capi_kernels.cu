@@ -384,29 +384,31 @@ int gpl_kernel_csr_from_triplets(int64_t n, int64_t nt, const int32_t *rows, con
 
 static_assert(GPL_SPMV_ROWS == kSpmvRows && GPL_SPMV_TILED == kSpmvTiled, "the C ABI's SpMV forms");
 
-int gpl_kernel_spmv(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *x, float *y, int32_t form, void *stream) {
-  CsrDev A{n, row_start, cols, vals};
-  cudaStream_t s = (cudaStream_t)stream;
-  if (form != kSpmvSliced || n <= 0) return (int)spmv(A, x, y, form, s);
-  // the sliced copy: the order by length and the slice widths on the device, their
-  // exclusive scan here, the entries
+// A matrix's sliced copy: the order by length and the slice widths on the device, their
+// exclusive scan here, the entries.
+struct SlicedCopy {
   int64_t *starts = nullptr;
   int32_t *row = nullptr, *len = nullptr, *count = nullptr;
   int2 *ent = nullptr;
-  int32_t n_long = 0;
-  cudaError_t e = cudaMalloc(&row, (size_t)n * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&len, (size_t)n * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&count, (size_t)(kSliceLenCap + 1) * sizeof(int32_t));
-  if (e == cudaSuccess) e = csr_slice_order(A, row, len, count, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&n_long, count + kSliceLongRow + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  const int64_t ns = (n - n_long + kSliceRows - 1) / kSliceRows;
-  std::vector<int64_t> h((size_t)ns + 1, 0);
-  if (e == cudaSuccess) e = cudaMalloc(&starts, (size_t)(ns + 1) * sizeof(int64_t));
-  if (e == cudaSuccess) e = csr_slice_widths(n, n_long, len, starts, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), starts, (size_t)ns * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) {
+  ~SlicedCopy() {
+    for (void *p : {(void *)starts, (void *)row, (void *)len, (void *)count, (void *)ent}) cudaFree(p);
+  }
+  cudaError_t make(CsrDev &A, cudaStream_t s) {
+    const int64_t n = A.n;
+    int32_t n_long = 0;
+    cudaError_t e = cudaMalloc(&row, (size_t)n * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&len, (size_t)n * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&count, (size_t)(kSliceLenCap + 1) * sizeof(int32_t));
+    if (e == cudaSuccess) e = csr_slice_order(A, row, len, count, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&n_long, count + kSliceLongRow + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const int64_t ns = (n - n_long + kSliceRows - 1) / kSliceRows;
+    std::vector<int64_t> h((size_t)ns + 1, 0);
+    if (e == cudaSuccess) e = cudaMalloc(&starts, (size_t)(ns + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = csr_slice_widths(n, n_long, len, starts, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), starts, (size_t)ns * sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
     int64_t run = 0;
     for (int64_t k = 0; k < ns; k++) {
       const int64_t w = h[(size_t)k];
@@ -415,22 +417,53 @@ int gpl_kernel_spmv(int64_t n, const int64_t *row_start, const int32_t *cols, co
     }
     h[(size_t)ns] = run;
     e = cudaMemcpyAsync(starts, h.data(), (size_t)(ns + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, s);
-  }
-  const size_t total = (size_t)std::max<int64_t>(h[(size_t)ns], 1);
-  if (e == cudaSuccess) e = cudaMalloc(&ent, total * sizeof(int2));
-  if (e == cudaSuccess) {
+    if (e == cudaSuccess) e = cudaMalloc(&ent, (size_t)std::max<int64_t>(run, 1) * sizeof(int2));
+    if (e != cudaSuccess) return e;
     A.sl_long = n_long;
     A.sl_row = row;
     A.sl_len = len;
     A.sl_start = starts;
     e = csr_slice_fill(A, ent, s);
-  }
-  if (e == cudaSuccess) {
     A.sl_ent = ent;
-    e = spmv(A, x, y, form, s);
+    // the host's starts have been read
+    cudaError_t e2 = cudaStreamSynchronize(s);
+    return e != cudaSuccess ? e : e2;
   }
+};
+
+int gpl_kernel_spmv(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *x, float *y, int32_t form, void *stream) {
+  CsrDev A{n, row_start, cols, vals};
+  cudaStream_t s = (cudaStream_t)stream;
+  if (form != kSpmvSliced || n <= 0) return (int)spmv(A, x, y, form, s);
+  SlicedCopy copy;
+  cudaError_t e = copy.make(A, s);
+  if (e == cudaSuccess) e = spmv(A, x, y, form, s);
   cudaError_t e2 = cudaStreamSynchronize(s);
-  for (void *p : {(void *)starts, (void *)row, (void *)len, (void *)count, (void *)ent}) cudaFree(p);
+  return (int)(e != cudaSuccess ? e : e2);
+}
+
+// Test-only (not in include/gpl.h): the initial placement's pair solve in one of the SpMV's
+// forms, the same matrix and right-hand side on both axes, each with its own start point and
+// solution; iterations and error of each.
+int gpl_rules_bicgstab_pair(int64_t n, const int64_t *row_start, const int32_t *cols, const float *vals, const float *rhs, float *x0, float *x1, int32_t max_iters, int32_t form, int32_t *iterations, float *error, void *stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  if (n <= 0) return (int)cudaErrorInvalidValue;
+  CsrDev A{n, row_start, cols, vals};
+  SlicedCopy copy;
+  cudaError_t e = form == kSpmvSliced ? copy.make(A, s) : cudaSuccess;
+  if (e != cudaSuccess) return (int)e;
+  const size_t bytes = (bicgstab_pair_scratch_bytes(n) + 255) / 256 * 256;
+  char *mem = nullptr;
+  if ((e = cudaMalloc((void **)&mem, 2 * bytes)) != cudaSuccess) return (int)e;
+  const CsrDev m[2] = {A, A};
+  const float *b[2] = {rhs, rhs};
+  float *x[2] = {x0, x1};
+  void *scratch[2] = {mem, mem + bytes};
+  BicgResult r[2]{};
+  e = bicgstab_solve_pair(m, b, x, max_iters, scratch, s, r, form);
+  cudaError_t e2 = cudaStreamSynchronize(s);
+  cudaFree(mem);
+  for (int a = 0; a < 2; a++) iterations[a] = r[a].iterations, error[a] = r[a].error;
   return (int)(e != cudaSuccess ? e : e2);
 }
 
