@@ -382,6 +382,46 @@ int gpl_kernel_csr_from_triplets(int64_t n, int64_t nt, const int32_t *rows, con
   return (int)dev.csr_from_triplets(n, nt, rows, cols, vals, row_start, out_cols, out_vals, nnz);
 }
 
+// Test-only (not in include/gpl.h): both axes' assembled matrix and right-hand side for given
+// instances and pins (host arrays); per axis row_start[n + 1], rhs[n] and at most cap entries.
+int gpl_rules_b2b(int64_t n, const int32_t *box, const uint8_t *locked, const int64_t n_pins, const int32_t *pin_e, const int32_t *pin_inst, const uint8_t *pin_mio, const int32_t *pin_xy, int32_t n_nets, const int64_t *net_start, int32_t max_fanout, int32_t min_diff,
+                  float weight_scale, int64_t cap, int64_t *row_start, int32_t *cols, float *vals, float *rhs, void *stream) {
+  IpSetup s;
+  s.box.assign(reinterpret_cast<const int4 *>(box), reinterpret_cast<const int4 *>(box) + n);
+  s.locked.assign(locked, locked + n);
+  s.clamp.assign(n, int4{});
+  s.grouped.assign(n, 0);
+  s.db_box.assign(n, int4{});
+  s.db_size.assign(n, int2{});
+  s.pin_e.assign(pin_e, pin_e + n_pins);
+  s.pin_inst.assign(pin_inst, pin_inst + n_pins);
+  s.pin_mio.assign(pin_mio, pin_mio + n_pins);
+  s.pin_off.assign(n_pins, int2{});
+  s.pin_xy.assign(reinterpret_cast<const int2 *>(pin_xy), reinterpret_cast<const int2 *>(pin_xy) + n_pins);
+  s.pin_hp.assign(n_pins, 2);
+  s.pin_static.assign(n_pins, int4{});
+  s.net_start.assign(net_start, net_start + n_nets + 1);
+  s.max_fanout = max_fanout;
+  s.min_diff = min_diff;
+  s.weight_scale = weight_scale;
+  IpDevice dev((cudaStream_t)stream);
+  IpAxisResult r[2];
+  cudaError_t e = dev.upload(s);
+  if (e == cudaSuccess) e = dev.assemble(r);
+  for (int a = 0; a < 2 && e == cudaSuccess; a++) {
+    std::vector<int64_t> st;
+    std::vector<int32_t> c;
+    std::vector<float> v, b;
+    if ((e = dev.rows(a, st, c, v, b)) != cudaSuccess) break;
+    if ((int64_t)c.size() > cap) return (int)cudaErrorInvalidValue;
+    std::copy(st.begin(), st.end(), row_start + a * (n + 1));
+    std::copy(c.begin(), c.end(), cols + a * cap);
+    std::copy(v.begin(), v.end(), vals + a * cap);
+    std::copy(b.begin(), b.end(), rhs + a * n);
+  }
+  return (int)e;
+}
+
 static_assert(GPL_SPMV_ROWS == kSpmvRows && GPL_SPMV_TILED == kSpmvTiled, "the C ABI's SpMV forms");
 
 // A matrix's sliced copy: the order by length and the slice widths on the device, their

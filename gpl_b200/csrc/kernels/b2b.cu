@@ -1192,6 +1192,20 @@ cudaError_t IpDevice::solution(int axis, std::vector<float> &x) {
   return cudaStreamSynchronize(s_);
 }
 
+cudaError_t IpDevice::rows(int axis, std::vector<int64_t> &starts, std::vector<int32_t> &cols, std::vector<float> &vals, std::vector<float> &rhs) {
+  Axis &A = ax_[axis];
+  CK(pack(Rows{A.row_off, A.ucount, A.ucol, A.uval}, A.starts, &A.cols, &A.vals, &A.cap, &A.nnz));
+  starts.resize(n_ + 1);
+  cols.resize(A.nnz);
+  vals.resize(A.nnz);
+  rhs.resize(n_);
+  CK(cudaMemcpyAsync(starts.data(), A.starts, (n_ + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s_));
+  if (A.nnz) CK(cudaMemcpyAsync(cols.data(), A.cols, A.nnz * sizeof(int32_t), cudaMemcpyDeviceToHost, s_));
+  if (A.nnz) CK(cudaMemcpyAsync(vals.data(), A.vals, A.nnz * sizeof(float), cudaMemcpyDeviceToHost, s_));
+  if (n_) CK(cudaMemcpyAsync(rhs.data(), A.rhs, n_ * sizeof(float), cudaMemcpyDeviceToHost, s_));
+  return cudaStreamSynchronize(s_);
+}
+
 cudaError_t IpDevice::download(std::vector<int4> &box, std::vector<int4> &db_box) {
   box.resize(n_);
   db_box.resize(n_);

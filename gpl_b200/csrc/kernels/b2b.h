@@ -69,6 +69,8 @@ class IpDevice {
   cudaError_t update();
   // The solution vector of an axis (for the trace's probe lines).
   cudaError_t solution(int axis, std::vector<float> &x);
+  // An axis's assembled rows, packed, and its right-hand side (for the tests).
+  cudaError_t rows(int axis, std::vector<int64_t> &starts, std::vector<int32_t> &cols, std::vector<float> &vals, std::vector<float> &rhs);
   // The placed instances' boxes and database boxes.
   cudaError_t download(std::vector<int4> &box, std::vector<int4> &db_box);
   // `Csr::from_triplets` (src/bicgstab.rs:501-541) on its own, on device triplets: n rows,
