@@ -717,6 +717,13 @@ void load_module_poisson() {
 
 }  // namespace gpl
 
+// Test-only: the double GEMM, D[M][N] = A[M][K] B[N][K]^T on device arrays.
+extern "C" int gpl_rules_dgemm(int32_t M, int32_t N, int32_t K, const double *A, int32_t lda, const double *B, int32_t ldb, double *D, int32_t ldd, void *stream) {
+  gpl::GemmBatchT<double> g{};
+  g.p[0] = gpl::GemmProblemT<double>{M, N, K, A, lda, B, ldb, D, ldd};
+  return (int)gpl::dgemm_tn(g, 1, (cudaStream_t)stream);
+}
+
 // Test-only: the six matrices the device makes, in float, one after the other into host memory
 // (sides ny, nx, ny, ny, nx, nx).
 extern "C" int gpl_rules_basis(int32_t nx, int32_t ny, float *out) {
