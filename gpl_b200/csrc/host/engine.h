@@ -101,7 +101,8 @@ class Engine {
   void hold_locked(int b);
   void swap_slots(int b, SlotId a, SlotId c);
   void copy_slot(int b, SlotId dst, SlotId src);
-  // Every region's scalars (one synchronisation).
+  // Every region's scalars: those the trial's last kernel published, or copied after a
+  // synchronisation.
   void fetch();
   const RegionScalars &scalars(int b) const { return host_scal_[b]; }
   int64_t hpwl();  // synchronises

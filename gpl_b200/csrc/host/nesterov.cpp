@@ -1820,7 +1820,6 @@ struct Placer {
 
 static RegionSetup region_setup(const Nb &nb);
 // Builds the placer (init_nesterov_place + nesterov_base, src/nesterov.rs:787-933) on the
-// host and uploads it.
 // host, in two parts. `prepare` takes what the instances' positions do not change (the cells'
 // and pins' constants, the fillers, the perturbation's draws, the bins and the fixed area in
 // them), so it runs beside the initial placement's rounds, when the host waits for the device;

@@ -51,10 +51,10 @@ void Tuner::stop(cudaStream_t s) {
   if (timed_ && cudaEventRecord(ev_[1], s) != cudaSuccess) timed_ = false;
 }
 
-void Tuner::finish(bool count) {
+void Tuner::finish() {
   if (!in_flight_) return;
   in_flight_ = false;
-  if (timed_ && count) {
+  if (timed_) {
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, ev_[0], ev_[1]) == cudaSuccess)
       samples_[cur_].push_back(ms);

@@ -1,13 +1,14 @@
 // The engine's autotuner: picks, where it runs, the fastest of a launch group's forms that
 // give the same results bit for bit (the scatter's shared-tile and straight-to-HBM forms, the
-// small nets' three WA kernels). Which form wins depends on
-// the data (how far a block's cells spread, the degree mix) and changes as the
-// loop moves cells, so each Tuner times its candidates in place with CUDA events on the
-// stream they run on: every candidate in turn for a few uses, then the fastest by its median
-// time, and the probe again every `period` uses. A use is bracketed by start() and stop();
-// finish() is called once the stream has synchronised (the trial's read-back), reads the use's
-// time and counts it or, for a use that did less work than the others, drops it. A probe that keeps the form in use
-// doubles the period to the next (up to 16 times `period`); one that changes it starts over.
+// small nets' three WA kernels). Which form wins depends on the data (how far a block's cells
+// spread, the degree mix) and changes as the loop moves cells, so each Tuner times its candidates
+// in place with CUDA events on the stream they run on: every candidate in turn for a few uses,
+// then the fastest by its median time, and the probe again every `period` uses. A use is bracketed
+// by start() and stop(); finish() is called once the trial's scalars have been read. They come from
+// its last kernel, which starts after the timed launches have ended, so the use's events are
+// complete although nothing has synchronised; a use whose events are not is dropped. A probe that
+// keeps the form in use doubles the period to the next (up to 16 times `period`); one that changes
+// it starts over.
 //
 // An environment variable can fix the form instead (its accepted values name the candidates
 // in order): the forms give the same results, so it changes only the speed.
@@ -32,8 +33,8 @@ class Tuner {
   // The candidate this use runs, with the start event recorded on `s` when the use is timed.
   int start(cudaStream_t s);
   void stop(cudaStream_t s);
-  // After the stream has synchronised: the use's time counted (or dropped), the choice updated.
-  void finish(bool count = true);
+  // After the use's launches have ended: its time counted, the choice updated.
+  void finish();
   int best() const { return best_; }
   bool fixed() const { return fixed_ >= 0; }
   int64_t probes() const { return probes_; }

@@ -33,7 +33,7 @@ __device__ __forceinline__ double loop_state(const double *S) {
 }
 
 // y = A x, then `0 + 1 * tmp` as the library writes it, each row's products summed in
-// column order (the reference's order). Two forms with the same results (SpmvForm):
+// column order (the reference's order). Three forms with the same results (SpmvForm):
 //  rows:  a thread per row straight from memory;
 //  tiled: a block's rows are contiguous in the CSR arrays, so the block first forms every
 //         product vals[k] * x[cols[k]] of its rows with coalesced loads into shared memory
@@ -384,12 +384,12 @@ __global__ void k_fill(int64_t n, float *a, float v) {
 // chained) they cost 65 us an iteration for two systems of 100k rows, most of it launch and
 // drain latency; here each system's blocks stay resident and meet at barriers in global memory
 // (1.4 us among 148 blocks), and every block takes the scalar steps itself from the partials
-// instead of waiting for one to publish them. Measured, the initial placement's pair: 37 us an
-// iteration at 100k rows (65 before), 149 us at 400k (165), 10 us at 300 (45); one system of
-// 300k rows 72 us (310, a thread per row). What is left at 100k: two products of 9.7 us each,
-// bound by their gathers of x (1.3 of them a clock and SM), seven barriers, five vector steps
-// of 1.2 to 2.3 us. Two blocks of 512 threads an SM (64 registers); the two systems' barriers
-// are their own, so each takes exactly the steps it would take alone.
+// instead of waiting for one to publish them. Measured, the initial placement's pair: 38 us an
+// iteration at 100k rows (65 before), 107 us at 400k (165), 10 us at 300 (45); one system of
+// 300k rows 81 us (310, a thread per row). What is left at 100k: two products of 11 us each,
+// bound by their gathers of x, seven barriers, five vector steps of 1.2 to 2.3 us. Two blocks of
+// 512 threads an SM (64 registers); the two systems' barriers are their own, so each takes exactly
+// the steps it would take alone.
 constexpr int kSolveThreads = 512;
 // A block's products of the tiled form at once (40 KB); longer runs go in pieces.
 constexpr int kSolveTile = 10240;

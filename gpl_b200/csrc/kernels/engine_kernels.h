@@ -214,9 +214,9 @@ void load_module_poisson_tc();
 void load_module_cell_order();
 // Kernel launches one poisson_solve makes.
 int poisson_launches(const PoissonPlan *p);
-// The FP32 solves of n plans (mode 0) with their densities and fields fixed, as five
-// launches in all: each GEMM stage over every plan's problems, the spectral step over every
-// plan's spectrum (the fields equal poisson_solve's bit for bit).
+// The FP32 solves of n plans (mode 0) with their densities and fields fixed, as four
+// launches in all: each GEMM stage over every plan's problems, the spectral step in the second
+// stage's epilogue (the fields equal poisson_solve's bit for bit).
 struct PoissonGroup;
 PoissonGroup *poisson_group_create(PoissonPlan *const *plans, const float *const *density, float *const *field_x, float *const *field_y, int n, cudaError_t *err);
 void poisson_group_destroy(PoissonGroup *g);

@@ -27,14 +27,14 @@ __device__ __forceinline__ float inside_axis(float c, float half, float lo, floa
   return adj;
 }
 
-// The block's cells lie close together (the device orders each region's cells along a Z
-// curve): the block first sums its addends in a shared-memory tile of the bins its cells
-// cover, then adds each touched bin to HBM once. A block whose cells spread over more than
-// kTileBins bins adds straight to HBM. Into the tile, a warp's lanes walk their cells' bins
-// in step, and lanes that hit the same bin in a step pool their addends first (one shared
-// atomic per distinct bin): after the initial placement many cells share a bin. The tile
-// holds 32-bit sums when a block's sum for one bin cannot reach 2^32 (RegionArgs::narrow).
-// Integer adds throughout: the same accumulators in any order.
+// The block's cells lie close together (the device orders each region's cells along a Hilbert
+// curve): where enough of their addends share a bin, the block first sums them in a shared-memory
+// tile of the bins its cells cover (kTileBins slots of 64 bits, or twice as many of 32 when a
+// block's sum for one bin cannot reach 2^32, RegionArgs::narrow), then adds each touched bin to
+// HBM once. Into 32-bit slots each lane adds its own cell's (share_scatter); into 64-bit ones,
+// which have no native add in shared memory, a warp's lanes walk their cells' bins in step and
+// pool what hits one bin (tile_scatter). Other blocks add straight to HBM; place_cells_block has
+// the rule. Integer adds throughout: the same accumulators in any order.
 constexpr int kTileBins = 2048;
 
 // Exact conversions on the FMA and integer pipes for the small values the addends take (the
@@ -414,7 +414,7 @@ __device__ __forceinline__ void place_cells_block(const RegionArgs &r, const Cel
     return;
   }
   if (tile && tiles && s_box[4] >= kDense * slots) {
-    tile_scatter<true>(r, narrow, s_tile, t32, s_red, bcap, s_box[0], s_box[2], s_box[3] - s_box[2], s_box[1] - s_box[0], any, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
+    tile_scatter<true>(r, false, s_tile, nullptr, s_red, bcap, s_box[0], s_box[2], s_box[3] - s_box[2], s_box[1] - s_box[0], any, x0, x1, y0, y1, dlx, dux, dly, duy, scale, kind);
     return;
   }
   const int wcap = bcap / (kThreads / 32);
