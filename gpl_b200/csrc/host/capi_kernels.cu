@@ -174,12 +174,28 @@ __device__ __forceinline__ int net_class(const int64_t *start, int64_t n) {
   const int64_t d = start[n + 1] - start[n];
   return d < 0 ? 0 : d > kWaTilePins ? kWaTilePins + 1 : (int)d;
 }
-static __global__ void __launch_bounds__(256) k_net_classes(int64_t n, const int64_t *__restrict__ start, int32_t *__restrict__ count) {
+// The classes' counts, and the pins the windows reach to (past the last start, where the starts do
+// not ascend).
+struct NetCounts {
+  long long reach;
+  int32_t count[kClasses];
+};
+static __global__ void __launch_bounds__(256) k_net_classes(int64_t n, const int64_t *__restrict__ start, NetCounts *__restrict__ out) {
   __shared__ int32_t h[kClasses];
+  __shared__ long long reach;
+  int32_t *count = out->count;
   for (int k = threadIdx.x; k < kClasses; k += 256) h[k] = 0;
+  if (threadIdx.x == 0) reach = 0;
   __syncthreads();
-  for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) atomicAdd(&h[net_class(start, i)], 1);
+  long long top = 0;
+  for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+    const int c = net_class(start, i);
+    if (c > 0) top = max(top, (long long)start[i + 1]);
+    atomicAdd(&h[c], 1);
+  }
+  if (top > 0) atomicMax(&reach, top);
   __syncthreads();
+  if (threadIdx.x == 0) atomicMax(&out->reach, reach);
   for (int k = threadIdx.x; k < kClasses; k += 256)
     if (h[k]) atomicAdd(&count[k], h[k]);
 }
@@ -218,20 +234,18 @@ struct DeviceNets {
   explicit DeviceNets(cudaStream_t st) : s(st) {}
   cudaError_t build(int64_t n_nets, const int64_t *net_start, const int32_t *pin_xy, const float *net_weight) {
     if (n_nets >= ((int64_t)1 << 31)) return cudaErrorInvalidValue;  // net numbers are 32-bit
-    Scratch hist(kClasses * sizeof(int32_t), s);
+    Scratch hist(sizeof(NetCounts), s);
     cudaError_t e = hist.error();
-    int32_t *d_count = static_cast<int32_t *>(hist.get());
-    int32_t count[kClasses];
-    int64_t np = 0;
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, sizeof count, s);
+    NetCounts *d_count = static_cast<NetCounts *>(hist.get()), got;
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, sizeof got, s);
     if (e != cudaSuccess) return e;
     k_net_classes<<<(unsigned)std::min<int64_t>((n_nets + 255) / 256, 148 * 8), 256, 0, s>>>(n_nets, net_start, d_count);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    e = cudaMemcpyAsync(count, d_count, sizeof count, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&np, net_start + n_nets, sizeof np, cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(&got, d_count, sizeof got, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
-    n_pins = np;
+    const int32_t *count = got.count;
+    const int64_t np = n_pins = got.reach;
     if (np >= ((int64_t)1 << 31)) return cudaErrorInvalidValue;  // pin numbers are 32-bit
     // the classes' places, the tiles of the degrees outside 2..4
     std::vector<int32_t> first(kClasses);
@@ -256,6 +270,7 @@ struct DeviceNets {
       net += count[c];
       pin += (int64_t)count[c] * c;
     }
+    if (pin >= ((int64_t)1 << 31)) return cudaErrorInvalidValue;  // the same of the copies, where windows share pins
     first[kWaTilePins + 1] = 0;  // the larger nets' list
     const int32_t n_big = count[kWaTilePins + 1];
     // one block of scratch: the tables (uploaded together), then what the placement writes

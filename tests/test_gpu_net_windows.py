@@ -1,7 +1,8 @@
-"""The wirelength objective with net starts that do not ascend: each net is its own window
-[start, next start) of the pins, one that ends before it starts is empty, and windows may share
-pins. Value and (where one net alone holds a pin) gradient against the same formula in torch
-double precision; pins of no window keep what the gradient array held."""
+"""Net starts that do not ascend: each net is its own window [start, next start) of the pins, one that
+ends before it starts is empty, and windows may share pins or reach past the last start. The
+wirelength objective's value and (where one net alone holds a pin) gradient against the same formula in torch
+double precision, pins of no window keeping what the gradient array held; and the HPWL, with and
+without the forces beside it, whose array is the call's own."""
 import ctypes as C
 
 import numpy as np
@@ -55,3 +56,25 @@ def test_windows_in_any_order(case):
     one, none = torch.from_numpy(holds == 1).cuda(), torch.from_numpy(holds == 0).cuda()
     assert float((g - 1.7 * want)[one].abs().max() if bool(one.any()) else 0.0) <= 1e-11 * max(float(want.abs().max()), 1.0)
     assert bool((g[none] == 5.0).all())
+
+
+@pytest.mark.parametrize("fused", [0, 1])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("case", list(CASES) + ["all_past_the_last"])
+def test_hpwl_of_windows_in_any_order(case, shift, fused):
+    import torch
+    from gpl_b200 import engine
+    start = np.array(CASES.get(case, [0, 3000, 5000, 5004, 2]), np.int64)
+    n, pins = len(start) - 1, int(start.max())
+    xy = np.random.default_rng(n).integers(-20000, 20000, (pins, 2)).astype(np.int32)
+    buf = torch.zeros(2 * pins + 1, dtype=torch.int32, device="cuda")
+    p = buf[shift:shift + 2 * pins]  # on an 8-byte boundary or off one
+    p.copy_(dev(xy.reshape(-1)))
+    d, h = dev(start), C.c_int64()
+    assert engine.lib().gpl_kernel_hpwl(n, ptr(d), ptr(p), fused, C.byref(h), stream()) == 0
+    want = 0
+    for a, b in zip(start, start[1:]):
+        if b > a:
+            w = xy[a:b].astype(np.int64)
+            want += int((w.max(0) - w.min(0)).sum())
+    assert h.value == want
