@@ -322,9 +322,16 @@ cudaError_t make_map(CUtensorMap *m, const __nv_bfloat16 *base, int rows, int k,
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// The shared memory of one form's kernel, for the current device's context: asked for with each
+// plan, as another device, or the same one after a reset, has its own.
 template <int EPI, int BN>
-void tc_allow() {
-  cudaFuncSetAttribute(k_tc_gemm<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::SMEM_BYTES);
+cudaError_t tc_allow() {
+  return cudaFuncSetAttribute(k_tc_gemm<EPI, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::SMEM_BYTES);
+}
+template <int BN>
+cudaError_t tc_allow_pair() {
+  const cudaError_t e = tc_allow<EPI_SPLIT, BN>();
+  return e != cudaSuccess ? e : tc_allow<EPI_F32, BN>();
 }
 template <int EPI, int BN>
 cudaError_t tc_gemm(const TcArgs &a, int batch, cudaStream_t s, const CUtensorMap &A0, const CUtensorMap &B0, const CUtensorMap &A1, const CUtensorMap &B1) {
@@ -404,19 +411,10 @@ cudaError_t tc_plan_init(PoissonPlan *p, char *base, BasisOut &out) {
   TRY(make_map(&t->mEyh, t->eyh, nx, ny, t->bn2));
   TRY(make_map(&t->mT2, t->t2, ny, nx, t->bn2));         // rows y, K = u
   TRY(make_map(&t->mT3, t->t3, ny, nx, t->bn2));
+  TRY(t->bn1 == 32 ? (tc_allow<EPI_SPLIT, 32>()) : (tc_allow<EPI_SPLIT, 64>()));
+  TRY(t->bn1 == 32 ? (tc_allow<EPI_SPECTRAL, 32>()) : (tc_allow<EPI_SPECTRAL, 64>()));
+  TRY(t->bn2 == 32 ? tc_allow_pair<32>() : t->bn2 == 64 ? tc_allow_pair<64>() : tc_allow_pair<128>());
 #undef TRY
-  static bool attr = false;
-  if (!attr) {
-    tc_allow<EPI_SPLIT, 32>();
-    tc_allow<EPI_SPLIT, 64>();
-    tc_allow<EPI_SPLIT, 128>();
-    tc_allow<EPI_SPECTRAL, 32>();
-    tc_allow<EPI_SPECTRAL, 64>();
-    tc_allow<EPI_F32, 32>();
-    tc_allow<EPI_F32, 64>();
-    tc_allow<EPI_F32, 128>();
-    attr = true;
-  }
   return cudaGetLastError();
 }
 
